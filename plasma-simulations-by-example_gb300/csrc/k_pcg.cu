@@ -178,6 +178,14 @@ __device__ __forceinline__ void grid_sum_t(cg::grid_group &grid, const T (&v)[NV
     for (int q = 0; q < NV; q++) out[q] = tot[q];
 }
 
+/* Whether the inner type takes the cheaper sweeps.  The float64 inner solve
+ * is bound by the narrow float64 pipe, and its last bits reach phi far below
+ * any tolerance, so it multiplies by stored reciprocal diagonals and leaves
+ * out terms that cancel.  The float inner solve keeps the arithmetic of the
+ * plain formulas (its last bits reach the particles' float E). */
+template <typename T>
+constexpr bool LIGHT = sizeof(T) == sizeof(double);
+
 constexpr int MG_MAX = 12;
 /* threads per block of the cooperative solve (one block per SM) */
 constexpr int PCG_THREADS = 1024;
@@ -188,6 +196,7 @@ struct MgLevel {
     int nx, ny, nz, pad;
     int64_t n;
     T *diag, *w, *b, *e; /* w: 6 weights per node, [m][n] */
+    T *id;               /* 1 / diag, 0 where diag is 0 (an aggregate without unknowns) */
 };
 
 template <typename T>
@@ -204,14 +213,14 @@ struct MgArgs {
     MgLevel<T> L[MG_MAX];
 };
 
-/* bytes of one level's arrays (diag, 6 weights, b, e) in shared memory */
+/* bytes of one level's arrays (diag or 1 / diag, 6 weights, b, e) in shared memory */
 template <typename T>
 __host__ __device__ inline size_t level_smem_bytes(int64_t n) {
     return ((size_t)n * sizeof(T) + 15) / 16 * 16 * 9;
 }
 
 /* block 0's view of the levels it works alone: shared-memory copies of
- * L[smem_from..] (diag and weights copied once per launch) */
+ * L[smem_from..] (the diagonal or its reciprocal and the weights copied once per launch) */
 template <typename T>
 __device__ void smem_levels_init(const MgArgs<T> &A, MgArgs<T> &S, unsigned char *base) {
     if (threadIdx.x == 0) {
@@ -220,7 +229,7 @@ __device__ void smem_levels_init(const MgArgs<T> &A, MgArgs<T> &S, unsigned char
         for (int i = A.smem_from; i < A.nlev; i++) {
             const int64_t n = A.L[i].n;
             const size_t a = ((size_t)n * sizeof(T) + 15) / 16 * 16;
-            S.L[i].diag = (T *)(base + off);
+            S.L[i].diag = S.L[i].id = (T *)(base + off); /* the one that the sweeps read */
             S.L[i].w = (T *)(base + off + a);
             S.L[i].b = (T *)(base + off + 7 * a);
             S.L[i].e = (T *)(base + off + 8 * a);
@@ -230,7 +239,7 @@ __device__ void smem_levels_init(const MgArgs<T> &A, MgArgs<T> &S, unsigned char
     __syncthreads();
     for (int i = A.smem_from; i < A.nlev; i++) {
         const int64_t n = A.L[i].n;
-        for (int64_t t = threadIdx.x; t < n; t += blockDim.x) S.L[i].diag[t] = A.L[i].diag[t];
+        for (int64_t t = threadIdx.x; t < n; t += blockDim.x) S.L[i].diag[t] = LIGHT<T> ? A.L[i].id[t] : A.L[i].diag[t];
         for (int64_t t = threadIdx.x; t < 6 * n; t += blockDim.x) S.L[i].w[t] = A.L[i].w[t];
     }
     __syncthreads();
@@ -247,8 +256,9 @@ struct Fine {
     Geo g;
     const uint16_t *code;
     T ct[3];
-    int64_t off[6];
+    int32_t off[6];
     T *dg, *r, *z; /* dg: the Boltzmann part of the Jacobian diagonal */
+    T *id;         /* 1 / the full diagonal on the unknowns, 0 elsewhere */
     const int32_t *list[2]; /* interior nodes of each colour (-1: padding) */
     const int32_t *pk[2];   /* their coordinates, i | j<<10 | k<<20 */
     int32_t nlist;          /* entries per list */
@@ -275,14 +285,27 @@ __global__ void k_pcg_lists(Geo g, int c, int32_t *list, int32_t *pk) {
     pk[t] = i | (j << 10) | (k << 20);
 }
 
-__device__ __forceinline__ void span(bool whole, int64_t &t0, int64_t &ts) {
-    if (whole) {
-        t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-        ts = (int64_t)gridDim.x * blockDim.x;
-    } else {
-        t0 = threadIdx.x;
-        ts = blockDim.x;
-    }
+/* A thread's share of count work items: t, t + step, ... below end. */
+struct Span {
+    int64_t t, end, step;
+};
+
+/* The block alone (whole = false), or the whole grid: with more items than
+ * threads a grid stride (all blocks near each other, so that the neighbour
+ * planes stay in L2); with fewer, one contiguous range of whole warps per
+ * block.  A grid stride over a small count leaves it to the first few blocks
+ * (a colour of 31,000 nodes on 31 of 152 SMs, whose narrow float64 pipes
+ * then work alone); even ranges use every SM.  Up to one item per thread,
+ * both give a warp the same 32 items, so the float warp sums of the dot
+ * products do not depend on the rule. */
+__device__ __forceinline__ Span span(bool whole, int64_t count) {
+    if (!whole) return {(int64_t)threadIdx.x, count, (int64_t)blockDim.x};
+    const int64_t all = (int64_t)gridDim.x * blockDim.x;
+    if (count > all) return {(int64_t)blockIdx.x * blockDim.x + threadIdx.x, count, all};
+    const int32_t per = (int32_t)((((uint32_t)count + gridDim.x - 1) / gridDim.x + 31u) & ~31u);
+    const int64_t t0 = (int64_t)blockIdx.x * per;
+    const int64_t end = t0 + per < count ? t0 + per : count;
+    return {t0 + threadIdx.x, end, (int64_t)blockDim.x};
 }
 
 /* Full Jacobian diagonal of an unknown: its Boltzmann part plus c per
@@ -312,7 +335,6 @@ __device__ __forceinline__ T jacobian_apply(uint16_t cc, T dB, const T ct[3], T 
  * neighbours, whose values are never used) */
 __device__ __forceinline__ int64_t clamp_node(int64_t v, int64_t nn) { return v < 0 ? 0 : (v >= nn ? nn - 1 : v); }
 
-/* red-black half sweep on the node grid: z = (r + sum c z_nb) / diag */
 /* Red-black Gauss-Seidel pieces.  A Gauss-Seidel update never reads the
  * node's own old value, which allows three fusions: the first red half
  * sweep from a zero guess is pointwise (e = b / diag) and is done by whoever
@@ -320,61 +342,65 @@ __device__ __forceinline__ int64_t clamp_node(int64_t v, int64_t nn) { return v 
  * fly to the red neighbours read by the following black half sweep (the red
  * nodes are overwritten next anyway); and the dot products r.z and z.z are
  * accumulated by the last two half sweeps, which produce the final z. */
-/* node-grid half sweep of colour c over the unknowns; with C != null the
- * neighbours are read with the coarse correction added (post-smoothing);
- * adds r*z and z*z of the nodes it updated to rz and zz.  Each thread takes
- * two entries of the colour's enumeration per pass and issues every load of
+/* Red-black half sweep of colour c on the node grid, z = (r + sum c z_nb) /
+ * diag; adds r*z and z*z of the nodes it updated to rz and zz.  With C !=
+ * null the red neighbours are read with the coarse correction added.
+ * LIGHT: z is 0 on every node that is not an unknown, so a Dirichlet or
+ * Neumann neighbour adds nothing without a look at the code, and id, the
+ * reciprocal diagonal written once per Newton step, is 0 there, which marks
+ * the nodes to skip (9 float64 instructions a node; ~25 with the diagonal
+ * summed from the code word and a division).  Each thread takes two
+ * entries of the colour's enumeration per pass and issues every load of
  * both before any store (a padding entry reads the interior node (1,1,1) and
- * stores nothing), so twice as many loads are in flight as with one node per
- * pass.  Entry t is node i = 1 + 2 i2 + ((1+j+k+c)&1) of interior row
- * (j, k), with i2 = t mod hx; below 2^24 entries the coordinates come from
- * float-estimated divisions, above from the precomputed lists. */
+ * stores nothing).  Entry t is node i = 1 + 2 i2 + ((1+j+k+c)&1) of interior
+ * row (j, k), with i2 = t mod hx; below 2^24 entries the coordinates come
+ * from float-estimated divisions, above from the precomputed lists. */
 template <typename T>
 __device__ void fine_half(const Fine<T> &F, int c, const MgLevel<T> *C, T scale, T &rz_out, T &zz_out) {
     T rz = 0, zz = 0;
-    int64_t t0, ts;
-    span(true, t0, ts);
+    const Span S = span(true, F.nlist);
     const int32_t *list = F.list[c], *pk = F.pk[c];
     const Geo &g = F.g;
-    const int64_t safe = ((int64_t)g.nj + 1) * g.ni + 1;
+    const uint32_t safe = ((uint32_t)g.nj + 1u) * (uint32_t)g.ni + 1u;
     const bool arith = F.nlist < (1 << 24);
     const uint32_t hx = (uint32_t)((g.ni - 1) / 2), rj = (uint32_t)(g.nj - 2);
     const float inv_hx = 1.f / (float)hx, inv_rj = 1.f / (float)rj;
-    for (int64_t t = t0; t < F.nlist; t += 2 * ts) {
-        const int64_t tq[2] = {t, t + ts};
-        int64_t u[2];
+    for (int64_t t = S.t; t < S.end; t += 2 * S.step) {
+        const int64_t tq[2] = {t, t + S.step};
+        uint32_t u[2];
         bool ok[2];
         int32_t pq[2];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
+            const bool in = tq[q] < S.end;
             if (arith) {
-                const bool in = tq[q] < F.nlist;
                 const uint32_t tt = in ? (uint32_t)tq[q] : 0u;
                 const uint32_t row = div_small(tt, hx, inv_hx);
                 const uint32_t kk = div_small(row, rj, inv_rj);
                 const int j = 1 + (int)(row - kk * rj), k = 1 + (int)kk;
                 const int i = 1 + 2 * (int)(tt - row * hx) + ((1 + j + k + c) & 1);
                 ok[q] = in && i <= g.ni - 2;
-                u[q] = ok[q] ? ((int64_t)k * g.nj + j) * g.ni + i : safe;
+                u[q] = ok[q] ? ((uint32_t)k * (uint32_t)g.nj + (uint32_t)j) * (uint32_t)g.ni + (uint32_t)i : safe;
                 pq[q] = i | (j << 10) | (k << 20);
             } else {
-                const int32_t uu = tq[q] < F.nlist ? list[tq[q]] : -1;
+                const int32_t uu = in ? list[tq[q]] : -1;
                 ok[q] = uu >= 0;
-                u[q] = ok[q] ? (int64_t)uu : safe;
+                u[q] = ok[q] ? (uint32_t)uu : safe;
                 pq[q] = C && ok[q] ? pk[tq[q]] : 0;
             }
         }
         /* interior node: all six neighbours are in bounds, so their loads
          * are issued before the code word arrives; the code only selects */
+        T ru[2], du[2], zn[2][6]; /* du: 1 / diag, or the diagonal's Boltzmann part */
         uint16_t cc[2];
-        T ru[2], dBu[2], zn[2][6];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            cc[q] = F.code[u[q]];
             ru[q] = F.r[u[q]];
-            dBu[q] = F.dg[u[q]];
+            du[q] = LIGHT<T> ? F.id[u[q]] : F.dg[u[q]];
+            if (C || !LIGHT<T>) cc[q] = F.code[u[q]];
+            const T *zu = F.z + u[q];
 #pragma unroll
-            for (int m = 0; m < 6; m++) zn[q][m] = F.z[u[q] + F.off[m]];
+            for (int m = 0; m < 6; m++) zn[q][m] = zu[F.off[m]];
         }
         if (C) {
             /* the coarse correction at the six neighbours: for each axis one
@@ -397,22 +423,34 @@ __device__ void fine_half(const Fine<T> &F, int c, const MgLevel<T> *C, T scale,
             }
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                const bool oi = par[q] & 1, oj = par[q] & 2, ok_ = par[q] & 4;
-                zn[q][0] += scale * (oi ? ea[q] : ex[q]);
-                zn[q][1] += scale * (oi ? ex[q] : ea[q]);
-                zn[q][2] += scale * (oj ? ea[q] : ey[q]);
-                zn[q][3] += scale * (oj ? ey[q] : ea[q]);
-                zn[q][4] += scale * (ok_ ? ea[q] : ez[q]);
-                zn[q][5] += scale * (ok_ ? ez[q] : ea[q]);
+                const bool odd[3] = {(bool)(par[q] & 1), (bool)(par[q] & 2), (bool)(par[q] & 4)};
+                const T en[3] = {ex[q], ey[q], ez[q]};
+#pragma unroll
+                for (int m = 0; m < 6; m++) {
+                    const bool own = odd[m >> 1] != (bool)(m & 1); /* the neighbour inside the aggregate */
+                    if (LIGHT<T>)
+                        zn[q][m] += (cc[q] & (1u << m)) ? scale * (own ? ea[q] : en[m >> 1]) : (T)0;
+                    else
+                        zn[q][m] += scale * (own ? ea[q] : en[m >> 1]);
+                }
             }
         }
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            if (!ok[q] || !(cc[q] & SELF)) continue;
-            T s = ru[q];
+            T zu;
+            if (LIGHT<T>) {
+                if (!ok[q] || du[q] == (T)0) continue;
+                T s = ru[q];
 #pragma unroll
-            for (int m = 0; m < 6; m++) s += (cc[q] & (1u << m)) ? F.ct[m >> 1] * zn[q][m] : (T)0;
-            const T zu = s / full_diag(cc[q], dBu[q], F.ct);
+                for (int a = 0; a < 3; a++) s += F.ct[a] * (zn[q][2 * a] + zn[q][2 * a + 1]);
+                zu = s * du[q];
+            } else {
+                if (!ok[q] || !(cc[q] & SELF)) continue;
+                T s = ru[q];
+#pragma unroll
+                for (int m = 0; m < 6; m++) s += (cc[q] & (1u << m)) ? F.ct[m >> 1] * zn[q][m] : (T)0;
+                zu = s / full_diag(cc[q], du[q], F.ct);
+            }
             F.z[u[q]] = zu;
             rz += ru[q] * zu;
             zz += zu * zu;
@@ -423,19 +461,19 @@ __device__ void fine_half(const Fine<T> &F, int c, const MgLevel<T> *C, T scale,
 }
 
 /* one half sweep of colour c on a coarse level; with C != null the
- * neighbours are read with C's correction added.  Coordinates come from the
- * sweep index by float-estimated divisions (levels below 2^24 nodes), the
- * neighbours' aggregates from the coordinates. */
+ * neighbours are read with C's correction added (per axis one neighbour
+ * shares the node's aggregate, the other is in the next one).  Coordinates
+ * come from the sweep index by float-estimated divisions (levels below 2^24
+ * nodes). */
 template <typename T>
 __device__ void coarse_half(const MgLevel<T> &L, int c, bool whole, const MgLevel<T> *C, T scale) {
     const int hx = (L.nx + 1) / 2;
     const int64_t count = (int64_t)hx * L.ny * L.nz;
-    const int64_t offs[6] = {-1, 1, -(int64_t)L.nx, L.nx, -(int64_t)L.nx * L.ny, (int64_t)L.nx * L.ny};
+    const int32_t offs[6] = {-1, 1, -L.nx, L.nx, -L.nx * L.ny, L.nx * L.ny};
     const bool fast = count < (1 << 24);
     const float inv_hx = 1.f / (float)hx, inv_ny = 1.f / (float)L.ny;
-    int64_t t0, ts;
-    span(whole, t0, ts);
-    for (int64_t t = t0; t < count; t += ts) {
+    const Span S = span(whole, count);
+    for (int64_t t = S.t; t < S.end; t += S.step) {
         const uint32_t tt = (uint32_t)t;
         uint32_t rr, kk;
         if (fast) {
@@ -450,33 +488,45 @@ __device__ void coarse_half(const MgLevel<T> &L, int c, bool whole, const MgLeve
         const int k = (int)kk;
         const int i = 2 * i2 + ((j + k + c) & 1);
         if (i >= L.nx) continue;
-        const int64_t I = ((int64_t)k * L.ny + j) * L.nx + i;
+        const int32_t I = (k * L.ny + j) * L.nx + i;
         /* all loads first (a missing neighbour reads a clamped node; its zero
          * weight deselects it), then the arithmetic */
-        T d = L.diag[I];
+        const T d = LIGHT<T> ? L.id[I] : L.diag[I];
         T s = L.b[I];
         T wm[6], en[6];
-        const int ci[6] = {i > 0 ? i - 1 : 0, i + 1 < L.nx ? i + 1 : i, i, i, i, i};
-        const int cj[6] = {j, j, j > 0 ? j - 1 : 0, j + 1 < L.ny ? j + 1 : j, j, j};
-        const int ck[6] = {k, k, k, k, k > 0 ? k - 1 : 0, k + 1 < L.nz ? k + 1 : k};
 #pragma unroll
         for (int m = 0; m < 6; m++) {
-            int64_t nb = I + offs[m];
-            nb = nb < 0 ? 0 : (nb >= L.n ? L.n - 1 : nb);
+            int32_t nb = I + offs[m];
+            nb = nb < 0 ? 0 : (nb >= (int32_t)L.n ? (int32_t)L.n - 1 : nb);
             wm[m] = L.w[m * L.n + I];
             en[m] = L.e[nb];
-            if (C) en[m] += scale * C->e[((ck[m] >> 1) * C->ny + (cj[m] >> 1)) * C->nx + (ci[m] >> 1)];
+        }
+        if (C) {
+            const int A = ((k >> 1) * C->ny + (j >> 1)) * C->nx + (i >> 1);
+            /* the next aggregate along each axis; a neighbour off the level
+             * has weight 0 and may read the node's own */
+            const int ax = (i & 1) ? (i + 1 < L.nx ? A + 1 : A) : (i > 0 ? A - 1 : A);
+            const int ay = (j & 1) ? (j + 1 < L.ny ? A + C->nx : A) : (j > 0 ? A - C->nx : A);
+            const int az = (k & 1) ? (k + 1 < L.nz ? A + C->nx * C->ny : A) : (k > 0 ? A - C->nx * C->ny : A);
+            const T ea = C->e[A];
+            const T ex[3] = {C->e[ax], C->e[ay], C->e[az]};
+            const bool odd[3] = {(bool)(i & 1), (bool)(j & 1), (bool)(k & 1)};
+#pragma unroll
+            for (int m = 0; m < 6; m++) en[m] += scale * (odd[m >> 1] != (bool)(m & 1) ? ea : ex[m >> 1]);
         }
         if (d == (T)0) continue;
 #pragma unroll
         for (int m = 0; m < 6; m++) s += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
-        L.e[I] = s / d;
+        L.e[I] = LIGHT<T> ? s * d : s / d;
     }
 }
 
 /* The red children of a coarse node (its 2x2x2 block), in the order in which
  * their residuals are summed: offsets dx | dy<<1 | dz<<2 with dx+dy+dz even
- * (black residuals are zero after the black half sweep). */
+ * (black residuals are zero after the black half sweep).  LIGHT: a red
+ * child's residual r - J z is sum c z over its black neighbours, because its
+ * own value is r / diag from the first red half sweep: neither r nor the
+ * diagonal is read. */
 __device__ __forceinline__ int red_child(int q) { return q == 0 ? 0 : (q == 1 ? 3 : (q == 2 ? 5 : 6)); }
 
 /* Coordinates of coarse node I (float-estimated divisions below 2^24 nodes). */
@@ -508,8 +558,8 @@ __device__ __forceinline__ void restrict_store(const MgLevel<T> &C, bool valid, 
     sum += r3;
     C.b[I] = sum;
     if (((ci + cj + ck) & 1) == 0) {
-        const T d = C.diag[I];
-        if (d != (T)0) C.e[I] = sum / d;
+        const T d = LIGHT<T> ? C.id[I] : C.diag[I];
+        if (d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
     }
 }
 
@@ -520,138 +570,145 @@ __device__ __forceinline__ void restrict_store(const MgLevel<T> &C, bool valid, 
  * grid; a child that is not an unknown contributes zero); otherwise
  * (bandwidth-bound) a thread takes a coarse node and its four children, so
  * that a warp's loads of one child cover consecutive nodes of a row. */
+/* A red child of the node grid: what its residual needs, loaded at once, and
+ * the residual (0 for a node that is not an unknown, or not interior). */
+template <typename T>
+struct FineChild {
+    T id, r, dg, z, zn[6];
+    uint16_t cc;
+    __device__ __forceinline__ void load(const Fine<T> &F, uint32_t u, bool in) {
+        if (LIGHT<T>) {
+            id = in ? F.id[u] : (T)0;
+        } else {
+            cc = in ? F.code[u] : (uint16_t)0;
+            r = F.r[u];
+            dg = F.dg[u];
+            z = F.z[u];
+        }
+        const T *zu = F.z + u;
+#pragma unroll
+        for (int m = 0; m < 6; m++) zn[m] = zu[F.off[m]];
+    }
+    __device__ __forceinline__ T residual(const Fine<T> &F) const {
+        if (LIGHT<T>) {
+            T res = 0;
+#pragma unroll
+            for (int a = 0; a < 3; a++) res += F.ct[a] * (zn[2 * a] + zn[2 * a + 1]);
+            return id != (T)0 ? res : (T)0;
+        }
+        return (cc & SELF) ? r - jacobian_apply(cc, dg, F.ct, z, zn) : (T)0;
+    }
+};
+
+/* interior node of the grid (i, j, k), or the interior node (1,1,1) */
+__device__ __forceinline__ uint32_t interior_or_safe(const Geo &g, int i, int j, int k, bool &in) {
+    in = in && i > 0 && j > 0 && k > 0 && i < g.ni - 1 && j < g.nj - 1 && k < g.nk - 1;
+    const uint32_t ii = in ? (uint32_t)i : 1u, jj = in ? (uint32_t)j : 1u, kk = in ? (uint32_t)k : 1u;
+    return (kk * (uint32_t)g.nj + jj) * (uint32_t)g.ni + ii;
+}
+
 template <typename T>
 __device__ void restrict_fine(const Fine<T> &F, const MgLevel<T> &C) {
     const Geo &g = F.g;
-    const int64_t nn = (int64_t)g.ni * g.nj * g.nk;
-    const int64_t safe = ((int64_t)g.nj + 1) * g.ni + 1;
-    int64_t t0, ts;
-    span(true, t0, ts);
     const bool fast = C.n < (1 << 24);
     const float inv_nx = 1.f / (float)C.nx, inv_ny = 1.f / (float)C.ny;
-    if (C.n > ts) {
-        for (int64_t I = t0; I < C.n; I += ts) {
+    if (C.n > (int64_t)gridDim.x * blockDim.x) {
+        const Span S = span(true, C.n);
+        for (int64_t I = S.t; I < S.end; I += S.step) {
             int ci, cj, ck;
             coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
             T sum = 0;
-            int64_t uu[4];
-            uint16_t cc[4];
+            FineChild<T> ch[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int d = red_child(q);
-                const int i = 2 * ci + (d & 1), j = 2 * cj + ((d >> 1) & 1), k = 2 * ck + (d >> 2);
-                const bool in = i < g.ni && j < g.nj && k < g.nk;
-                uu[q] = in ? ((int64_t)k * g.nj + j) * g.ni + i : 0;
-                cc[q] = in ? F.code[uu[q]] : (uint16_t)0;
+                bool in = true;
+                const uint32_t u =
+                    interior_or_safe(g, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), in);
+                ch[q].load(F, u, in);
             }
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if (!(cc[q] & SELF)) continue;
-                const int64_t u = uu[q];
-                T zn[6];
-#pragma unroll
-                for (int m = 0; m < 6; m++) zn[m] = F.z[u + F.off[m]];
-                sum += F.r[u] - jacobian_apply(cc[q], F.dg[u], F.ct, F.z[u], zn);
-            }
+            for (int q = 0; q < 4; q++) sum += ch[q].residual(F);
             C.b[I] = sum;
             if (((ci + cj + ck) & 1) == 0) {
-                const T d = C.diag[I];
-                if (d != (T)0) C.e[I] = sum / d;
+                const T d = LIGHT<T> ? C.id[I] : C.diag[I];
+                if (d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
             }
         }
         return;
     }
     const int64_t total = 4 * C.n, padded = (total + 31) & ~(int64_t)31;
-    for (int64_t t = t0; t < padded; t += ts) {
+    const Span S = span(true, padded);
+    for (int64_t t = S.t; t < S.end; t += S.step) {
         const bool valid = t < total;
         const int64_t I = valid ? (t >> 2) : 0;
         int ci, cj, ck;
         coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
         const int d = red_child((int)(t & 3));
-        const int i = 2 * ci + (d & 1), j = 2 * cj + ((d >> 1) & 1), k = 2 * ck + (d >> 2);
-        const bool in = valid && i < g.ni && j < g.nj && k < g.nk;
-        const int64_t u = in ? ((int64_t)k * g.nj + j) * g.ni + i : safe;
-        const uint16_t cc = F.code[u];
-        const T ru = F.r[u], dBu = F.dg[u], zu = F.z[u];
-        T zn[6];
-#pragma unroll
-        for (int m = 0; m < 6; m++) {
-            int64_t nb = u + F.off[m];
-            nb = nb < 0 ? 0 : (nb >= nn ? nn - 1 : nb);
-            zn[m] = F.z[nb];
-        }
-        const T res = (in && (cc & SELF)) ? ru - jacobian_apply(cc, dBu, F.ct, zu, zn) : (T)0;
-        restrict_store(C, valid, I, ci, cj, ck, res);
+        bool in = valid;
+        const uint32_t u = interior_or_safe(g, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), in);
+        FineChild<T> ch;
+        ch.load(F, u, in);
+        restrict_store(C, valid, I, ci, cj, ck, ch.residual(F));
     }
 }
 
-/* b of level l+1 from level l, laid out like restrict_fine */
+/* b of level l+1 from level l, laid out like restrict_fine (an aggregate
+ * without unknowns has no weights and contributes 0) */
+template <typename T>
+__device__ __forceinline__ T coarse_child_residual(const MgLevel<T> &L, int i, int j, int k, bool in) {
+    const int32_t offs[6] = {-1, 1, -L.nx, L.nx, -L.nx * L.ny, L.nx * L.ny};
+    in = in && i < L.nx && j < L.ny && k < L.nz;
+    const int32_t u = in ? (k * L.ny + j) * L.nx + i : 0;
+    T wm[6], en[6];
+    const T dd = LIGHT<T> ? (T)1 : L.diag[u], bu = LIGHT<T> ? (T)0 : L.b[u], eu = LIGHT<T> ? (T)0 : L.e[u];
+#pragma unroll
+    for (int m = 0; m < 6; m++) {
+        int32_t nb = u + offs[m];
+        nb = nb < 0 ? 0 : (nb >= (int32_t)L.n ? (int32_t)L.n - 1 : nb);
+        wm[m] = L.w[m * L.n + u];
+        en[m] = L.e[nb];
+    }
+    if (!in || dd == (T)0) return (T)0;
+    T res = LIGHT<T> ? (T)0 : bu - dd * eu;
+#pragma unroll
+    for (int m = 0; m < 6; m++) res += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
+    return res;
+}
+
 template <typename T>
 __device__ void restrict_coarse(const MgLevel<T> &L, const MgLevel<T> &C, bool whole) {
-    const int64_t offs[6] = {-1, 1, -(int64_t)L.nx, L.nx, -(int64_t)L.nx * L.ny, (int64_t)L.nx * L.ny};
-    int64_t t0, ts;
-    span(whole, t0, ts);
     const bool fast = C.n < (1 << 24);
     const float inv_nx = 1.f / (float)C.nx, inv_ny = 1.f / (float)C.ny;
-    if (C.n > ts) {
-        for (int64_t I = t0; I < C.n; I += ts) {
+    if (C.n > (int64_t)(whole ? gridDim.x : 1u) * blockDim.x) {
+        const Span S = span(whole, C.n);
+        for (int64_t I = S.t; I < S.end; I += S.step) {
             int ci, cj, ck;
             coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
             T sum = 0;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int d = red_child(q);
-                const int i = 2 * ci + (d & 1), j = 2 * cj + ((d >> 1) & 1), k = 2 * ck + (d >> 2);
-                const bool in = i < L.nx && j < L.ny && k < L.nz;
-                const int64_t u = in ? ((int64_t)k * L.ny + j) * L.nx + i : 0;
-                const T dd = L.diag[u], bu = L.b[u], eu = L.e[u];
-                T wm[6], en[6];
-#pragma unroll
-                for (int m = 0; m < 6; m++) {
-                    int64_t nb = u + offs[m];
-                    nb = nb < 0 ? 0 : (nb >= L.n ? L.n - 1 : nb);
-                    wm[m] = L.w[m * L.n + u];
-                    en[m] = L.e[nb];
-                }
-                if (!in || dd == (T)0) continue;
-                T res = bu - dd * eu;
-#pragma unroll
-                for (int m = 0; m < 6; m++) res += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
-                sum += res;
+                sum += coarse_child_residual(L, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), true);
             }
             C.b[I] = sum;
             if (((ci + cj + ck) & 1) == 0) {
-                const T d = C.diag[I];
-                if (d != (T)0) C.e[I] = sum / d;
+                const T d = LIGHT<T> ? C.id[I] : C.diag[I];
+                if (d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
             }
         }
         return;
     }
     const int64_t total = 4 * C.n, padded = (total + 31) & ~(int64_t)31;
-    for (int64_t t = t0; t < padded; t += ts) {
+    const Span S = span(whole, padded);
+    for (int64_t t = S.t; t < S.end; t += S.step) {
         const bool valid = t < total;
         const int64_t I = valid ? (t >> 2) : 0;
         int ci, cj, ck;
         coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
         const int d = red_child((int)(t & 3));
-        const int i = 2 * ci + (d & 1), j = 2 * cj + ((d >> 1) & 1), k = 2 * ck + (d >> 2);
-        const bool in = valid && i < L.nx && j < L.ny && k < L.nz;
-        const int64_t u = in ? ((int64_t)k * L.ny + j) * L.nx + i : 0;
-        const T dd = L.diag[u], bu = L.b[u], eu = L.e[u];
-        T wm[6], en[6];
-#pragma unroll
-        for (int m = 0; m < 6; m++) {
-            int64_t nb = u + offs[m];
-            nb = nb < 0 ? 0 : (nb >= L.n ? L.n - 1 : nb);
-            wm[m] = L.w[m * L.n + u];
-            en[m] = L.e[nb];
-        }
-        T res = 0;
-        if (in && dd != (T)0) {
-            res = bu - dd * eu;
-#pragma unroll
-            for (int m = 0; m < 6; m++) res += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
-        }
+        const T res =
+            coarse_child_residual(L, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), valid);
         restrict_store(C, valid, I, ci, cj, ck, res);
     }
 }
@@ -705,9 +762,8 @@ __device__ double vcycle_rest(cg::grid_group &grid, const Fine<T> &F, const MgAr
     if (NL == 0) { /* Jacobi: the caller computed z on every node */
         T rz = 0, z2 = 0;
         int64_t nn = (int64_t)F.g.ni * F.g.nj * F.g.nk;
-        int64_t t0, ts;
-        span(true, t0, ts);
-        for (int64_t u = t0; u < nn; u += ts)
+        const Span S = span(true, nn);
+        for (int64_t u = S.t; u < S.end; u += S.step)
             if (F.code[u] & SELF) {
                 T zu = F.z[u];
                 rz += F.r[u] * zu;
@@ -829,17 +885,17 @@ __device__ double vcycle_rest(cg::grid_group &grid, const Fine<T> &F, const MgAr
  * 3 phi - 3 p1 + p2 (quadratic), and p2 = p1.  In double-float. */
 __device__ __noinline__ void df_prepass(const double *__restrict__ phi, const double *__restrict__ rho, float2 *phf,
                                         float2 *rhf, const uint16_t *__restrict__ code, double *phi_prev,
-                                        int predict, dfl d_inv_eps0, int64_t nn, int64_t gtid, int64_t gsize) {
+                                        int predict, dfl d_inv_eps0, int64_t nn, Span S) {
     /* four nodes a pass, every load before any store (the pass is bound by
      * the loads in flight) */
-    for (int64_t u0 = gtid; u0 < nn; u0 += 4 * gsize) {
+    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         double cur[4], prev[4], prev2[4], rh[4];
         uint16_t c[4];
         bool on[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * gsize;
-            on[h] = u < nn;
+            const int64_t u = u0 + h * S.step;
+            on[h] = u < S.end;
             const int64_t v = on[h] ? u : 0;
             cur[h] = phi[v];
             rh[h] = rho[v];
@@ -850,7 +906,7 @@ __device__ __noinline__ void df_prepass(const double *__restrict__ phi, const do
 #pragma unroll
         for (int h = 0; h < 4; h++) {
             if (!on[h]) continue;
-            const int64_t u = u0 + h * gsize;
+            const int64_t u = u0 + h * S.step;
             dfl x = df_split(cur[h]);
             if (predict) {
                 if (predict >= 2 && (c[h] & SELF)) {
@@ -875,25 +931,25 @@ __device__ __noinline__ void df_prepass(const double *__restrict__ phi, const do
  * thread's sum of y^2 */
 template <typename T>
 __device__ __noinline__ float df_update(const uint16_t *__restrict__ code, const T *__restrict__ yv, float2 *phf,
-                                        int64_t nn, int64_t gtid, int64_t gsize) {
+                                        Span S) {
     float yys = 0.f;
     /* four nodes a pass, every load before any store */
-    for (int64_t u0 = gtid; u0 < nn; u0 += 4 * gsize) {
+    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         uint16_t c[4];
         float yu[4];
         float2 x[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * gsize;
-            const int64_t v = u < nn ? u : 0;
-            c[h] = u < nn ? code[v] : (uint16_t)0;
+            const int64_t u = u0 + h * S.step;
+            const int64_t v = u < S.end ? u : 0;
+            c[h] = u < S.end ? code[v] : (uint16_t)0;
             yu[h] = (float)yv[v];
             x[h] = phf[v];
         }
 #pragma unroll
         for (int h = 0; h < 4; h++) {
             if (!(c[h] & SELF)) continue;
-            phf[u0 + h * gsize] = df_pack(df_add(df_unpack(x[h]), {-yu[h], 0.f}));
+            phf[u0 + h * S.step] = df_pack(df_add(df_unpack(x[h]), {-yu[h], 0.f}));
             yys = __fmaf_rn(yu[h], yu[h], yys);
         }
     }
@@ -903,37 +959,36 @@ __device__ __noinline__ float df_update(const uint16_t *__restrict__ code, const
 /* phi of the unknowns from their pairs (hi + lo rounded once), four nodes
  * a pass with every load before any store */
 __device__ __noinline__ void df_rebuild(const uint16_t *__restrict__ code, const float2 *__restrict__ phf,
-                                        double *phi, int64_t nn, int64_t gtid, int64_t gsize) {
-    for (int64_t u0 = gtid; u0 < nn; u0 += 4 * gsize) {
+                                        double *phi, Span S) {
+    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         uint16_t c[4];
         float2 x[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * gsize;
-            c[h] = u < nn ? code[u] : (uint16_t)0;
-            x[h] = phf[u < nn ? u : 0];
+            const int64_t u = u0 + h * S.step;
+            c[h] = u < S.end ? code[u] : (uint16_t)0;
+            x[h] = phf[u < S.end ? u : 0];
         }
 #pragma unroll
         for (int h = 0; h < 4; h++)
-            if (c[h] & SELF) phi[u0 + h * gsize] = (double)x[h].x + (double)x[h].y;
+            if (c[h] & SELF) phi[u0 + h * S.step] = (double)x[h].x + (double)x[h].y;
     }
 }
 
 /* Neumann boundary nodes take the value at the end of their chain (the
  * chains end at unknowns or Dirichlet nodes, which this pass does not
  * write), four nodes a pass */
-__device__ __noinline__ void neumann_copies(const int32_t *__restrict__ target, double *phi, int64_t nn,
-                                            int64_t gtid, int64_t gsize) {
-    for (int64_t u0 = gtid; u0 < nn; u0 += 4 * gsize) {
+__device__ __noinline__ void neumann_copies(const int32_t *__restrict__ target, double *phi, Span S) {
+    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         int32_t t[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * gsize;
-            t[h] = u < nn ? target[u] : -1;
+            const int64_t u = u0 + h * S.step;
+            t[h] = u < S.end ? target[u] : -1;
         }
 #pragma unroll
         for (int h = 0; h < 4; h++)
-            if (t[h] >= 0) phi[u0 + h * gsize] = phi[t[h]];
+            if (t[h] >= 0) phi[u0 + h * S.step] = phi[t[h]];
     }
 }
 
@@ -948,22 +1003,22 @@ __device__ __noinline__ void neumann_copies(const int32_t *__restrict__ target, 
  * need no clamp (s1, s2: the y and z strides). */
 template <typename T>
 __device__ __noinline__ float df_residual(const uint16_t *__restrict__ code, const float2 *__restrict__ phf,
-                                          const float2 *__restrict__ rhf, T *z, T *dg, T *r, T *y, int64_t nn,
-                                          int64_t gtid, int64_t gsize, int32_t s1, int32_t s2, const T ct[3],
+                                          const float2 *__restrict__ rhf, T *z, T *dg, T *r, T *y, Span S,
+                                          int32_t s1, int32_t s2, const T ct[3],
                                           const float cl[3], dfl d_phi0, dfl d_inv_te0, dfl d_A0, float A0_te0,
                                           bool jacobi) {
     float ffs = 0.f;
     /* two nodes a pass, every load before the arithmetic; a node that is
      * not an unknown reads the interior node safe_u and stores nothing */
     const int64_t safe_u = (int64_t)s2 + s1 + 1;
-    for (int64_t u0 = gtid; u0 < nn; u0 += 2 * gsize) {
+    for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
         uint16_t cq[2];
         int64_t uq[2];
         float2 xq[2], pq[2][6], bq[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int64_t u = u0 + h * gsize;
-            cq[h] = u < nn ? code[u] : (uint16_t)0;
+            const int64_t u = u0 + h * S.step;
+            cq[h] = u < S.end ? code[u] : (uint16_t)0;
             uq[h] = (cq[h] & SELF) ? u : safe_u;
         }
 #pragma unroll
@@ -1017,7 +1072,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                                                         const int32_t *__restrict__ target, double phi0,
                                                         double te0, double n0, int nr_max, double nr_tol,
                                                         int pcg_max, double pcg_tol, T *y, T *r, T *z, T *p0,
-                                                        T *p1, T *q, T *dg, MgArgs<T> mg, const int32_t *lists,
+                                                        T *p1, T *q, T *dg, T *id, MgArgs<T> mg, const int32_t *lists,
                                                         double *partials, SolveStatus *st, int *err,
                                                         double *lin_y, const double *__restrict__ lin_b,
                                                         int gs_max, double gs_tol, float2 *dfbuf, double *phi_prev,
@@ -1034,7 +1089,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
     }
     const int64_t nn = (int64_t)g.ni * g.nj * g.nk;
     const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    const int64_t off[6] = {-1, 1, -sy, sy, -sz, sz};
+    const int32_t off[6] = {-1, 1, -(int32_t)sy, (int32_t)sy, -(int32_t)sz, (int32_t)sz};
     const int64_t safe = sz + sy + 1; /* the interior node (1,1,1) */
     const double cd[3] = {1.0 / (g.dh[0] * g.dh[0]), 1.0 / (g.dh[1] * g.dh[1]), 1.0 / (g.dh[2] * g.dh[2])};
     /* (T)cd from the host: derived here from cd, the compiler re-derived it
@@ -1045,7 +1100,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
     const double A0 = PCG_QE * n0 / PCG_EPS_0;
     const double inv_te0 = 1.0 / te0, A0_te0 = A0 / te0, inv_eps0 = 1.0 / PCG_EPS_0;
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t gsize = (int64_t)gridDim.x * blockDim.x;
+    const Span S = span(true, nn); /* this thread's nodes */
     const bool jacobi = mg.nlev == 0;
     Fine<T> F;
     F.g = g;
@@ -1053,6 +1108,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
     for (int m = 0; m < 3; m++) F.ct[m] = ct[m];
     for (int m = 0; m < 6; m++) F.off[m] = off[m];
     F.dg = dg;
+    F.id = id;
     F.r = r;
     F.z = z;
     F.nlist = (int32_t)((int64_t)((g.ni - 1) / 2) * (g.nj - 2) * (g.nk - 2));
@@ -1074,7 +1130,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
     float2 *phf = dfbuf, *rhf = dfbuf ? dfbuf + nn : nullptr;
     const dfl d_phi0 = df_of(phi0), d_inv_te0 = df_of(inv_te0), d_A0 = df_of(A0), d_inv_eps0 = df_of(inv_eps0);
     if (dfm) {
-        df_prepass(phi, rho, phf, rhf, code, phi_prev, predict, d_inv_eps0, nn, gtid, gsize);
+        df_prepass(phi, rho, phf, rhf, code, phi_prev, predict, d_inv_eps0, nn, S);
         grid.sync();
     }
     const float cl[3] = {(float)(cd[0] - (double)ct[0]), (float)(cd[1] - (double)ct[1]),
@@ -1092,24 +1148,24 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
              * per axis c (2 x_u - x_w - x_e) (a missing link reads x_u), the
              * Boltzmann factor as expf of the leading part times a
              * first-order factor for the rest, rho / eps0 from its pair */
-            const float ffs = df_residual<T>(code, phf, rhf, z, dg, r, y, nn, gtid, gsize, (int32_t)sy, (int32_t)sz,
-                                             ct, cl, d_phi0, d_inv_te0, d_A0, (float)A0_te0, jacobi);
+            const float ffs = df_residual<T>(code, phf, rhf, z, dg, r, y, S, (int32_t)sy, (int32_t)sz, ct, cl,
+                                             d_phi0, d_inv_te0, d_A0, (float)A0_te0, jacobi);
             ff = (double)ffs;
         } else
         /* two nodes per pass, every load before any store; the loads do not
          * wait for the code word (neighbour indices are clamped into the
          * grid, a node past the end reads the interior node (1,1,1)), and
          * a node that is not an unknown stores nothing */
-        for (int64_t u0 = gtid; u0 < nn; u0 += 2 * gsize) {
-            const int64_t uq[2] = {u0, u0 + gsize};
+        for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+            const int64_t uq[2] = {u0, u0 + S.step};
             bool onq[2];
             uint16_t c[2];
             int64_t u[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                c[h] = uq[h] < nn ? code[uq[h]] : (uint16_t)0;
+                c[h] = uq[h] < S.end ? code[uq[h]] : (uint16_t)0;
                 onq[h] = c[h] & SELF;
-                u[h] = uq[h] < nn ? uq[h] : safe;
+                u[h] = uq[h] < S.end ? uq[h] : safe;
             }
             double xu[2], pn[2][6], ph[2], bv[2];
 #pragma unroll
@@ -1170,7 +1226,9 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                     Fv = linear ? L + dB * xu[h] - bv[h] : L + A0 * e - bv[h] * inv_eps0;
                     rv = (T)Fv;
                     dBt = (T)dB;
-                    if (jacobi || !(c[h] & BLACK)) z[u[h]] = rv / (T)(dL + dB);
+                    const T iv = (T)(1.0 / (dL + dB));
+                    if (jacobi || !(c[h] & BLACK)) z[u[h]] = rv * iv;
+                    id[u[h]] = iv;
                 }
                 dg[u[h]] = dBt;
                 r[u[h]] = rv;
@@ -1204,16 +1262,16 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                  * do not wait for the code word (neighbour indices clamped
                  * into the grid, a node past the end reads the interior node
                  * (1,1,1)); a node that is not an unknown stores nothing */
-                for (int64_t u0 = gtid; u0 < nn; u0 += 2 * gsize) {
-                    const int64_t uq[2] = {u0, u0 + gsize};
+                for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+                    const int64_t uq[2] = {u0, u0 + S.step};
                     bool on[2];
                     uint16_t c[2];
                     int64_t u[2];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        c[h] = uq[h] < nn ? code[uq[h]] : (uint16_t)0;
+                        c[h] = uq[h] < S.end ? code[uq[h]] : (uint16_t)0;
                         on[h] = c[h] & SELF;
-                        u[h] = uq[h] < nn ? uq[h] : safe;
+                        u[h] = uq[h] < S.end ? uq[h] : safe;
                     }
                     /* an unknown is interior: neighbour loads need no code bit */
                     T zc[2], pc[2], dB[2], zn[2][6], pn[2][6];
@@ -1252,16 +1310,16 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                 const T alpha = bc_alpha;
                 /* y += alpha p, r -= alpha q, and the first red half sweep */
                 T rr = 0;
-                for (int64_t u0 = gtid; u0 < nn; u0 += 2 * gsize) {
-                    const int64_t uq[2] = {u0, u0 + gsize};
+                for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+                    const int64_t uq[2] = {u0, u0 + S.step};
                     bool on[2];
                     uint16_t c[2];
                     int64_t u[2];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        c[h] = uq[h] < nn ? code[uq[h]] : (uint16_t)0;
+                        c[h] = uq[h] < S.end ? code[uq[h]] : (uint16_t)0;
                         on[h] = c[h] & SELF;
-                        u[h] = uq[h] < nn ? uq[h] : safe;
+                        u[h] = uq[h] < S.end ? uq[h] : safe;
                     }
                     T yv[2], pv[2], rv[2], qv[2], dv[2];
 #pragma unroll
@@ -1270,7 +1328,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                         pv[h] = pnew[u[h]];
                         rv[h] = r[u[h]];
                         qv[h] = q[u[h]];
-                        dv[h] = dg[u[h]];
+                        dv[h] = LIGHT<T> ? id[u[h]] : dg[u[h]];
                     }
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -1279,7 +1337,8 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                         T ru = rv[h] - alpha * qv[h];
                         r[u[h]] = ru;
                         rr += ru * ru;
-                        if (jacobi || !(c[h] & BLACK)) z[u[h]] = ru / full_diag(c[h], dv[h], ct);
+                        if (jacobi || !(c[h] & BLACK)) 
+                            z[u[h]] = LIGHT<T> ? ru * dv[h] : ru / full_diag(c[h], dv[h], ct);
                     }
                 }
                 const T t4[1] = {rr};
@@ -1320,25 +1379,25 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
              * the correction, J e = r from e = 0 (r = F - J y is the PCG's
              * residual), then y += e. */
             if (!inner_ok && gs_max > 0) {
-                for (int64_t u = gtid; u < nn; u += gsize) z[u] = (T)0;
+                for (int64_t u = S.t; u < S.end; u += S.step) z[u] = (T)0;
                 grid.sync();
                 for (int sw = 0; sw < gs_max; sw++) {
                     for (int col = 0; col < 2; col++) {
-                        for (int64_t u = gtid; u < nn; u += gsize) {
+                        for (int64_t u = S.t; u < S.end; u += S.step) {
                             const uint16_t cc = code[u];
                             if (!(cc & SELF) || ((cc & BLACK) ? 1 : 0) != col) continue;
                             T acc = r[u];
 #pragma unroll
                             for (int m = 0; m < 6; m++)
                                 if (cc & (1u << m)) acc += ct[m >> 1] * z[u + off[m]];
-                            z[u] = acc / full_diag(cc, dg[u], ct);
+                            z[u] = LIGHT<T> ? acc * id[u] : acc / full_diag(cc, dg[u], ct);
                         }
                         grid.sync();
                     }
                     fallback++;
                     if (sw % 25 == 0) {
                         T rr2 = 0;
-                        for (int64_t u = gtid; u < nn; u += gsize) {
+                        for (int64_t u = S.t; u < S.end; u += S.step) {
                             const uint16_t cc = code[u];
                             if (!(cc & SELF)) continue;
                             T xn[6];
@@ -1355,7 +1414,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                         if (bc_stop) break;
                     }
                 }
-                for (int64_t u = gtid; u < nn; u += gsize)
+                for (int64_t u = S.t; u < S.end; u += S.step)
                     if (code[u] & SELF) y[u] += z[u];
                 grid.sync();
             }
@@ -1364,19 +1423,19 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
         double yy = 0;
         double *X = linear ? lin_y : phi;
         if (dfm) {
-            yy = (double)df_update<T>(code, take_z ? z : y, phf, nn, gtid, gsize);
+            yy = (double)df_update<T>(code, take_z ? z : y, phf, S);
         } else
         /* two nodes per pass, loads ahead of the code test and the stores */
-        for (int64_t u0 = gtid; u0 < nn; u0 += 2 * gsize) {
-            const int64_t uq[2] = {u0, u0 + gsize};
+        for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+            const int64_t uq[2] = {u0, u0 + S.step};
             int64_t u[2];
             uint16_t c[2];
             T yv[2];
             double xv[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                u[h] = uq[h] < nn ? uq[h] : safe;
-                c[h] = uq[h] < nn ? code[u[h]] : (uint16_t)0;
+                u[h] = uq[h] < S.end ? uq[h] : safe;
+                c[h] = uq[h] < S.end ? code[u[h]] : (uint16_t)0;
                 yv[h] = take_z ? z[u[h]] : y[u[h]];
                 xv[h] = X[u[h]];
             }
@@ -1406,10 +1465,10 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
         }
     }
     if (dfm) {
-        df_rebuild(code, phf, phi, nn, gtid, gsize);
+        df_rebuild(code, phf, phi, S);
         grid.sync();
     }
-    if (!linear) neumann_copies(target, phi, nn, gtid, gsize);
+    if (!linear) neumann_copies(target, phi, S);
     if (gtid == 0) {
         st->converged = conv;
         st->iterations = nr;
@@ -1472,6 +1531,7 @@ __global__ void k_mg_setup(Geo g, const uint16_t *__restrict__ code, MgLevel<T> 
         (void)offs;
     }
     C.diag[I] = (T)diag;
+    C.id[I] = diag != 0 ? (T)(1.0 / diag) : (T)0;
     for (int m = 0; m < 6; m++) C.w[m * C.n + I] = (T)w[m];
 }
 
@@ -1569,6 +1629,8 @@ static size_t mg_layout(World &w, MgArgs<T> &A, char *base) {
         size_t bytes = ((L.n * sizeof(T) + 255) / 256) * 256;
         L.diag = (T *)(base ? base + off : nullptr);
         off += bytes;
+        L.id = (T *)(base ? base + off : nullptr);
+        off += bytes;
         L.w = (T *)(base ? base + off : nullptr);
         off += 6 * bytes;
         L.b = (T *)(base ? base + off : nullptr);
@@ -1638,7 +1700,7 @@ static int run_pcg(World &w) {
     size_t listb = need_lists ? ((4 * nlist * sizeof(int32_t) + 255) / 256) * 256 : 0;
     /* float inner solves: the (hi, lo) pairs of phi and rho / eps0 */
     size_t dfb = sizeof(T) == sizeof(float) ? 2 * (((size_t)w.nn * sizeof(float2) + 255) / 256) * 256 : 0;
-    size_t need = 7 * vec + codeb + mgb + listb + dfb;
+    size_t need = 8 * vec + codeb + mgb + listb + dfb;
     if (w.pcg_bytes < need || w.pcg_elem != (int)es) {
         if (w.pcg_buf) {
             cudaStreamSynchronize(w.stream);
@@ -1653,10 +1715,12 @@ static int run_pcg(World &w) {
         w.pcg_codes_valid = false;
     }
     char *base = (char *)w.pcg_buf;
-    uint16_t *code = (uint16_t *)(base + 7 * vec);
-    int32_t *lists = (int32_t *)(base + 7 * vec + codeb + mgb);
-    mg_layout<T>(w, A, base + 7 * vec + codeb);
+    uint16_t *code = (uint16_t *)(base + 8 * vec);
+    int32_t *lists = (int32_t *)(base + 8 * vec + codeb + mgb);
+    mg_layout<T>(w, A, base + 8 * vec + codeb);
     if (!w.pcg_codes_valid) {
+        /* the sweeps rely on zeros off the unknowns, which just changed */
+        cudaMemsetAsync(base, 0, 8 * vec, w.stream);
         k_pcg_codes<<<blocks_for(w.nn, 256), 256, 0, w.stream>>>(w.g, w.obj, code);
         w.nlaunch++;
         for (int c = 0; c < 2 && need_lists; c++) {
@@ -1702,7 +1766,11 @@ static int run_pcg(World &w) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn);
     if (per_sm < 1) per_sm = 1;
     int64_t maxb = (int64_t)per_sm * w.sm_count;
-    int64_t needb = (w.nn + threads - 1) / threads;
+    /* every SM as soon as there is a warp of nodes for each: the phases of a
+     * small grid are bound by the instructions and float64 operations that
+     * one SM issues between two barriers, and a barrier of 152 blocks costs
+     * what one of 16 does (1.29 and 1.30 us) */
+    int64_t needb = (w.nn + 31) / 32;
     int grid = (int)(needb < maxb ? needb : maxb);
     if (grid > w.partial_slots / 4) grid = w.partial_slots / 4;
     if (w.solver_blocks > 0 && grid > w.solver_blocks) grid = w.solver_blocks;
@@ -1713,8 +1781,8 @@ static int run_pcg(World &w) {
     const uint16_t *cc = code;
     double phi0 = w.phi0, te0 = w.te0, n0 = w.n0, nr_tol = w.nr_tol, pcg_tol = w.pcg_tol;
     int nr_max = w.nr_max, pcg_max = w.pcg_max;
-    T *v[7];
-    for (int i = 0; i < 7; i++) v[i] = (T *)(base + i * vec);
+    T *v[8];
+    for (int i = 0; i < 8; i++) v[i] = (T *)(base + i * vec);
     double *part = w.d_partials;
     SolveStatus *st = w.d_status;
     int *err = w.d_err;
@@ -1724,7 +1792,7 @@ static int run_pcg(World &w) {
     int gs_max = w.gs_fallback ? w.max_it : 0;
     double gs_tol = w.tol;
     /* the pairs hold nn float2 each, the second array 256-byte aligned */
-    float2 *dfp = dfb ? (float2 *)(base + 7 * vec + codeb + mgb + listb) : nullptr;
+    float2 *dfp = dfb ? (float2 *)(base + 8 * vec + codeb + mgb + listb) : nullptr;
     /* the predictor rides on the pairs' pass (the caller skipped k_predict) */
     double *pp = w.phi_prev;
     int predict = dfp && !ly ? w.predict_mode : 0;
@@ -1733,7 +1801,7 @@ static int run_pcg(World &w) {
     Coef3<T> ctp;
     for (int a = 0; a < 3; a++) ctp.c[a] = (T)(1.0 / (g.dh[a] * g.dh[a]));
     void *args[] = {&g,    &phi,  &rho,  &cc,   &tg,   &phi0, &te0, &n0,  &nr_max, &nr_tol, &pcg_max, &pcg_tol,
-                    &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6], &A,  &lst,   &part,   &st,      &err,
+                    &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6], &v[7], &A,  &lst,   &part,   &st,      &err,
                     &ly,   &lb,   &gs_max, &gs_tol, &dfp,  &pp,   &predict, &ctp};
     w.nlaunch++;
     return (int)cudaLaunchCooperativeKernel(fn, grid, threads, args, dyn, w.stream);
