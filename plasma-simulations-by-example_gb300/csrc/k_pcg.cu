@@ -187,8 +187,13 @@ template <typename T>
 constexpr bool LIGHT = sizeof(T) == sizeof(double);
 
 constexpr int MG_MAX = 12;
-/* threads per block of the cooperative solve (one block per SM) */
-constexpr int PCG_THREADS = 1024;
+/* threads per block of the cooperative solve (one block per SM): 1024 for
+ * large grids, whose passes live on loads in flight (256x256x512 float: 20
+ * ms against 28 with 512 threads), 512 for small ones, whose passes are a
+ * chain of latencies that the 64 registers of 1024 threads lengthen by
+ * spills (33x29x65 float solve: 0.75 ms with 1024, 0.63 with 512; 64x64x128
+ * float64: 7.5 and 6.8 ms a cold solve) */
+constexpr int PCG_THREADS = 1024, PCG_THREADS_SMALL = 512;
 constexpr size_t PCG_SMEM_MAX = 160 * 1024; /* shared memory for block 0's coarse levels */
 
 template <typename T>
@@ -257,8 +262,8 @@ struct Fine {
     const uint16_t *code;
     T ct[3];
     int32_t off[6];
-    T *dg, *r, *z; /* dg: the Boltzmann part of the Jacobian diagonal */
-    T *id;         /* 1 / the full diagonal on the unknowns, 0 elsewhere */
+    T *dg, *r, *z; /* dg: the Boltzmann part of the Jacobian diagonal (LIGHT: the whole of it) */
+    T *id;         /* LIGHT: 1 / the diagonal on the unknowns, 0 elsewhere */
     const int32_t *list[2]; /* interior nodes of each colour (-1: padding) */
     const int32_t *pk[2];   /* their coordinates, i | j<<10 | k<<20 */
     int32_t nlist;          /* entries per list */
@@ -1066,8 +1071,8 @@ __device__ __noinline__ float df_residual(const uint16_t *__restrict__ code, con
     return ffs;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *phi, const double *__restrict__ rho,
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, const double *__restrict__ rho,
                                                         const uint16_t *__restrict__ code,
                                                         const int32_t *__restrict__ target, double phi0,
                                                         double te0, double n0, int nr_max, double nr_tol,
@@ -1225,7 +1230,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                     const double dB = A0_te0 * e;
                     Fv = linear ? L + dB * xu[h] - bv[h] : L + A0 * e - bv[h] * inv_eps0;
                     rv = (T)Fv;
-                    dBt = (T)dB;
+                    dBt = (T)(dL + dB); /* the whole diagonal (LIGHT) */
                     const T iv = (T)(1.0 / (dL + dB));
                     if (jacobi || !(c[h] & BLACK)) z[u[h]] = rv * iv;
                     id[u[h]] = iv;
@@ -1259,9 +1264,10 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                  * q = J p */
                 T pq = 0;
                 /* two nodes per pass, every load before any store; the loads
-                 * do not wait for the code word (neighbour indices clamped
-                 * into the grid, a node past the end reads the interior node
-                 * (1,1,1)); a node that is not an unknown stores nothing */
+                 * do not wait for the code word (a plane of padding around
+                 * the vectors takes a boundary node's missing neighbours, a
+                 * node past the end reads the interior node (1,1,1)); a node
+                 * that is not an unknown stores nothing */
                 for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
                     const int64_t uq[2] = {u0, u0 + S.step};
                     bool on[2];
@@ -1281,15 +1287,31 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                         pc[h] = it ? pold[u[h]] : (T)0;
                         dB[h] = dg[u[h]];
 #pragma unroll
-                        for (int m = 0; m < 6; m++) {
-                            const int64_t nb = clamp_node(u[h] + off[m], nn);
-                            zn[h][m] = z[nb];
-                            pn[h][m] = it ? pold[nb] : (T)0;
+                        for (int m = 0; m < 6; m++) zn[h][m] = z[u[h] + off[m]];
+                        if (LIGHT<T>) {
+                            pn[h][0] = it ? q[u[h]] : (T)0;
+                        } else {
+#pragma unroll
+                            for (int m = 0; m < 6; m++) pn[h][m] = it ? pold[u[h] + off[m]] : (T)0;
                         }
                     }
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         if (!on[h]) continue;
+                        if (LIGHT<T>) {
+                            /* J p = J z + beta J p_old: the last q instead of
+                             * p's neighbours (10 float64 instructions, 28
+                             * with p formed at seven nodes) */
+                            T s = dB[h] * zc[h];
+#pragma unroll
+                            for (int a = 0; a < 3; a++) s -= ct[a] * (zn[h][2 * a] + zn[h][2 * a + 1]);
+                            s += beta * pn[h][0];
+                            const T pl = zc[h] + beta * pc[h];
+                            pnew[u[h]] = pl;
+                            q[u[h]] = s;
+                            pq += pl * s;
+                            continue;
+                        }
                         T pu = zc[h] + beta * pc[h];
 #pragma unroll
                         for (int m = 0; m < 6; m++) pn[h][m] = zn[h][m] + beta * pn[h][m];
@@ -1403,7 +1425,15 @@ __global__ void __launch_bounds__(PCG_THREADS, 1) k_newton_pcg(Geo g, double *ph
                             T xn[6];
 #pragma unroll
                             for (int m = 0; m < 6; m++) xn[m] = (cc & (1u << m)) ? z[u + off[m]] : (T)0;
-                            const T R = r[u] - jacobian_apply(cc, dg[u], ct, z[u], xn);
+                            T Jz;
+                            if (LIGHT<T>) {
+                                Jz = dg[u] * z[u];
+#pragma unroll
+                                for (int a = 0; a < 3; a++) Jz -= ct[a] * (xn[2 * a] + xn[2 * a + 1]);
+                            } else {
+                                Jz = jacobian_apply(cc, dg[u], ct, z[u], xn);
+                            }
+                            const T R = r[u] - Jz;
                             rr2 += R * R;
                         }
                         const T t5[1] = {rr2};
@@ -1689,7 +1719,10 @@ static int run_pcg(World &w) {
     /* the colour lists pack coordinates in 10 + 10 + 11 bits */
     if (w.g.ni > 1024 || w.g.nj > 1024 || w.g.nk > 2048) return (int)cudaErrorInvalidValue;
     size_t es = sizeof(T);
-    size_t vec = ((w.nn * es + 255) / 256) * 256;
+    /* a plane of padding on both sides of each vector, so that reads of a
+     * boundary node's neighbours need no clamp */
+    const size_t pad = (((size_t)w.g.ni * w.g.nj * es + 255) / 256) * 256;
+    size_t vec = ((w.nn * es + 255) / 256) * 256 + 2 * pad;
     size_t codeb = ((w.nn * sizeof(uint16_t) + 255) / 256) * 256;
     MgArgs<T> A;
     size_t mgb = mg_layout<T>(w, A, nullptr);
@@ -1756,8 +1789,11 @@ static int run_pcg(World &w) {
         }
         w.pcg_codes_valid = true;
     }
-    const void *fn = (const void *)k_newton_pcg<T>;
-    const int threads = PCG_THREADS;
+    /* float: up to one node per thread, where both give a warp the same
+     * nodes and so the same dot products; float64: up to 2^20 nodes */
+    const bool small = sizeof(T) == sizeof(float) ? w.nn <= (int64_t)PCG_THREADS_SMALL * w.sm_count : w.nn <= 1 << 20;
+    const int threads = small ? PCG_THREADS_SMALL : PCG_THREADS;
+    const void *fn = small ? (const void *)k_newton_pcg<T, PCG_THREADS_SMALL> : (const void *)k_newton_pcg<T, PCG_THREADS>;
     size_t dyn = 0;
     if (A.smem_from >= 0)
         for (int i = A.smem_from; i < A.nlev; i++) dyn += level_smem_bytes<T>(A.L[i].n);
@@ -1782,7 +1818,7 @@ static int run_pcg(World &w) {
     double phi0 = w.phi0, te0 = w.te0, n0 = w.n0, nr_tol = w.nr_tol, pcg_tol = w.pcg_tol;
     int nr_max = w.nr_max, pcg_max = w.pcg_max;
     T *v[8];
-    for (int i = 0; i < 8; i++) v[i] = (T *)(base + i * vec);
+    for (int i = 0; i < 8; i++) v[i] = (T *)(base + i * vec + pad);
     double *part = w.d_partials;
     SolveStatus *st = w.d_status;
     int *err = w.d_err;
