@@ -177,9 +177,6 @@ struct World {
     int64_t prof_n[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
 
-/* n / d for n < 2^24 without an integer division: the float estimate is
- * within one of the quotient (n is exact in float and 1/d is rounded once),
- * and one remainder test corrects it */
 /* x == +-0, tested on the 32-bit halves of its bits: written as a 64-bit
  * test of the bits it compiles to a float64 compare, which issues on this
  * GPU's narrow float64 pipe */
@@ -187,6 +184,9 @@ __device__ __forceinline__ bool zero_bits(double x) {
     return (((unsigned int)__double2hiint(x) << 1) | (unsigned int)__double2loint(x)) == 0u;
 }
 
+/* n / d for n < 2^24, or n < 2^31 with a quotient below 2^22, without an
+ * integer division: the float estimate (n, 1/d and the product each rounded
+ * once) is within one of the quotient, and one remainder test corrects it */
 __device__ __forceinline__ uint32_t div_small(uint32_t n, uint32_t d, float inv_d) {
     uint32_t q = __float2uint_rz((float)n * inv_d);
     const int32_t r = (int32_t)(n - q * d);

@@ -84,94 +84,84 @@ __global__ void k_pcg_codes(Geo g, const int32_t *__restrict__ obj, uint16_t *co
     code[u] = c;
 }
 
-/* Grid-wide sums of NV values: block partials, one grid barrier, then every
- * block sums the partials with its first warp (lane l takes partials l,
- * l+32, ... in order; a fixed shuffle tree combines the lanes).  Every block
- * computes bit-identical totals, so all blocks take the same branches. */
-template <int NV>
-__device__ __forceinline__ void grid_sum_n(cg::grid_group &grid, double (&v)[NV], double *partials, int &round) {
-    __shared__ double sh[NV][32];
-    __shared__ double tot[NV];
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; q++) {
-        double x = v[q];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[q][wid] = x;
-    }
-    __syncthreads();
-    double *slot = partials + (size_t)(round & 1) * gridDim.x * NV;
-    if (wid == 0) {
-        /* the warps' sums by a fixed shuffle tree (blocks of 32 warps) */
-#pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double s = lane < (int)(blockDim.x >> 5) ? sh[q][lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) slot[(size_t)blockIdx.x * NV + q] = s;
-        }
-    }
-    round++;
-    grid.sync();
-    if (wid == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double s = 0;
-#pragma unroll 4
-            for (unsigned b = lane; b < gridDim.x; b += 32) s += __ldcg(slot + (size_t)b * NV + q);
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) tot[q] = s;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NV; q++) v[q] = tot[q];
-}
-
-
-/* The same for per-thread values of the inner-solve type T: the warp stage
- * adds in T (for float, five float shuffle steps instead of five float64
- * ones in each of a block's 32 warps, which the narrow float64 pipe
- * serialised), then the warps' sums, the blocks' partials and the grid
- * total are float64 as above. */
+/* Grid-wide sums of NV per-thread values of type T: block partials, one grid
+ * barrier, then every block sums the partials with its first warp (lane l
+ * takes partials l, l+32, ... in order; a fixed shuffle tree combines the
+ * lanes).  Every block computes bit-identical totals, so all blocks take the
+ * same branches.  Floats are added in float within a warp; the warps' sums,
+ * the blocks' partials and the total are float64.  Doubles go through shared
+ * memory, 128 threads per value adding blockDim / 128 of them first: a
+ * shuffle tree would issue five full-warp float64 additions per warp and
+ * value, half of a pass over a small grid.  The partials of up to 160 blocks
+ * are loaded at once (loaded in a rolled loop, they cost two L2 latencies
+ * per value). */
 template <int NV, typename T>
-__device__ __forceinline__ void grid_sum_t(cg::grid_group &grid, const T (&v)[NV], double (&out)[NV],
-                                           double *partials, int &round) {
-    if (sizeof(T) == sizeof(double)) {
-#pragma unroll
-        for (int q = 0; q < NV; q++) out[q] = (double)v[q];
-        grid_sum_n<NV>(grid, out, partials, round);
-        return;
-    }
+__device__ __forceinline__ void grid_sum(cg::grid_group &grid, const T (&v)[NV], double (&out)[NV], double *partials,
+                                         int &round) {
     __shared__ double shw[NV][32];
     __shared__ double tot[NV];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int nw = (int)(blockDim.x >> 5); /* entries of shw per value */
+    if (sizeof(T) == sizeof(double)) {
+        __shared__ double all[NV][1024];
 #pragma unroll
-    for (int q = 0; q < NV; q++) {
-        T x = v[q];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if (lane == 0) shw[q][wid] = (double)x;
+        for (int q = 0; q < NV; q++) all[q][threadIdx.x] = (double)v[q];
+        __syncthreads();
+        if ((int)threadIdx.x < 128 * NV) {
+            const int q = threadIdx.x >> 7, t = threadIdx.x & 127;
+            double x = all[q][t];
+            for (int b = t + 128; b < (int)blockDim.x; b += 128) x += all[q][b];
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == 0) shw[q][wid & 3] = x;
+        }
+        nw = 4;
+    } else {
+#pragma unroll
+        for (int q = 0; q < NV; q++) {
+            T x = v[q];
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            if (lane == 0) shw[q][wid] = (double)x;
+        }
     }
     __syncthreads();
     double *slot = partials + (size_t)(round & 1) * gridDim.x * NV;
     if (wid == 0) {
+        double x[NV];
 #pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double sum = lane < (int)(blockDim.x >> 5) ? shw[q][lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (lane == 0) slot[(size_t)blockIdx.x * NV + q] = sum;
-        }
+        for (int q = 0; q < NV; q++) x[q] = lane < nw ? shw[q][lane] : 0.0;
+#pragma unroll
+        for (int o = sizeof(T) == sizeof(double) ? 2 : 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < NV; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < NV; q++) slot[(size_t)blockIdx.x * NV + q] = x[q];
     }
     round++;
     grid.sync();
     if (wid == 0) {
+        double x[NV];
 #pragma unroll
-        for (int q = 0; q < NV; q++) {
-            double sum = 0;
-#pragma unroll 4
-            for (unsigned b = lane; b < gridDim.x; b += 32) sum += __ldcg(slot + (size_t)b * NV + q);
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (lane == 0) tot[q] = sum;
+        for (int q = 0; q < NV; q++) x[q] = 0;
+        for (unsigned b0 = lane; b0 < gridDim.x; b0 += 160) {
+            double t[5][NV];
+#pragma unroll
+            for (int i = 0; i < 5; i++)
+#pragma unroll
+                for (int q = 0; q < NV; q++)
+                    t[i][q] = b0 + 32 * i < gridDim.x ? __ldcg(slot + (size_t)(b0 + 32 * i) * NV + q) : 0.0;
+#pragma unroll
+            for (int i = 0; i < 5; i++)
+#pragma unroll
+                for (int q = 0; q < NV; q++) x[q] += t[i][q];
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < NV; q++) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < NV; q++) tot[q] = x[q];
     }
     __syncthreads();
 #pragma unroll
@@ -224,32 +214,6 @@ __host__ __device__ inline size_t level_smem_bytes(int64_t n) {
     return ((size_t)n * sizeof(T) + 15) / 16 * 16 * 9;
 }
 
-/* block 0's view of the levels it works alone: shared-memory copies of
- * L[smem_from..] (the diagonal or its reciprocal and the weights copied once per launch) */
-template <typename T>
-__device__ void smem_levels_init(const MgArgs<T> &A, MgArgs<T> &S, unsigned char *base) {
-    if (threadIdx.x == 0) {
-        S = A;
-        size_t off = 0;
-        for (int i = A.smem_from; i < A.nlev; i++) {
-            const int64_t n = A.L[i].n;
-            const size_t a = ((size_t)n * sizeof(T) + 15) / 16 * 16;
-            S.L[i].diag = S.L[i].id = (T *)(base + off); /* the one that the sweeps read */
-            S.L[i].w = (T *)(base + off + a);
-            S.L[i].b = (T *)(base + off + 7 * a);
-            S.L[i].e = (T *)(base + off + 8 * a);
-            off += 9 * a;
-        }
-    }
-    __syncthreads();
-    for (int i = A.smem_from; i < A.nlev; i++) {
-        const int64_t n = A.L[i].n;
-        for (int64_t t = threadIdx.x; t < n; t += blockDim.x) S.L[i].diag[t] = LIGHT<T> ? A.L[i].id[t] : A.L[i].diag[t];
-        for (int64_t t = threadIdx.x; t < 6 * n; t += blockDim.x) S.L[i].w[t] = A.L[i].w[t];
-    }
-    __syncthreads();
-}
-
 /* everything the level-0 (node grid) operations need */
 template <typename T>
 struct Coef3 {
@@ -261,38 +225,66 @@ struct Fine {
     Geo g;
     const uint16_t *code;
     T ct[3];
-    int32_t off[6];
+    uint32_t nn;
     T *dg, *r, *z; /* dg: the Boltzmann part of the Jacobian diagonal (LIGHT: the whole of it) */
     T *id;         /* LIGHT: 1 / the diagonal on the unknowns, 0 elsewhere */
-    const int32_t *list[2]; /* interior nodes of each colour (-1: padding) */
-    const int32_t *pk[2];   /* their coordinates, i | j<<10 | k<<20 */
-    int32_t nlist;          /* entries per list */
+    uint32_t ncolour; /* entries of a colour's enumeration */
 };
 
-/* the interior nodes of colour c in a fixed order, with packed coordinates
- * (built once per geometry so that the sweeps need no division) */
-__global__ void k_pcg_lists(Geo g, int c, int32_t *list, int32_t *pk) {
-    int hx = (g.ni - 1) / 2;
-    int64_t count = (int64_t)hx * (g.nj - 2) * (g.nk - 2);
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    int i2 = (int)(t % hx);
-    int64_t rr = t / hx;
-    int j = 1 + (int)(rr % (g.nj - 2));
-    int k = 1 + (int)(rr / (g.nj - 2));
-    int i = 1 + 2 * i2 + ((1 + j + k + c) & 1);
-    if (i > g.ni - 2) {
-        list[t] = -1;
-        pk[t] = 0;
-        return;
-    }
-    list[t] = (int32_t)(((int64_t)k * g.nj + j) * g.ni + i);
-    pk[t] = i | (j << 10) | (k << 20);
+/* What the passes of a solve share, kept once per block in shared memory: the
+ * passes are functions of their own (not inlined) that read it there, so
+ * that each has the block's registers to itself.  Inlined into one kernel,
+ * 1024 threads of 64 registers spilled in the node loops (256x256x512 float:
+ * the black post-smoothing half took 262 us against 116 us for the same half
+ * without the prolongation). */
+template <typename T>
+struct SolveShared {
+    Fine<T> F;
+    MgArgs<T> A; /* the levels in global memory */
+    MgArgs<T> B; /* block 0's view of the levels it works alone: shared-memory copies of L[smem_from..] */
+};
+
+template <typename T>
+__device__ __forceinline__ SolveShared<T> &shared_of() {
+    __shared__ SolveShared<T> st;
+    return st;
 }
 
-/* A thread's share of count work items: t, t + step, ... below end. */
+/* fills the shared state; block 0 also copies the diagonals (or their
+ * reciprocals, what the sweeps read) and weights of the levels it works alone
+ * into shared memory, once per launch */
+template <typename T>
+__device__ __forceinline__ void shared_init(const Fine<T> &F, const MgArgs<T> &A, unsigned char *base) {
+    SolveShared<T> &st = shared_of<T>();
+    const bool staged = A.smem_from >= 0 && A.nlev > 0 && blockIdx.x == 0;
+    if (threadIdx.x == 0) {
+        st.F = F;
+        st.A = A;
+        st.B = A;
+        size_t off = 0;
+        for (int i = A.smem_from; staged && i < A.nlev; i++) {
+            const size_t a = ((size_t)A.L[i].n * sizeof(T) + 15) / 16 * 16;
+            st.B.L[i].diag = st.B.L[i].id = (T *)(base + off); /* the one that the sweeps read */
+            st.B.L[i].w = (T *)(base + off + a);
+            st.B.L[i].b = (T *)(base + off + 7 * a);
+            st.B.L[i].e = (T *)(base + off + 8 * a);
+            off += 9 * a;
+        }
+    }
+    __syncthreads();
+    for (int i = A.smem_from; staged && i < A.nlev; i++) {
+        const int64_t n = st.A.L[i].n;
+        for (int64_t t = threadIdx.x; t < n; t += blockDim.x)
+            st.B.L[i].diag[t] = LIGHT<T> ? st.A.L[i].id[t] : st.A.L[i].diag[t];
+        for (int64_t t = threadIdx.x; t < 6 * n; t += blockDim.x) st.B.L[i].w[t] = st.A.L[i].w[t];
+    }
+    __syncthreads();
+}
+
+/* A thread's share of count work items: t, t + step, ... below end (grids
+ * have at most 2^31 nodes). */
 struct Span {
-    int64_t t, end, step;
+    uint32_t t, end, step;
 };
 
 /* The block alone (whole = false), or the whole grid: with more items than
@@ -303,14 +295,13 @@ struct Span {
  * then work alone); even ranges use every SM.  Up to one item per thread,
  * both give a warp the same 32 items, so the float warp sums of the dot
  * products do not depend on the rule. */
-__device__ __forceinline__ Span span(bool whole, int64_t count) {
-    if (!whole) return {(int64_t)threadIdx.x, count, (int64_t)blockDim.x};
-    const int64_t all = (int64_t)gridDim.x * blockDim.x;
-    if (count > all) return {(int64_t)blockIdx.x * blockDim.x + threadIdx.x, count, all};
-    const int32_t per = (int32_t)((((uint32_t)count + gridDim.x - 1) / gridDim.x + 31u) & ~31u);
-    const int64_t t0 = (int64_t)blockIdx.x * per;
-    const int64_t end = t0 + per < count ? t0 + per : count;
-    return {t0 + threadIdx.x, end, (int64_t)blockDim.x};
+__device__ __forceinline__ Span span(bool whole, uint32_t count) {
+    if (!whole) return {threadIdx.x, count, blockDim.x};
+    const uint32_t all = gridDim.x * blockDim.x;
+    if (count > all) return {blockIdx.x * blockDim.x + threadIdx.x, count, all};
+    const uint32_t per = ((count + gridDim.x - 1) / gridDim.x + 31u) & ~31u;
+    const uint32_t t0 = blockIdx.x * per;
+    return {t0 + threadIdx.x, t0 + per < count ? t0 + per : count, blockDim.x};
 }
 
 /* Full Jacobian diagonal of an unknown: its Boltzmann part plus c per
@@ -347,148 +338,164 @@ __device__ __forceinline__ int64_t clamp_node(int64_t v, int64_t nn) { return v 
  * fly to the red neighbours read by the following black half sweep (the red
  * nodes are overwritten next anyway); and the dot products r.z and z.z are
  * accumulated by the last two half sweeps, which produce the final z. */
-/* Red-black half sweep of colour c on the node grid, z = (r + sum c z_nb) /
- * diag; adds r*z and z*z of the nodes it updated to rz and zz.  With C !=
- * null the red neighbours are read with the coarse correction added.
- * LIGHT: z is 0 on every node that is not an unknown, so a Dirichlet or
- * Neumann neighbour adds nothing without a look at the code, and id, the
+/* Keeps a loaded value where it was loaded: without it the compiler moves a
+ * pass's loads behind the test of the code word, and each pass waits for two
+ * memory latencies instead of one. */
+__device__ __forceinline__ void pin(float &x) { asm volatile("" : "+f"(x)); }
+__device__ __forceinline__ void pin(double &x) { asm volatile("" : "+d"(x)); }
+template <typename T, int N>
+__device__ __forceinline__ void pin(T (&x)[N]) {
+#pragma unroll
+    for (int m = 0; m < N; m++) pin(x[m]);
+}
+
+/* The six neighbours of u in order -x, +x, -y, +y, -z, +z */
+template <typename T>
+__device__ __forceinline__ void load_neighbours(const T *__restrict__ x, uint32_t u, int32_t sy, int32_t sz, T xn[6]) {
+    const T *p = x + u;
+    xn[0] = p[-1];
+    xn[1] = p[1];
+    xn[2] = p[-sy];
+    xn[3] = p[sy];
+    xn[4] = p[-sz];
+    xn[5] = p[sz];
+}
+
+/* Red-black half sweep of a colour on the node grid, z = (r + sum c z_nb) /
+ * diag; POST_* return the thread's sums of r*z and z*z over the nodes it
+ * updated.  POST_BLACK reads the red neighbours with the coarse correction
+ * added.  LIGHT: z is 0 on every node that is not an unknown, so a Dirichlet
+ * or Neumann neighbour adds nothing without a look at the code, and id, the
  * reciprocal diagonal written once per Newton step, is 0 there, which marks
  * the nodes to skip (9 float64 instructions a node; ~25 with the diagonal
- * summed from the code word and a division).  Each thread takes two
- * entries of the colour's enumeration per pass and issues every load of
- * both before any store (a padding entry reads the interior node (1,1,1) and
- * stores nothing).  Entry t is node i = 1 + 2 i2 + ((1+j+k+c)&1) of interior
- * row (j, k), with i2 = t mod hx; below 2^24 entries the coordinates come
- * from float-estimated divisions, above from the precomputed lists. */
+ * summed from the code word and a division).  Each thread takes PER entries
+ * of the colour's enumeration per pass and issues every load of theirs before
+ * any store (a padding entry reads the interior node (1,1,1) and stores
+ * nothing).  Entry t is node i = 1 + 2 i2 + ((1+j+k+c)&1) of interior row
+ * (j, k), with i2 = t mod hx. */
+enum { PRE_BLACK = 0, POST_BLACK = 1, POST_RED = 2 };
+
 template <typename T>
-__device__ void fine_half(const Fine<T> &F, int c, const MgLevel<T> *C, T scale, T &rz_out, T &zz_out) {
+struct Dots {
+    T rz, zz;
+};
+
+template <typename T, int MODE, int PER>
+__device__ __forceinline__ Dots<T> fine_half() {
+    const Fine<T> &F = shared_of<T>().F;
+    constexpr int c = MODE == POST_RED ? 0 : 1;
     T rz = 0, zz = 0;
-    const Span S = span(true, F.nlist);
-    const int32_t *list = F.list[c], *pk = F.pk[c];
-    const Geo &g = F.g;
-    const uint32_t safe = ((uint32_t)g.nj + 1u) * (uint32_t)g.ni + 1u;
-    const bool arith = F.nlist < (1 << 24);
-    const uint32_t hx = (uint32_t)((g.ni - 1) / 2), rj = (uint32_t)(g.nj - 2);
+    T *__restrict__ z = F.z;
+    const T *__restrict__ r = F.r;
+    const T *__restrict__ dd = LIGHT<T> ? F.id : F.dg;
+    const uint16_t *__restrict__ code = F.code;
+    const T ct[3] = {F.ct[0], F.ct[1], F.ct[2]};
+    const int32_t ni = F.g.ni, sz = F.g.ni * F.g.nj;
+    const uint32_t hx = (uint32_t)((ni - 1) / 2), rj = (uint32_t)(F.g.nj - 2);
     const float inv_hx = 1.f / (float)hx, inv_rj = 1.f / (float)rj;
-    for (int64_t t = S.t; t < S.end; t += 2 * S.step) {
-        const int64_t tq[2] = {t, t + S.step};
-        uint32_t u[2];
-        bool ok[2];
-        int32_t pq[2];
+    const Span S = span(true, F.ncolour);
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += PER * S.step) {
+        uint32_t u[PER];
+        bool ok[PER];
+        T ru[PER], du[PER], zn[PER][6], ea[PER], en[PER][3];
+        uint16_t cc[PER];
+        int par[PER];
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const bool in = tq[q] < S.end;
-            if (arith) {
-                const uint32_t tt = in ? (uint32_t)tq[q] : 0u;
-                const uint32_t row = div_small(tt, hx, inv_hx);
-                const uint32_t kk = div_small(row, rj, inv_rj);
-                const int j = 1 + (int)(row - kk * rj), k = 1 + (int)kk;
-                const int i = 1 + 2 * (int)(tt - row * hx) + ((1 + j + k + c) & 1);
-                ok[q] = in && i <= g.ni - 2;
-                u[q] = ok[q] ? ((uint32_t)k * (uint32_t)g.nj + (uint32_t)j) * (uint32_t)g.ni + (uint32_t)i : safe;
-                pq[q] = i | (j << 10) | (k << 20);
-            } else {
-                const int32_t uu = in ? list[tq[q]] : -1;
-                ok[q] = uu >= 0;
-                u[q] = ok[q] ? (uint32_t)uu : safe;
-                pq[q] = C && ok[q] ? pk[tq[q]] : 0;
-            }
-        }
-        /* interior node: all six neighbours are in bounds, so their loads
-         * are issued before the code word arrives; the code only selects */
-        T ru[2], du[2], zn[2][6]; /* du: 1 / diag, or the diagonal's Boltzmann part */
-        uint16_t cc[2];
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            ru[q] = F.r[u[q]];
-            du[q] = LIGHT<T> ? F.id[u[q]] : F.dg[u[q]];
-            if (C || !LIGHT<T>) cc[q] = F.code[u[q]];
-            const T *zu = F.z + u[q];
-#pragma unroll
-            for (int m = 0; m < 6; m++) zn[q][m] = zu[F.off[m]];
-        }
-        if (C) {
-            /* the coarse correction at the six neighbours: for each axis one
-             * neighbour shares the node's aggregate, the other is the next
-             * aggregate on the side of the node's parity */
-            const MgLevel<T> &Cc = *C;
-            T ea[2], ex[2], ey[2], ez[2];
-            int par[2];
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int32_t p = ok[q] ? pq[q] : (1 | (1 << 10) | (1 << 20));
-                const int i = p & 1023, j = (p >> 10) & 1023, k = p >> 20;
-                const int32_t sy = Cc.nx, sz = Cc.nx * Cc.ny;
-                const int32_t A = ((k >> 1) * Cc.ny + (j >> 1)) * Cc.nx + (i >> 1);
+        for (int q = 0; q < PER; q++) {
+            const bool in = t + q * S.step < S.end;
+            const uint32_t tt = in ? t + q * S.step : 0u;
+            const uint32_t row = div_small(tt, hx, inv_hx);
+            const uint32_t kk = div_small(row, rj, inv_rj);
+            int j = 1 + (int)(row - kk * rj), k = 1 + (int)kk;
+            int i = 1 + 2 * (int)(tt - row * hx) + ((1 + j + k + c) & 1);
+            ok[q] = in && i <= ni - 2;
+            if (!ok[q]) i = j = k = 1;
+            u[q] = (uint32_t)k * (uint32_t)sz + (uint32_t)(j * ni + i);
+            /* interior node: all six neighbours are in bounds, so their loads
+             * do not wait for the code word, which only selects */
+            ru[q] = r[u[q]];
+            du[q] = dd[u[q]];
+            if (MODE == POST_BLACK || !LIGHT<T>) cc[q] = code[u[q]];
+            load_neighbours(z, u[q], ni, sz, zn[q]);
+            if (MODE == POST_BLACK) {
+                /* the coarse correction at the six neighbours: for each axis
+                 * one neighbour shares the node's aggregate, the other is
+                 * the next aggregate on the side of the node's parity */
+                const MgLevel<T> &C = shared_of<T>().A.L[0];
+                const int32_t cy = C.nx, cz = C.nx * C.ny;
+                const T *e = C.e + ((k >> 1) * cz + (j >> 1) * cy + (i >> 1));
                 par[q] = (i & 1) | ((j & 1) << 1) | ((k & 1) << 2);
-                ea[q] = Cc.e[A];
-                ex[q] = Cc.e[(i & 1) ? A + 1 : A - 1];
-                ey[q] = Cc.e[(j & 1) ? A + sy : A - sy];
-                ez[q] = Cc.e[(k & 1) ? A + sz : A - sz];
+                ea[q] = e[0];
+                en[q][0] = e[(i & 1) ? 1 : -1];
+                en[q][1] = e[(j & 1) ? cy : -cy];
+                en[q][2] = e[(k & 1) ? cz : -cz];
             }
+        }
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const bool odd[3] = {(bool)(par[q] & 1), (bool)(par[q] & 2), (bool)(par[q] & 4)};
-                const T en[3] = {ex[q], ey[q], ez[q]};
+        for (int q = 0; q < PER; q++) {
+            pin(ru[q]);
+            pin(du[q]);
+            pin(zn[q]);
+            if (MODE == POST_BLACK) {
+                pin(ea[q]);
+                pin(en[q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            if (MODE == POST_BLACK) {
+                const T scale = shared_of<T>().A.scale;
 #pragma unroll
                 for (int m = 0; m < 6; m++) {
-                    const bool own = odd[m >> 1] != (bool)(m & 1); /* the neighbour inside the aggregate */
+                    /* the neighbour inside the aggregate? */
+                    const bool own = (bool)(par[q] & (1 << (m >> 1))) != (bool)(m & 1);
+                    const T cor = scale * (own ? ea[q] : en[q][m >> 1]);
                     if (LIGHT<T>)
-                        zn[q][m] += (cc[q] & (1u << m)) ? scale * (own ? ea[q] : en[m >> 1]) : (T)0;
+                        zn[q][m] += (cc[q] & (1u << m)) ? cor : (T)0;
                     else
-                        zn[q][m] += scale * (own ? ea[q] : en[m >> 1]);
+                        zn[q][m] += cor;
                 }
             }
-        }
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            T zu;
+            T zu, s = ru[q];
             if (LIGHT<T>) {
                 if (!ok[q] || du[q] == (T)0) continue;
-                T s = ru[q];
 #pragma unroll
-                for (int a = 0; a < 3; a++) s += F.ct[a] * (zn[q][2 * a] + zn[q][2 * a + 1]);
+                for (int a = 0; a < 3; a++) s += ct[a] * (zn[q][2 * a] + zn[q][2 * a + 1]);
                 zu = s * du[q];
             } else {
                 if (!ok[q] || !(cc[q] & SELF)) continue;
-                T s = ru[q];
 #pragma unroll
-                for (int m = 0; m < 6; m++) s += (cc[q] & (1u << m)) ? F.ct[m >> 1] * zn[q][m] : (T)0;
-                zu = s / full_diag(cc[q], du[q], F.ct);
+                for (int m = 0; m < 6; m++) s += (cc[q] & (1u << m)) ? ct[m >> 1] * zn[q][m] : (T)0;
+                zu = s / full_diag(cc[q], du[q], ct);
             }
-            F.z[u[q]] = zu;
-            rz += ru[q] * zu;
-            zz += zu * zu;
+            z[u[q]] = zu;
+            if (MODE != PRE_BLACK) {
+                rz += ru[q] * zu;
+                zz += zu * zu;
+            }
         }
     }
-    rz_out += rz;
-    zz_out += zz;
+    return {rz, zz};
 }
 
-/* one half sweep of colour c on a coarse level; with C != null the
- * neighbours are read with C's correction added (per axis one neighbour
- * shares the node's aggregate, the other is in the next one).  Coordinates
- * come from the sweep index by float-estimated divisions (levels below 2^24
- * nodes). */
-template <typename T>
-__device__ void coarse_half(const MgLevel<T> &L, int c, bool whole, const MgLevel<T> *C, T scale) {
+/* one half sweep of colour c on level l (0: the first coarse one), by the
+ * grid or by block 0 on its own view; POST reads the neighbours with the next
+ * level's correction added (per axis one neighbour
+ * shares the node's aggregate, the other is in the next one) */
+template <typename T, bool POST>
+__device__ __forceinline__ void coarse_half(int l, int c, bool whole) {
+    const MgArgs<T> &A = whole ? shared_of<T>().A : shared_of<T>().B;
+    const MgLevel<T> L = A.L[l];
     const int hx = (L.nx + 1) / 2;
-    const int64_t count = (int64_t)hx * L.ny * L.nz;
     const int32_t offs[6] = {-1, 1, -L.nx, L.nx, -L.nx * L.ny, L.nx * L.ny};
-    const bool fast = count < (1 << 24);
     const float inv_hx = 1.f / (float)hx, inv_ny = 1.f / (float)L.ny;
-    const Span S = span(whole, count);
-    for (int64_t t = S.t; t < S.end; t += S.step) {
-        const uint32_t tt = (uint32_t)t;
-        uint32_t rr, kk;
-        if (fast) {
-            rr = div_small(tt, (uint32_t)hx, inv_hx);
-            kk = div_small(rr, (uint32_t)L.ny, inv_ny);
-        } else {
-            rr = tt / (uint32_t)hx;
-            kk = rr / (uint32_t)L.ny;
-        }
-        const int i2 = (int)(tt - rr * (uint32_t)hx);
+    const Span S = span(whole, (uint32_t)(hx * L.ny * L.nz));
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
+        const uint32_t rr = div_small(t, (uint32_t)hx, inv_hx);
+        const uint32_t kk = div_small(rr, (uint32_t)L.ny, inv_ny);
+        const int i2 = (int)(t - rr * (uint32_t)hx);
         const int j = (int)(rr - kk * (uint32_t)L.ny);
         const int k = (int)kk;
         const int i = 2 * i2 + ((j + k + c) & 1);
@@ -506,19 +513,24 @@ __device__ void coarse_half(const MgLevel<T> &L, int c, bool whole, const MgLeve
             wm[m] = L.w[m * L.n + I];
             en[m] = L.e[nb];
         }
-        if (C) {
-            const int A = ((k >> 1) * C->ny + (j >> 1)) * C->nx + (i >> 1);
+        if (POST) {
+            const MgLevel<T> *C = &A.L[l + 1];
+            const T scale = A.scale;
+            const int g = ((k >> 1) * C->ny + (j >> 1)) * C->nx + (i >> 1);
             /* the next aggregate along each axis; a neighbour off the level
              * has weight 0 and may read the node's own */
-            const int ax = (i & 1) ? (i + 1 < L.nx ? A + 1 : A) : (i > 0 ? A - 1 : A);
-            const int ay = (j & 1) ? (j + 1 < L.ny ? A + C->nx : A) : (j > 0 ? A - C->nx : A);
-            const int az = (k & 1) ? (k + 1 < L.nz ? A + C->nx * C->ny : A) : (k > 0 ? A - C->nx * C->ny : A);
-            const T ea = C->e[A];
+            const int ax = (i & 1) ? (i + 1 < L.nx ? g + 1 : g) : (i > 0 ? g - 1 : g);
+            const int ay = (j & 1) ? (j + 1 < L.ny ? g + C->nx : g) : (j > 0 ? g - C->nx : g);
+            const int az = (k & 1) ? (k + 1 < L.nz ? g + C->nx * C->ny : g) : (k > 0 ? g - C->nx * C->ny : g);
+            const T ea = C->e[g];
             const T ex[3] = {C->e[ax], C->e[ay], C->e[az]};
             const bool odd[3] = {(bool)(i & 1), (bool)(j & 1), (bool)(k & 1)};
 #pragma unroll
             for (int m = 0; m < 6; m++) en[m] += scale * (odd[m >> 1] != (bool)(m & 1) ? ea : ex[m >> 1]);
         }
+        pin(s);
+        pin(wm);
+        pin(en);
         if (d == (T)0) continue;
 #pragma unroll
         for (int m = 0; m < 6; m++) s += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
@@ -534,24 +546,24 @@ __device__ void coarse_half(const MgLevel<T> &L, int c, bool whole, const MgLeve
  * diagonal is read. */
 __device__ __forceinline__ int red_child(int q) { return q == 0 ? 0 : (q == 1 ? 3 : (q == 2 ? 5 : 6)); }
 
-/* Coordinates of coarse node I (float-estimated divisions below 2^24 nodes). */
+/* Coordinates of coarse node I. */
 template <typename T>
-__device__ __forceinline__ void coarse_coords(const MgLevel<T> &C, int64_t I, bool fast, float inv_nx, float inv_ny,
-                                              int &ci, int &cj, int &ck) {
-    const uint32_t I32 = (uint32_t)I;
-    const uint32_t cr = fast ? div_small(I32, (uint32_t)C.nx, inv_nx) : I32 / (uint32_t)C.nx;
-    const uint32_t ckk = fast ? div_small(cr, (uint32_t)C.ny, inv_ny) : cr / (uint32_t)C.ny;
-    ci = (int)(I32 - cr * (uint32_t)C.nx);
+__device__ __forceinline__ void coarse_coords(const MgLevel<T> &C, uint32_t I, float inv_nx, float inv_ny, int &ci,
+                                              int &cj, int &ck) {
+    const uint32_t cr = div_small(I, (uint32_t)C.nx, inv_nx);
+    const uint32_t ckk = div_small(cr, (uint32_t)C.ny, inv_ny);
+    ci = (int)(I - cr * (uint32_t)C.nx);
     cj = (int)(cr - ckk * (uint32_t)C.ny);
     ck = (int)ckk;
 }
 
 /* The sum of four lanes' residuals (lanes 4g..4g+3, in lane order) into
- * b of the coarse node, and the fused first red half sweep (e = b / diag).
- * Every lane of the warp calls it. */
+ * b of the coarse node, and the fused first red half sweep (e = b / diag; d:
+ * the node's diagonal, or LIGHT its reciprocal).  Every lane of the warp
+ * calls it. */
 template <typename T>
-__device__ __forceinline__ void restrict_store(const MgLevel<T> &C, bool valid, int64_t I, int ci, int cj, int ck,
-                                               T res) {
+__device__ __forceinline__ void restrict_store(const MgLevel<T> &C, bool valid, uint32_t I, int ci, int cj, int ck,
+                                               T res, T d) {
     const T r1 = __shfl_down_sync(0xffffffffu, res, 1);
     const T r2 = __shfl_down_sync(0xffffffffu, res, 2);
     const T r3 = __shfl_down_sync(0xffffffffu, res, 3);
@@ -562,10 +574,7 @@ __device__ __forceinline__ void restrict_store(const MgLevel<T> &C, bool valid, 
     sum += r2;
     sum += r3;
     C.b[I] = sum;
-    if (((ci + cj + ck) & 1) == 0) {
-        const T d = LIGHT<T> ? C.id[I] : C.diag[I];
-        if (d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
-    }
+    if (((ci + cj + ck) & 1) == 0 && d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
 }
 
 /* b of level 1 = sum of the node-grid children's residuals (r - J z).  When
@@ -581,7 +590,7 @@ template <typename T>
 struct FineChild {
     T id, r, dg, z, zn[6];
     uint16_t cc;
-    __device__ __forceinline__ void load(const Fine<T> &F, uint32_t u, bool in) {
+    __device__ __forceinline__ void load(const Fine<T> &F, int32_t sy, int32_t sz, uint32_t u, bool in) {
         if (LIGHT<T>) {
             id = in ? F.id[u] : (T)0;
         } else {
@@ -590,9 +599,17 @@ struct FineChild {
             dg = F.dg[u];
             z = F.z[u];
         }
-        const T *zu = F.z + u;
-#pragma unroll
-        for (int m = 0; m < 6; m++) zn[m] = zu[F.off[m]];
+        load_neighbours<T>(F.z, u, sy, sz, zn);
+    }
+    __device__ __forceinline__ void hold() {
+        if (LIGHT<T>) {
+            pin(id);
+        } else {
+            pin(r);
+            pin(dg);
+            pin(z);
+        }
+        pin(zn);
     }
     __device__ __forceinline__ T residual(const Fine<T> &F) const {
         if (LIGHT<T>) {
@@ -613,48 +630,61 @@ __device__ __forceinline__ uint32_t interior_or_safe(const Geo &g, int i, int j,
 }
 
 template <typename T>
-__device__ void restrict_fine(const Fine<T> &F, const MgLevel<T> &C) {
-    const Geo &g = F.g;
-    const bool fast = C.n < (1 << 24);
+__device__ __forceinline__ void restrict_fine() {
+    const Fine<T> &F = shared_of<T>().F;
+    const MgLevel<T> &C = shared_of<T>().A.L[0];
+    const Geo g = F.g;
+    const int32_t sy = g.ni, sz = g.ni * g.nj;
     const float inv_nx = 1.f / (float)C.nx, inv_ny = 1.f / (float)C.ny;
-    if (C.n > (int64_t)gridDim.x * blockDim.x) {
-        const Span S = span(true, C.n);
-        for (int64_t I = S.t; I < S.end; I += S.step) {
+    const T *__restrict__ diag = LIGHT<T> ? C.id : C.diag;
+    const uint32_t n = (uint32_t)C.n;
+    if (n > gridDim.x * blockDim.x) {
+        const Span S = span(true, n);
+#pragma unroll 1
+        for (uint32_t I = S.t; I < S.end; I += S.step) {
             int ci, cj, ck;
-            coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
+            coarse_coords(C, I, inv_nx, inv_ny, ci, cj, ck);
+            const T cd = diag[I];
             T sum = 0;
-            FineChild<T> ch[4];
+            /* two children at a time: four spill at 64 registers */
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int d = red_child(q);
-                bool in = true;
-                const uint32_t u =
-                    interior_or_safe(g, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), in);
-                ch[q].load(F, u, in);
+            for (int q0 = 0; q0 < 4; q0 += 2) {
+                FineChild<T> ch[2];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const int d = red_child(q0 + q);
+                    bool in = true;
+                    const uint32_t u =
+                        interior_or_safe(g, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), in);
+                    ch[q].load(F, sy, sz, u, in);
+                }
+                ch[0].hold();
+                ch[1].hold();
+#pragma unroll
+                for (int q = 0; q < 2; q++) sum += ch[q].residual(F);
             }
-#pragma unroll
-            for (int q = 0; q < 4; q++) sum += ch[q].residual(F);
             C.b[I] = sum;
-            if (((ci + cj + ck) & 1) == 0) {
-                const T d = LIGHT<T> ? C.id[I] : C.diag[I];
-                if (d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
-            }
+            if (((ci + cj + ck) & 1) == 0 && cd != (T)0) C.e[I] = LIGHT<T> ? sum * cd : sum / cd;
         }
         return;
     }
-    const int64_t total = 4 * C.n, padded = (total + 31) & ~(int64_t)31;
-    const Span S = span(true, padded);
-    for (int64_t t = S.t; t < S.end; t += S.step) {
+    const uint32_t total = 4 * n;
+    const Span S = span(true, (total + 31u) & ~31u);
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
         const bool valid = t < total;
-        const int64_t I = valid ? (t >> 2) : 0;
+        const uint32_t I = valid ? (t >> 2) : 0;
         int ci, cj, ck;
-        coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
+        coarse_coords(C, I, inv_nx, inv_ny, ci, cj, ck);
         const int d = red_child((int)(t & 3));
         bool in = valid;
         const uint32_t u = interior_or_safe(g, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), in);
         FineChild<T> ch;
-        ch.load(F, u, in);
-        restrict_store(C, valid, I, ci, cj, ck, ch.residual(F));
+        T cd = diag[I];
+        ch.load(F, sy, sz, u, in);
+        ch.hold();
+        pin(cd);
+        restrict_store(C, valid, I, ci, cj, ck, ch.residual(F), cd);
     }
 }
 
@@ -674,6 +704,8 @@ __device__ __forceinline__ T coarse_child_residual(const MgLevel<T> &L, int i, i
         wm[m] = L.w[m * L.n + u];
         en[m] = L.e[nb];
     }
+    pin(wm);
+    pin(en);
     if (!in || dd == (T)0) return (T)0;
     T res = LIGHT<T> ? (T)0 : bu - dd * eu;
 #pragma unroll
@@ -682,14 +714,19 @@ __device__ __forceinline__ T coarse_child_residual(const MgLevel<T> &L, int i, i
 }
 
 template <typename T>
-__device__ void restrict_coarse(const MgLevel<T> &L, const MgLevel<T> &C, bool whole) {
-    const bool fast = C.n < (1 << 24);
+__device__ __forceinline__ void restrict_coarse(int l, bool whole) {
+    const MgArgs<T> &A = whole ? shared_of<T>().A : shared_of<T>().B;
+    const MgLevel<T> &L = A.L[l], &C = A.L[l + 1];
     const float inv_nx = 1.f / (float)C.nx, inv_ny = 1.f / (float)C.ny;
-    if (C.n > (int64_t)(whole ? gridDim.x : 1u) * blockDim.x) {
-        const Span S = span(whole, C.n);
-        for (int64_t I = S.t; I < S.end; I += S.step) {
+    const T *__restrict__ diag = LIGHT<T> ? C.id : C.diag;
+    const uint32_t n = (uint32_t)C.n;
+    if (n > (whole ? gridDim.x : 1u) * blockDim.x) {
+        const Span S = span(whole, n);
+#pragma unroll 1
+        for (uint32_t I = S.t; I < S.end; I += S.step) {
             int ci, cj, ck;
-            coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
+            coarse_coords(C, I, inv_nx, inv_ny, ci, cj, ck);
+            const T cd = diag[I];
             T sum = 0;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -697,24 +734,24 @@ __device__ void restrict_coarse(const MgLevel<T> &L, const MgLevel<T> &C, bool w
                 sum += coarse_child_residual(L, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), true);
             }
             C.b[I] = sum;
-            if (((ci + cj + ck) & 1) == 0) {
-                const T d = LIGHT<T> ? C.id[I] : C.diag[I];
-                if (d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
-            }
+            if (((ci + cj + ck) & 1) == 0 && cd != (T)0) C.e[I] = LIGHT<T> ? sum * cd : sum / cd;
         }
         return;
     }
-    const int64_t total = 4 * C.n, padded = (total + 31) & ~(int64_t)31;
-    const Span S = span(whole, padded);
-    for (int64_t t = S.t; t < S.end; t += S.step) {
+    const uint32_t total = 4 * n;
+    const Span S = span(whole, (total + 31u) & ~31u);
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
         const bool valid = t < total;
-        const int64_t I = valid ? (t >> 2) : 0;
+        const uint32_t I = valid ? (t >> 2) : 0;
         int ci, cj, ck;
-        coarse_coords(C, I, fast, inv_nx, inv_ny, ci, cj, ck);
+        coarse_coords(C, I, inv_nx, inv_ny, ci, cj, ck);
         const int d = red_child((int)(t & 3));
+        T cd = diag[I];
+        pin(cd);
         const T res =
             coarse_child_residual(L, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), valid);
-        restrict_store(C, valid, I, ci, cj, ck, res);
+        restrict_store(C, valid, I, ci, cj, ck, res, cd);
     }
 }
 
@@ -724,8 +761,11 @@ __device__ void restrict_coarse(const MgLevel<T> &L, const MgLevel<T> &C, bool w
  * shuffle tree); the four quarter sums are added in order.  Every thread of
  * every block calls it (blocks of 128 threads or a multiple). */
 template <typename T>
-__device__ void dense_apply(const MgLevel<T> &L, const T *__restrict__ Ainv, int n) {
+__device__ __forceinline__ void dense_apply() {
     __shared__ T part[32];
+    const MgLevel<T> L = shared_of<T>().A.L[shared_of<T>().A.nlev - 1];
+    const T *__restrict__ Ainv = shared_of<T>().A.dense;
+    const int n = shared_of<T>().A.dense_n;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     constexpr int WPR = 4; /* warps per row */
     const int RPP = (int)(blockDim.x >> 5) / WPR; /* rows per pass */
@@ -756,18 +796,77 @@ __device__ void dense_apply(const MgLevel<T> &L, const T *__restrict__ Ainv, int
     }
 }
 
+/* The passes as calls (CALL) or inlined.  On large grids with 1024 threads the
+ * call gives a pass the 64 registers to itself (see SolveShared); with 512
+ * nothing spills, and inlining is quicker. */
+template <typename T, int MODE>
+__device__ __noinline__ Dots<T> fine_half_call() {
+    return fine_half<T, MODE, 2>();
+}
+template <typename T, bool POST>
+__device__ __noinline__ void coarse_half_call(int l, int c, bool whole) {
+    coarse_half<T, POST>(l, c, whole);
+}
+template <typename T>
+__device__ __noinline__ void restrict_fine_call() {
+    restrict_fine<T>();
+}
+template <typename T>
+__device__ __noinline__ void restrict_coarse_call(int l, bool whole) {
+    restrict_coarse<T>(l, whole);
+}
+template <typename T>
+__device__ __noinline__ void dense_apply_call() {
+    dense_apply<T>();
+}
+
+template <typename T, bool CALL>
+struct Pass {
+    template <int MODE>
+    static __device__ __forceinline__ Dots<T> fine() {
+        return CALL ? fine_half_call<T, MODE>() : fine_half<T, MODE, 2>();
+    }
+    template <bool POST>
+    static __device__ __forceinline__ void coarse(int l, int c, bool whole) {
+        if (CALL)
+            coarse_half_call<T, POST>(l, c, whole);
+        else
+            coarse_half<T, POST>(l, c, whole);
+    }
+    static __device__ __forceinline__ void restrict_to_first() {
+        if (CALL)
+            restrict_fine_call<T>();
+        else
+            restrict_fine<T>();
+    }
+    static __device__ __forceinline__ void restrict_from(int l, bool whole) {
+        if (CALL)
+            restrict_coarse_call<T>(l, whole);
+        else
+            restrict_coarse<T>(l, whole);
+    }
+    static __device__ __forceinline__ void dense() {
+        if (CALL)
+            dense_apply_call<T>();
+        else
+            dense_apply<T>();
+    }
+};
+
 /* The V-cycle z = M r after its first red half sweep on the node grid
  * (done by the caller, fused with the CG update of r).  Every block executes
  * the same grid barriers; returns the grid-wide r.z of the final z and puts
  * z.z in zz (the last barrier is the one of that reduction). */
-template <typename T>
-__device__ double vcycle_rest(cg::grid_group &grid, const Fine<T> &F, const MgArgs<T> &A, double *partials,
-                              int &round, double &zz, const MgArgs<T> *SB) {
+template <typename T, bool CALL>
+__device__ __forceinline__ double vcycle_rest(cg::grid_group &grid, double *partials, int &round, double &zz) {
+    using P = Pass<T, CALL>;
+    const MgArgs<T> &A = shared_of<T>().A;
+    const Fine<T> &F = shared_of<T>().F;
     const int NL = A.nlev;
     if (NL == 0) { /* Jacobi: the caller computed z on every node */
         T rz = 0, z2 = 0;
         int64_t nn = (int64_t)F.g.ni * F.g.nj * F.g.nk;
-        const Span S = span(true, nn);
+        const Span S = span(true, (uint32_t)nn);
         for (int64_t u = S.t; u < S.end; u += S.step)
             if (F.code[u] & SELF) {
                 T zu = F.z[u];
@@ -776,22 +875,20 @@ __device__ double vcycle_rest(cg::grid_group &grid, const Fine<T> &F, const MgAr
             }
         const T vt[2] = {rz, z2};
         double v[2];
-        grid_sum_t<2, T>(grid, vt, v, partials, round);
+        grid_sum<2, T>(grid, vt, v, partials, round);
         zz = v[1];
         return v[0];
     }
     const int GL = A.grid_levels;
-    const T sc = A.scale;
-    T rz = 0, z2 = 0, rz_unused = 0, z2_unused = 0;
-    fine_half(F, 1, (const MgLevel<T> *)nullptr, sc, rz_unused, z2_unused);
+    P::template fine<PRE_BLACK>();
     grid.sync();
-    restrict_fine(F, A.L[0]);
+    P::restrict_to_first();
     grid.sync();
     int l = 1; /* level l lives in A.L[l-1] and its red half was fused */
     for (; l < GL && l < NL; l++) {
-        coarse_half(A.L[l - 1], 1, true, (const MgLevel<T> *)nullptr, sc);
+        P::template coarse<false>(l - 1, 1, true);
         grid.sync();
-        restrict_coarse(A.L[l - 1], A.L[l], true);
+        P::restrict_from(l - 1, true);
         grid.sync();
     }
     const int lblock = l;
@@ -800,10 +897,10 @@ __device__ double vcycle_rest(cg::grid_group &grid, const Fine<T> &F, const MgAr
     if (!coarsest_whole) {
         if (blockIdx.x == 0) {
             /* with shared-memory levels, stage b and e of the first one */
-            const bool staged = SB && SB->smem_from == lblock - 1;
-            const MgArgs<T> &B = staged ? *SB : A;
+            const MgArgs<T> &B = shared_of<T>().B;
+            const bool staged = B.smem_from >= 0 && B.smem_from == lblock - 1;
             if (staged) {
-                const MgLevel<T> &G0 = A.L[lblock - 1], &S0 = SB->L[lblock - 1];
+                const MgLevel<T> &G0 = A.L[lblock - 1], &S0 = B.L[lblock - 1];
                 for (int64_t t = threadIdx.x; t < G0.n; t += blockDim.x) {
                     S0.b[t] = G0.b[t];
                     S0.e[t] = G0.e[t];
@@ -811,71 +908,69 @@ __device__ double vcycle_rest(cg::grid_group &grid, const Fine<T> &F, const MgAr
                 __syncthreads();
             }
             for (int b = lblock; b < NL; b++) {
-                coarse_half(B.L[b - 1], 1, false, (const MgLevel<T> *)nullptr, sc);
+                P::template coarse<false>(b - 1, 1, false);
                 __syncthreads();
-                restrict_coarse(B.L[b - 1], B.L[b], false);
+                P::restrict_from(b - 1, false);
                 __syncthreads();
             }
-            const MgLevel<T> &Lc = B.L[NL - 1];
             for (int s = 0; s < nuc; s++) {
                 if (s) {
-                    coarse_half(Lc, 0, false, (const MgLevel<T> *)nullptr, sc);
+                    P::template coarse<false>(NL - 1, 0, false);
                     __syncthreads();
                 }
-                coarse_half(Lc, 1, false, (const MgLevel<T> *)nullptr, sc);
+                P::template coarse<false>(NL - 1, 1, false);
                 __syncthreads();
             }
             for (int s = 0; s < nuc; s++) {
-                coarse_half(Lc, 1, false, (const MgLevel<T> *)nullptr, sc);
+                P::template coarse<false>(NL - 1, 1, false);
                 __syncthreads();
-                coarse_half(Lc, 0, false, (const MgLevel<T> *)nullptr, sc);
+                P::template coarse<false>(NL - 1, 0, false);
                 __syncthreads();
             }
             for (int b = NL - 1; b >= lblock; b--) {
-                coarse_half(B.L[b - 1], 1, false, &B.L[b], sc);
+                P::template coarse<true>(b - 1, 1, false);
                 __syncthreads();
-                coarse_half(B.L[b - 1], 0, false, (const MgLevel<T> *)nullptr, sc);
+                P::template coarse<false>(b - 1, 0, false);
                 __syncthreads();
             }
             if (staged) {
-                const MgLevel<T> &G0 = A.L[lblock - 1], &S0 = SB->L[lblock - 1];
+                const MgLevel<T> &G0 = A.L[lblock - 1], &S0 = B.L[lblock - 1];
                 for (int64_t t = threadIdx.x; t < G0.n; t += blockDim.x) G0.e[t] = S0.e[t];
             }
         }
         grid.sync();
     } else if (A.dense && *A.dense_ok) {
-        dense_apply(A.L[NL - 1], A.dense, A.dense_n);
+        P::dense();
         grid.sync();
     } else {
-        const MgLevel<T> &Lc = A.L[NL - 1];
         for (int s = 0; s < nuc; s++) {
             if (s) {
-                coarse_half(Lc, 0, true, (const MgLevel<T> *)nullptr, sc);
+                P::template coarse<false>(NL - 1, 0, true);
                 grid.sync();
             }
-            coarse_half(Lc, 1, true, (const MgLevel<T> *)nullptr, sc);
+            P::template coarse<false>(NL - 1, 1, true);
             grid.sync();
         }
         for (int s = 0; s < nuc; s++) {
-            coarse_half(Lc, 1, true, (const MgLevel<T> *)nullptr, sc);
+            P::template coarse<false>(NL - 1, 1, true);
             grid.sync();
-            coarse_half(Lc, 0, true, (const MgLevel<T> *)nullptr, sc);
+            P::template coarse<false>(NL - 1, 0, true);
             grid.sync();
         }
     }
     const int top = coarsest_whole ? NL - 1 : lblock - 1;
     for (int b = top; b >= 1; b--) {
-        coarse_half(A.L[b - 1], 1, true, &A.L[b], sc);
+        P::template coarse<true>(b - 1, 1, true);
         grid.sync();
-        coarse_half(A.L[b - 1], 0, true, (const MgLevel<T> *)nullptr, sc);
+        P::template coarse<false>(b - 1, 0, true);
         grid.sync();
     }
-    fine_half(F, 1, &A.L[0], sc, rz, z2);
+    const Dots<T> db = P::template fine<POST_BLACK>();
     grid.sync();
-    fine_half(F, 0, (const MgLevel<T> *)nullptr, sc, rz, z2);
-    const T vt[2] = {rz, z2};
+    const Dots<T> dr = P::template fine<POST_RED>();
+    const T vt[2] = {db.rz + dr.rz, db.zz + dr.zz};
     double v[2];
-    grid_sum_t<2, T>(grid, vt, v, partials, round);
+    grid_sum<2, T>(grid, vt, v, partials, round);
     zz = v[1];
     return v[0];
 }
@@ -893,15 +988,15 @@ __device__ __noinline__ void df_prepass(const double *__restrict__ phi, const do
                                         int predict, dfl d_inv_eps0, int64_t nn, Span S) {
     /* four nodes a pass, every load before any store (the pass is bound by
      * the loads in flight) */
-    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
+    for (uint32_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         double cur[4], prev[4], prev2[4], rh[4];
         uint16_t c[4];
         bool on[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * S.step;
+            const uint32_t u = u0 + h * S.step;
             on[h] = u < S.end;
-            const int64_t v = on[h] ? u : 0;
+            const uint32_t v = on[h] ? u : 0;
             cur[h] = phi[v];
             rh[h] = rho[v];
             c[h] = predict >= 2 ? code[v] : (uint16_t)0;
@@ -911,7 +1006,7 @@ __device__ __noinline__ void df_prepass(const double *__restrict__ phi, const do
 #pragma unroll
         for (int h = 0; h < 4; h++) {
             if (!on[h]) continue;
-            const int64_t u = u0 + h * S.step;
+            const uint32_t u = u0 + h * S.step;
             dfl x = df_split(cur[h]);
             if (predict) {
                 if (predict >= 2 && (c[h] & SELF)) {
@@ -939,14 +1034,14 @@ __device__ __noinline__ float df_update(const uint16_t *__restrict__ code, const
                                         Span S) {
     float yys = 0.f;
     /* four nodes a pass, every load before any store */
-    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
+    for (uint32_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         uint16_t c[4];
         float yu[4];
         float2 x[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * S.step;
-            const int64_t v = u < S.end ? u : 0;
+            const uint32_t u = u0 + h * S.step;
+            const uint32_t v = u < S.end ? u : 0;
             c[h] = u < S.end ? code[v] : (uint16_t)0;
             yu[h] = (float)yv[v];
             x[h] = phf[v];
@@ -965,12 +1060,12 @@ __device__ __noinline__ float df_update(const uint16_t *__restrict__ code, const
  * a pass with every load before any store */
 __device__ __noinline__ void df_rebuild(const uint16_t *__restrict__ code, const float2 *__restrict__ phf,
                                         double *phi, Span S) {
-    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
+    for (uint32_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         uint16_t c[4];
         float2 x[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * S.step;
+            const uint32_t u = u0 + h * S.step;
             c[h] = u < S.end ? code[u] : (uint16_t)0;
             x[h] = phf[u < S.end ? u : 0];
         }
@@ -984,11 +1079,11 @@ __device__ __noinline__ void df_rebuild(const uint16_t *__restrict__ code, const
  * chains end at unknowns or Dirichlet nodes, which this pass does not
  * write), four nodes a pass */
 __device__ __noinline__ void neumann_copies(const int32_t *__restrict__ target, double *phi, Span S) {
-    for (int64_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
+    for (uint32_t u0 = S.t; u0 < S.end; u0 += 4 * S.step) {
         int32_t t[4];
 #pragma unroll
         for (int h = 0; h < 4; h++) {
-            const int64_t u = u0 + h * S.step;
+            const uint32_t u = u0 + h * S.step;
             t[h] = u < S.end ? target[u] : -1;
         }
 #pragma unroll
@@ -1016,13 +1111,13 @@ __device__ __noinline__ float df_residual(const uint16_t *__restrict__ code, con
     /* two nodes a pass, every load before the arithmetic; a node that is
      * not an unknown reads the interior node safe_u and stores nothing */
     const int64_t safe_u = (int64_t)s2 + s1 + 1;
-    for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+    for (uint32_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
         uint16_t cq[2];
         int64_t uq[2];
         float2 xq[2], pq[2][6], bq[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int64_t u = u0 + h * S.step;
+            const uint32_t u = u0 + h * S.step;
             cq[h] = u < S.end ? code[u] : (uint16_t)0;
             uq[h] = (cq[h] & SELF) ? u : safe_u;
         }
@@ -1071,14 +1166,147 @@ __device__ __noinline__ float df_residual(const uint16_t *__restrict__ code, con
     return ffs;
 }
 
-template <typename T, int THREADS>
+/* p = z + beta p (on the fly at the node and its neighbours) and q = J p;
+ * returns the thread's sum of p q.  old: there is a previous p.  LIGHT: J p
+ * = J z + beta J p_old, the last q instead of p's neighbours (10 float64
+ * instructions a node, 28 with p formed at seven nodes).  PER nodes per pass,
+ * every load before any store; the loads do not wait for the code word (a
+ * plane of padding around the vectors takes a boundary node's missing
+ * neighbours, a node past the end reads node 0); a node that is not an
+ * unknown stores nothing. */
+template <typename T, int PER>
+__device__ __forceinline__ T pcg_direction(const T *__restrict__ pold, T *__restrict__ pnew, T *__restrict__ q,
+                                           T beta, bool old) {
+    const Fine<T> &F = shared_of<T>().F;
+    const uint16_t *__restrict__ code = F.code;
+    const T *__restrict__ z = F.z, *__restrict__ dg = F.dg;
+    const T ct[3] = {F.ct[0], F.ct[1], F.ct[2]};
+    const int32_t sy = F.g.ni, sz = F.g.ni * F.g.nj;
+    const Span S = span(true, F.nn);
+    T pq = 0;
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += PER * S.step) {
+        uint32_t u[PER];
+        uint16_t c[PER];
+        T zc[PER], pc[PER], dB[PER], zn[PER][6], pn[PER][6];
+#pragma unroll
+        for (int h = 0; h < PER; h++) {
+            const bool in = t + h * S.step < S.end;
+            u[h] = in ? t + h * S.step : 0u;
+            c[h] = in ? code[u[h]] : (uint16_t)0;
+            zc[h] = z[u[h]];
+            dB[h] = dg[u[h]];
+            load_neighbours(z, u[h], sy, sz, zn[h]);
+            pc[h] = old ? pold[u[h]] : (T)0;
+            if (LIGHT<T>) {
+                pn[h][0] = old ? q[u[h]] : (T)0;
+            } else if (old) {
+                load_neighbours(pold, u[h], sy, sz, pn[h]);
+            } else {
+#pragma unroll
+                for (int m = 0; m < 6; m++) pn[h][m] = (T)0;
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < PER; h++) {
+            pin(zc[h]);
+            pin(pc[h]);
+            pin(dB[h]);
+            pin(zn[h]);
+            if (LIGHT<T>)
+                pin(pn[h][0]);
+            else
+                pin(pn[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < PER; h++) {
+            if (!(c[h] & SELF)) continue;
+            const T pu = zc[h] + beta * pc[h];
+            T s;
+            if (LIGHT<T>) {
+                s = dB[h] * zc[h];
+#pragma unroll
+                for (int a = 0; a < 3; a++) s -= ct[a] * (zn[h][2 * a] + zn[h][2 * a + 1]);
+                s += beta * pn[h][0];
+            } else {
+#pragma unroll
+                for (int m = 0; m < 6; m++) pn[h][m] = zn[h][m] + beta * pn[h][m];
+                s = jacobian_apply(c[h], dB[h], ct, pu, pn[h]);
+            }
+            pnew[u[h]] = pu;
+            q[u[h]] = s;
+            pq += pu * s;
+        }
+    }
+    return pq;
+}
+
+/* y += alpha p, r -= alpha q, and the first red half sweep of the
+ * preconditioner; returns the thread's sum of r^2 */
+template <typename T>
+__device__ __forceinline__ T pcg_update(T *__restrict__ y, const T *__restrict__ p, const T *__restrict__ q, T alpha) {
+    const Fine<T> &F = shared_of<T>().F;
+    const uint16_t *__restrict__ code = F.code;
+    T *__restrict__ z = F.z, *__restrict__ r = F.r;
+    const T *__restrict__ dd = LIGHT<T> ? F.id : F.dg;
+    const T ct[3] = {F.ct[0], F.ct[1], F.ct[2]};
+    const bool jacobi = shared_of<T>().A.nlev == 0;
+    const Span S = span(true, F.nn);
+    T rr = 0;
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += 2 * S.step) {
+        uint32_t u[2];
+        uint16_t c[2];
+        T yv[2], pv[2], rv[2], qv[2], dv[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const bool in = t + h * S.step < S.end;
+            u[h] = in ? t + h * S.step : 0u;
+            c[h] = in ? code[u[h]] : (uint16_t)0;
+            yv[h] = y[u[h]];
+            pv[h] = p[u[h]];
+            rv[h] = r[u[h]];
+            qv[h] = q[u[h]];
+            dv[h] = dd[u[h]];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            pin(yv[h]);
+            pin(pv[h]);
+            pin(rv[h]);
+            pin(qv[h]);
+            pin(dv[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (!(c[h] & SELF)) continue;
+            y[u[h]] = yv[h] + alpha * pv[h];
+            const T ru = rv[h] - alpha * qv[h];
+            r[u[h]] = ru;
+            rr += ru * ru;
+            if (jacobi || !(c[h] & BLACK))
+                z[u[h]] = LIGHT<T> ? ru * dv[h] : ru / full_diag(c[h], dv[h], ct);
+        }
+    }
+    return rr;
+}
+
+template <typename T>
+__device__ __noinline__ T pcg_direction_call(const T *pold, T *pnew, T *q, T beta, bool old) {
+    return pcg_direction<T, 2>(pold, pnew, q, beta, old);
+}
+template <typename T>
+__device__ __noinline__ T pcg_update_call(T *y, const T *p, const T *q, T alpha) {
+    return pcg_update<T>(y, p, q, alpha);
+}
+
+template <typename T, int THREADS, bool CALL>
 __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, const double *__restrict__ rho,
                                                         const uint16_t *__restrict__ code,
                                                         const int32_t *__restrict__ target, double phi0,
                                                         double te0, double n0, int nr_max, double nr_tol,
                                                         int pcg_max, double pcg_tol, T *y, T *r, T *z, T *p0,
-                                                        T *p1, T *q, T *dg, T *id, MgArgs<T> mg, const int32_t *lists,
-                                                        double *partials, SolveStatus *st, int *err,
+                                                        T *p1, T *q, T *dg, T *id, MgArgs<T> mg, double *partials, SolveStatus *st, int *err,
                                                         double *lin_y, const double *__restrict__ lin_b,
                                                         int gs_max, double gs_tol, float2 *dfbuf, double *phi_prev,
                                                         int predict, Coef3<T> ctp) {
@@ -1086,15 +1314,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
     extern __shared__ __align__(16) unsigned char pcg_smem[];
     __shared__ T bc_alpha, bc_beta;
     __shared__ int bc_stop;
-    __shared__ MgArgs<T> smem_args;
-    const MgArgs<T> *SB = nullptr;
-    if (mg.smem_from >= 0 && mg.nlev > 0 && blockIdx.x == 0) {
-        smem_levels_init(mg, smem_args, pcg_smem);
-        SB = &smem_args;
-    }
     const int64_t nn = (int64_t)g.ni * g.nj * g.nk;
     const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    const int32_t off[6] = {-1, 1, -(int32_t)sy, (int32_t)sy, -(int32_t)sz, (int32_t)sz};
+    const int64_t off[6] = {-1, 1, -sy, sy, -sz, sz};
     const int64_t safe = sz + sy + 1; /* the interior node (1,1,1) */
     const double cd[3] = {1.0 / (g.dh[0] * g.dh[0]), 1.0 / (g.dh[1] * g.dh[1]), 1.0 / (g.dh[2] * g.dh[2])};
     /* (T)cd from the host: derived here from cd, the compiler re-derived it
@@ -1105,22 +1327,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
     const double A0 = PCG_QE * n0 / PCG_EPS_0;
     const double inv_te0 = 1.0 / te0, A0_te0 = A0 / te0, inv_eps0 = 1.0 / PCG_EPS_0;
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const Span S = span(true, nn); /* this thread's nodes */
+    const Span S = span(true, (uint32_t)nn); /* this thread's nodes */
     const bool jacobi = mg.nlev == 0;
     Fine<T> F;
     F.g = g;
     F.code = code;
     for (int m = 0; m < 3; m++) F.ct[m] = ct[m];
-    for (int m = 0; m < 6; m++) F.off[m] = off[m];
+    F.nn = (uint32_t)nn;
     F.dg = dg;
     F.id = id;
     F.r = r;
     F.z = z;
-    F.nlist = (int32_t)((int64_t)((g.ni - 1) / 2) * (g.nj - 2) * (g.nk - 2));
-    F.list[0] = lists;
-    F.pk[0] = lists + F.nlist;
-    F.list[1] = lists + 2 * (int64_t)F.nlist;
-    F.pk[1] = lists + 3 * (int64_t)F.nlist;
+    F.ncolour = (uint32_t)((g.ni - 1) / 2) * (uint32_t)(g.nj - 2) * (uint32_t)(g.nk - 2);
+    shared_init(F, mg, pcg_smem);
     int round = 0, nr, conv = 0, inner = 0, fallback = 0;
     double norm = 0;
     /* linear mode (lin_y != null): Newton on F(y) = J y - b with J frozen at
@@ -1161,7 +1380,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
          * wait for the code word (neighbour indices are clamped into the
          * grid, a node past the end reads the interior node (1,1,1)), and
          * a node that is not an unknown stores nothing */
-        for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+        for (uint32_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
             const int64_t uq[2] = {u0, u0 + S.step};
             bool onq[2];
             uint16_t c[2];
@@ -1241,8 +1460,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
                 ff += Fv * Fv;
             }
         }
-        double s1[1] = {ff};
-        grid_sum_n<1>(grid, s1, partials, round);
+        const double t1[1] = {ff};
+        double s1[1];
+        grid_sum<1, double>(grid, t1, s1, partials, round);
         double FF = s1[0];
         if (!isfinite(FF)) {
             if (gtid == 0) atomicOr(err, DERR_NONFINITE);
@@ -1252,7 +1472,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
         if (FF > 0) {
             const double stop2 = pcg_tol * pcg_tol * FF;
             double ZZ;
-            double RZ = vcycle_rest(grid, F, mg, partials, round, ZZ, SB);
+            double RZ = vcycle_rest<T, CALL>(grid, partials, round, ZZ);
             /* the first preconditioned residual already estimates an update
              * below the inner stop: it is the update */
             take_z = ZZ < zz_stop;
@@ -1260,112 +1480,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
             T beta = 0;
             T *pold = p0, *pnew = p1;
             for (int it = 0; it < pcg_max && !take_z; it++) {
-                /* p = z + beta p (on the fly at the node and its neighbours),
-                 * q = J p */
-                T pq = 0;
-                /* two nodes per pass, every load before any store; the loads
-                 * do not wait for the code word (a plane of padding around
-                 * the vectors takes a boundary node's missing neighbours, a
-                 * node past the end reads the interior node (1,1,1)); a node
-                 * that is not an unknown stores nothing */
-                for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
-                    const int64_t uq[2] = {u0, u0 + S.step};
-                    bool on[2];
-                    uint16_t c[2];
-                    int64_t u[2];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        c[h] = uq[h] < S.end ? code[uq[h]] : (uint16_t)0;
-                        on[h] = c[h] & SELF;
-                        u[h] = uq[h] < S.end ? uq[h] : safe;
-                    }
-                    /* an unknown is interior: neighbour loads need no code bit */
-                    T zc[2], pc[2], dB[2], zn[2][6], pn[2][6];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        zc[h] = z[u[h]];
-                        pc[h] = it ? pold[u[h]] : (T)0;
-                        dB[h] = dg[u[h]];
-#pragma unroll
-                        for (int m = 0; m < 6; m++) zn[h][m] = z[u[h] + off[m]];
-                        if (LIGHT<T>) {
-                            pn[h][0] = it ? q[u[h]] : (T)0;
-                        } else {
-#pragma unroll
-                            for (int m = 0; m < 6; m++) pn[h][m] = it ? pold[u[h] + off[m]] : (T)0;
-                        }
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        if (!on[h]) continue;
-                        if (LIGHT<T>) {
-                            /* J p = J z + beta J p_old: the last q instead of
-                             * p's neighbours (10 float64 instructions, 28
-                             * with p formed at seven nodes) */
-                            T s = dB[h] * zc[h];
-#pragma unroll
-                            for (int a = 0; a < 3; a++) s -= ct[a] * (zn[h][2 * a] + zn[h][2 * a + 1]);
-                            s += beta * pn[h][0];
-                            const T pl = zc[h] + beta * pc[h];
-                            pnew[u[h]] = pl;
-                            q[u[h]] = s;
-                            pq += pl * s;
-                            continue;
-                        }
-                        T pu = zc[h] + beta * pc[h];
-#pragma unroll
-                        for (int m = 0; m < 6; m++) pn[h][m] = zn[h][m] + beta * pn[h][m];
-                        T s = jacobian_apply(c[h], dB[h], ct, pu, pn[h]);
-                        pnew[u[h]] = pu;
-                        q[u[h]] = s;
-                        pq += pu * s;
-                    }
-                }
+                const T pq = CALL ? pcg_direction_call<T>(pold, pnew, q, beta, it > 0)
+                                  : pcg_direction<T, 2>(pold, pnew, q, beta, it > 0);
                 const T t3[1] = {pq};
                 double s3[1];
-                grid_sum_t<1, T>(grid, t3, s3, partials, round);
+                grid_sum<1, T>(grid, t3, s3, partials, round);
                 /* block-uniform scalars are computed by one thread and
                  * broadcast: 32 warps each dividing in float64 would queue
                  * on the narrow float64 pipe */
                 if (threadIdx.x == 0) bc_alpha = (T)(RZ / s3[0]);
                 __syncthreads();
                 const T alpha = bc_alpha;
-                /* y += alpha p, r -= alpha q, and the first red half sweep */
-                T rr = 0;
-                for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
-                    const int64_t uq[2] = {u0, u0 + S.step};
-                    bool on[2];
-                    uint16_t c[2];
-                    int64_t u[2];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        c[h] = uq[h] < S.end ? code[uq[h]] : (uint16_t)0;
-                        on[h] = c[h] & SELF;
-                        u[h] = uq[h] < S.end ? uq[h] : safe;
-                    }
-                    T yv[2], pv[2], rv[2], qv[2], dv[2];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        yv[h] = y[u[h]];
-                        pv[h] = pnew[u[h]];
-                        rv[h] = r[u[h]];
-                        qv[h] = q[u[h]];
-                        dv[h] = LIGHT<T> ? id[u[h]] : dg[u[h]];
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        if (!on[h]) continue;
-                        y[u[h]] = yv[h] + alpha * pv[h];
-                        T ru = rv[h] - alpha * qv[h];
-                        r[u[h]] = ru;
-                        rr += ru * ru;
-                        if (jacobi || !(c[h] & BLACK)) 
-                            z[u[h]] = LIGHT<T> ? ru * dv[h] : ru / full_diag(c[h], dv[h], ct);
-                    }
-                }
+                const T rr = CALL ? pcg_update_call<T>(y, pnew, q, alpha) : pcg_update<T>(y, pnew, q, alpha);
                 const T t4[1] = {rr};
                 double s4[1];
-                grid_sum_t<1, T>(grid, t4, s4, partials, round);
+                grid_sum<1, T>(grid, t4, s4, partials, round);
                 inner++;
                 if (threadIdx.x == 0) bc_stop = !(s4[0] > stop2); /* also leaves on NaN */
                 __syncthreads();
@@ -1373,7 +1502,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
                     inner_ok = true;
                     break;
                 }
-                double RZn = vcycle_rest(grid, F, mg, partials, round, ZZ, SB);
+                double RZn = vcycle_rest<T, CALL>(grid, partials, round, ZZ);
                 /* z = M r estimates the remaining error of y: once its RMS is
                  * below half the Newton tolerance, further inner
                  * iterations cannot change the outcome of the Newton test */
@@ -1438,7 +1567,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
                         }
                         const T t5[1] = {rr2};
                         double s5[1];
-                        grid_sum_t<1, T>(grid, t5, s5, partials, round);
+                        grid_sum<1, T>(grid, t5, s5, partials, round);
                         if (threadIdx.x == 0) bc_stop = sqrt(s5[0] / (double)nn) < gs_tol;
                         __syncthreads();
                         if (bc_stop) break;
@@ -1456,7 +1585,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
             yy = (double)df_update<T>(code, take_z ? z : y, phf, S);
         } else
         /* two nodes per pass, loads ahead of the code test and the stores */
-        for (int64_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
+        for (uint32_t u0 = S.t; u0 < S.end; u0 += 2 * S.step) {
             const int64_t uq[2] = {u0, u0 + S.step};
             int64_t u[2];
             uint16_t c[2];
@@ -1477,8 +1606,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_newton_pcg(Geo g, double *phi, c
                 yy += yu * yu;
             }
         }
-        double s6[1] = {yy};
-        grid_sum_n<1>(grid, s6, partials, round);
+        const double t6[1] = {yy};
+        double s6[1];
+        grid_sum<1, double>(grid, t6, s6, partials, round);
         norm = sqrt(s6[0] / (double)nn);
         if (!isfinite(norm)) {
             if (gtid == 0) atomicOr(err, DERR_NONFINITE);
@@ -1716,7 +1846,7 @@ static size_t mg_layout(World &w, MgArgs<T> &A, char *base) {
 
 template <typename T>
 static int run_pcg(World &w) {
-    /* the colour lists pack coordinates in 10 + 10 + 11 bits */
+    /* node indices fit 32 bits, and a row index 2^21 (div_small) */
     if (w.g.ni > 1024 || w.g.nj > 1024 || w.g.nk > 2048) return (int)cudaErrorInvalidValue;
     size_t es = sizeof(T);
     /* a plane of padding on both sides of each vector, so that reads of a
@@ -1726,14 +1856,9 @@ static int run_pcg(World &w) {
     size_t codeb = ((w.nn * sizeof(uint16_t) + 255) / 256) * 256;
     MgArgs<T> A;
     size_t mgb = mg_layout<T>(w, A, nullptr);
-    int64_t nlist = (int64_t)((w.g.ni - 1) / 2) * (w.g.nj - 2) * (w.g.nk - 2);
-    /* the colour lists are only read when the sweeps cannot enumerate their
-     * nodes arithmetically (2^24 entries or more, see fine_half) */
-    const bool need_lists = nlist >= (1 << 24);
-    size_t listb = need_lists ? ((4 * nlist * sizeof(int32_t) + 255) / 256) * 256 : 0;
     /* float inner solves: the (hi, lo) pairs of phi and rho / eps0 */
     size_t dfb = sizeof(T) == sizeof(float) ? 2 * (((size_t)w.nn * sizeof(float2) + 255) / 256) * 256 : 0;
-    size_t need = 8 * vec + codeb + mgb + listb + dfb;
+    size_t need = 8 * vec + codeb + mgb + dfb;
     if (w.pcg_bytes < need || w.pcg_elem != (int)es) {
         if (w.pcg_buf) {
             cudaStreamSynchronize(w.stream);
@@ -1749,18 +1874,12 @@ static int run_pcg(World &w) {
     }
     char *base = (char *)w.pcg_buf;
     uint16_t *code = (uint16_t *)(base + 8 * vec);
-    int32_t *lists = (int32_t *)(base + 8 * vec + codeb + mgb);
     mg_layout<T>(w, A, base + 8 * vec + codeb);
     if (!w.pcg_codes_valid) {
         /* the sweeps rely on zeros off the unknowns, which just changed */
         cudaMemsetAsync(base, 0, 8 * vec, w.stream);
         k_pcg_codes<<<blocks_for(w.nn, 256), 256, 0, w.stream>>>(w.g, w.obj, code);
         w.nlaunch++;
-        for (int c = 0; c < 2 && need_lists; c++) {
-            k_pcg_lists<<<blocks_for(nlist, 256), 256, 0, w.stream>>>(w.g, c, lists + 2 * c * nlist,
-                                                                      lists + (2 * c + 1) * nlist);
-            w.nlaunch++;
-        }
         for (int l = 0; l < A.nlev; l++) {
             MgLevel<T> prev = l ? A.L[l - 1] : A.L[0];
             k_mg_setup<T><<<blocks_for(A.L[l].n, 256), 256, 0, w.stream>>>(w.g, code, prev, A.L[l], l == 0);
@@ -1793,7 +1912,12 @@ static int run_pcg(World &w) {
      * nodes and so the same dot products; float64: up to 2^20 nodes */
     const bool small = sizeof(T) == sizeof(float) ? w.nn <= (int64_t)PCG_THREADS_SMALL * w.sm_count : w.nn <= 1 << 20;
     const int threads = small ? PCG_THREADS_SMALL : PCG_THREADS;
-    const void *fn = small ? (const void *)k_newton_pcg<T, PCG_THREADS_SMALL> : (const void *)k_newton_pcg<T, PCG_THREADS>;
+    const void *fn = (const void *)k_newton_pcg<T, PCG_THREADS, true>;
+    if (small) fn = (const void *)k_newton_pcg<T, PCG_THREADS_SMALL, false>;
+    /* between: the passes inlined (64x64x128 float sphere step: 1.09 ms, 1.12
+     * as calls; 256x256x512: 25.7 ms inlined, 24.9 as calls) */
+    if constexpr (sizeof(T) == sizeof(float))
+        if (!small && w.nn <= 1 << 21) fn = (const void *)k_newton_pcg<T, PCG_THREADS, false>;
     size_t dyn = 0;
     if (A.smem_from >= 0)
         for (int i = A.smem_from; i < A.nlev; i++) dyn += level_smem_bytes<T>(A.L[i].n);
@@ -1822,13 +1946,12 @@ static int run_pcg(World &w) {
     double *part = w.d_partials;
     SolveStatus *st = w.d_status;
     int *err = w.d_err;
-    const int32_t *lst = lists;
     double *ly = w.lin_y;
     const double *lb = w.lin_b;
     int gs_max = w.gs_fallback ? w.max_it : 0;
     double gs_tol = w.tol;
     /* the pairs hold nn float2 each, the second array 256-byte aligned */
-    float2 *dfp = dfb ? (float2 *)(base + 8 * vec + codeb + mgb + listb) : nullptr;
+    float2 *dfp = dfb ? (float2 *)(base + 8 * vec + codeb + mgb) : nullptr;
     /* the predictor rides on the pairs' pass (the caller skipped k_predict) */
     double *pp = w.phi_prev;
     int predict = dfp && !ly ? w.predict_mode : 0;
@@ -1837,7 +1960,7 @@ static int run_pcg(World &w) {
     Coef3<T> ctp;
     for (int a = 0; a < 3; a++) ctp.c[a] = (T)(1.0 / (g.dh[a] * g.dh[a]));
     void *args[] = {&g,    &phi,  &rho,  &cc,   &tg,   &phi0, &te0, &n0,  &nr_max, &nr_tol, &pcg_max, &pcg_tol,
-                    &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6], &v[7], &A,  &lst,   &part,   &st,      &err,
+                    &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6], &v[7], &A,  &part,   &st,      &err,
                     &ly,   &lb,   &gs_max, &gs_tol, &dfp,  &pp,   &predict, &ctp};
     w.nlaunch++;
     return (int)cudaLaunchCooperativeKernel(fn, grid, threads, args, dyn, w.stream);

@@ -4,6 +4,7 @@ csrc/espic_world.h): for n < 2^24, trunc(float(n) * RN(1/d)) is within one of
 n // d, so one remainder test makes it exact.  Emulated with numpy float32,
 whose products round to nearest like the device's float multiply."""
 import numpy as np
+import pytest
 
 
 def div_small(n, d):
@@ -29,6 +30,18 @@ def test_float_estimated_division_is_exact_below_2_pow_24():
         want = n // d
         assert np.all(np.abs(est - want) <= 1), d
         assert np.array_equal(q, want), d
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 127, 511, 512, 1022, 1024])
+def test_float_estimated_division_is_exact_for_quotients_below_2_pow_22(d):
+    """The largest grids: a colour of 2^30 nodes over rows of at most 512."""
+    rng = np.random.default_rng(d)
+    top = min(1 << 31, d << 22)
+    k = rng.integers(0, top // d, 4096)
+    n = np.concatenate([k * d, k * d + d - 1, rng.integers(0, top, 4096), np.arange(top - 4096, top)]).astype(np.int64)
+    est, q = div_small(n, d)
+    assert np.all(np.abs(est - n // d) <= 1)
+    assert np.array_equal(q, n // d)
 
 
 def dsmc_axis(x0, xm, dh, nc):
