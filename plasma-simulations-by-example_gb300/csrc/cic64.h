@@ -1,0 +1,101 @@
+/*
+ * cic64.h -- pieces of the float64 cloud-in-cell kernels that keep work off
+ * the float64 pipe.  GB300 issues a float64 instruction of a warp in 16
+ * clocks of its SM, in which the four schedulers issue 64 others, so a test,
+ * a truncation or a quotient done on the integer pipes is nearly free beside
+ * one done in float64.  Every function returns the bits of the plain
+ * expression it stands for (units that use them are built with -fmad=false).
+ */
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace espic {
+
+/* x == +-0 on the 32-bit halves of its bits: a 64-bit test of the bits
+ * compiles to a float64 compare */
+__device__ __forceinline__ bool zero_bits(double x) {
+    return (((unsigned int)__double2hiint(x) << 1) | (unsigned int)__double2loint(x)) == 0u;
+}
+
+/* isfinite without a float64 compare */
+__device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+/* a / b correctly rounded, given y = RN(1/b) for b > 0: q = a y, the exact
+ * remainder r = a - b q (one FMA), then q + r y rounded -- Markstein's
+ * correction (P. Markstein, IBM J. Res. Develop. 34(1), 1990), which yields
+ * the correctly rounded quotient for normal operands, so results equal the
+ * division's bit for bit; a = +-0 returns a y, the zero of the right sign. */
+__device__ __forceinline__ double div_rcp(double a, double b, double y) {
+    const double q = a * y;
+    const double r = __fma_rn(-q, b, a);
+    const double q2 = __fma_rn(r, y, q);
+    return zero_bits(a) ? q : q2;
+}
+
+/* integers in the order of the doubles (-0 and +0 equal); the order of NaN is
+ * that of a value beyond infinity of its sign */
+__device__ __forceinline__ long long order_key(double x) {
+    const long long b = __double_as_longlong(x);
+    const long long m = b & 0x7fffffffffffffffll;
+    return b < 0 ? -m : m;
+}
+
+/* lc, a logical coordinate along an axis of n nodes, as its cell and the
+ * offset lc - cell; the truncation is a mask on the exponent's integer bits
+ * (lc < 2^20).  False, with nothing set, for lc outside [0, n - 1) or not
+ * finite: the caller then takes its general path. */
+__device__ __forceinline__ bool cell_of(double lc, int n, int &cell, double &off) {
+    const int hi = __double2hiint(lc);
+    if ((unsigned)hi >= 0x41300000u) return false; /* negative, 2^20 or more, not finite */
+    const int e = (hi >> 20) - 1023;               /* lc >= 1: e in 0..19 */
+    const int sh = e < 0 ? 20 : 20 - e;
+    const int c = e < 0 ? 0 : ((hi & 0xfffff) | 0x100000) >> sh;
+    if (c > n - 2) return false;
+    const double t = __hiloint2double(e < 0 ? 0 : hi & ~((1 << sh) - 1), 0);
+    cell = c;
+    off = lc - t;
+    return true;
+}
+
+/* the 24 leading bits of x as a float (0 below 2^-126; false above the float
+ * range), within 2^-23 |x| of x */
+__device__ __forceinline__ bool cut_float(double x, float &xf) {
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const int fe = ((hi >> 20) & 0x7ff) - 896; /* float exponent field */
+    xf = 0.0f;
+    if (fe >= 1) xf = __int_as_float((hi & (int)0x80000000) | (fe << 23) | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
+    return fe <= 254;
+}
+
+/* Field_::scatter of `value` at cell offsets d, each corner weight
+ * value*(1-di)*(1-dj)*(1-dk) (the reference's operand order) rounded once to
+ * an integer count of 1/fx and added to acc.  fx is a power of two, so it
+ * multiplies the value once instead of eight weights.  unit_cell: d lies in
+ * [0, 1), so that no weight exceeds the value; a count below 2^50 is then
+ * rounded by adding 1.5 * 2^52, which leaves it in the low bits, instead of
+ * by a conversion. */
+__device__ __forceinline__ void scatter8(unsigned long long *acc, int64_t n0, int64_t sy, int64_t sz,
+                                         const double d[3], double value, double fx, bool unit_cell) {
+    const double magic = 6755399441055744.0;
+    const double v = value * fx;
+    const double a0 = v * (1 - d[0]), a1 = v * d[0], gj = 1 - d[1], gk = 1 - d[2];
+    const double b0 = a0 * gj, b1 = a1 * gj, b2 = a1 * d[1], b3 = a0 * d[1];
+    const double w[8] = {b0 * gk, b1 * gk, b2 * gk, b3 * gk, b0 * d[2], b1 * d[2], b2 * d[2], b3 * d[2]};
+    const int64_t idx[8] = {n0, n0 + 1, n0 + 1 + sy, n0 + sy, n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
+    if (unit_cell && (__double2hiint(v) & 0x7fffffff) < 0x43100000) { /* |v| < 2^50 */
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            const long long q = __double_as_longlong(w[m] + magic) - __double_as_longlong(magic);
+            if (q != 0) atomicAdd(acc + idx[m], (unsigned long long)q);
+        }
+    } else {
+        for (int m = 0; m < 8; m++) {
+            const long long q = __double2ll_rn(w[m]);
+            if (q != 0) atomicAdd(acc + idx[m], (unsigned long long)q);
+        }
+    }
+}
+
+}  // namespace espic

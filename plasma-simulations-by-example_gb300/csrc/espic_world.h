@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <vector>
 
+#include "cic64.h"
 #include "espic_internal.h"
 
 namespace espic {
@@ -176,13 +177,6 @@ struct World {
     double prof_ms[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int64_t prof_n[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
-
-/* x == +-0, tested on the 32-bit halves of its bits: written as a 64-bit
- * test of the bits it compiles to a float64 compare, which issues on this
- * GPU's narrow float64 pipe */
-__device__ __forceinline__ bool zero_bits(double x) {
-    return (((unsigned int)__double2hiint(x) << 1) | (unsigned int)__double2loint(x)) == 0u;
-}
 
 /* n / d for n < 2^24, or n < 2^31 with a quotient below 2^22, without an
  * integer division: the float estimate (n, 1/d and the product each rounded

@@ -56,21 +56,6 @@ namespace espic {
 constexpr int ENS_VW = 1024;      /* virtual width of the deterministic reductions */
 constexpr int ENS_SWEEPS = 25;    /* float32 sweeps between float64 residual checks */
 
-/* a / b correctly rounded, given y = RN(1/b) for b > 0: q = a y, the exact
- * remainder r = a - b q (one FMA) and q + r y rounded, Markstein's
- * correction (P. Markstein, IBM J. Res. Develop. 34(1), 1990), which yields
- * the correctly rounded quotient for normal operands; a = +-0 returns a y,
- * the zero of the right sign.  Three float64 operations instead of a
- * division, whose cost the GB300's float64 rate makes dominant. */
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-    const double q = a * y;
-    const double r = __fma_rn(-q, b, a);
-    const double q2 = __fma_rn(r, y, q);
-    /* a == +-0 tested on the bits: an integer compare keeps the narrow
-     * float64 pipe for the arithmetic */
-    return zero_bits(a) ? q : q2;
-}
-
 /* sum of part[0..ENS_VW) in a fixed tree; every thread gets the total */
 __device__ double ens_tree_sum(double *part) {
     __syncthreads();

@@ -43,14 +43,32 @@ __device__ __forceinline__ int64_t node_of(const Geo &g, int i, int j, int k) {
     return ((int64_t)k * g.nj + j) * g.ni + i;
 }
 
+/* The cell of logical coordinates lc with the index clamp, and the offsets
+ * lc - cell; true when every offset lies in [0, 1). */
+__device__ __forceinline__ bool cells_of(const Geo &g, const double lc[3], int c[3], double off[3]) {
+    const int n[3] = {g.ni, g.nj, g.nk};
+    bool unit = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        if (!cell_of(lc[d], n[d], c[d], off[d])) {
+            c[d] = clamp_cell((int)lc[d], n[d]);
+            off[d] = lc[d] - c[d];
+            unit = false;
+        }
+    return unit;
+}
+
 /* Field_<double3>::gather with the index clamp: out-of-range truncated
  * indices (only reachable at x == xm after a one-bounce reflection) are
  * moved to n-2 keeping di = lc - i, which gives the same weights without
  * reading node n. */
 __device__ __forceinline__ void gather3(const Geo &g, const double *__restrict__ ef, const double lc[3],
                                         double e[3]) {
-    int i = clamp_cell((int)lc[0], g.ni), j = clamp_cell((int)lc[1], g.nj), k = clamp_cell((int)lc[2], g.nk);
-    double di = lc[0] - i, dj = lc[1] - j, dk = lc[2] - k;
+    int cell[3];
+    double off[3];
+    cells_of(g, lc, cell, off);
+    const int i = cell[0], j = cell[1], k = cell[2];
+    const double di = off[0], dj = off[1], dk = off[2];
     int64_t n0 = node_of(g, i, j, k);
     int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
     const double *a = ef + 3 * n0;
@@ -82,22 +100,6 @@ __device__ __forceinline__ bool in_bounds(const Geo &g, const double x[3]) {
     return true;
 }
 
-/* a / b correctly rounded, given y = RN(1/b) for b > 0: q = a y, the exact
- * remainder r = a - b q (one FMA), then q + r y rounded -- Markstein's
- * correction (P. Markstein, IBM J. Res. Develop. 34(1), 1990), which yields
- * the correctly rounded quotient for normal operands, so results equal the
- * division's bit for bit; a = +-0 returns a y, the zero of the right sign.
- * Three float64 operations instead of a division: the GB300's float64 rate
- * makes the division dominate the kernels below. */
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-    const double q = a * y;
-    const double r = __fma_rn(-q, b, a);
-    const double q2 = __fma_rn(r, y, q);
-    /* a == +-0 tested on the bits: an integer compare keeps the narrow
-     * float64 pipe for the arithmetic */
-    return zero_bits(a) ? q : q2;
-}
-
 /* x to logical coordinates with the correctly rounded reciprocal of dh:
  * equal to World::XtoL's division bit for bit (div_rcp) */
 __device__ __forceinline__ void xtol_rcp(const Geo &g, double3 rdh, const double x[3], double lc[3]) {
@@ -112,45 +114,72 @@ __device__ __forceinline__ bool in_sphere(const double s[4], const double x[3]) 
     return rm2 <= s[3];
 }
 
-/* Field_::scatter of `value` at x as 64-bit fixed point: each corner weight
- * value*(1-di)*(1-dj)*(1-dk) (reference order) is rounded once to an integer
- * count of 1/fx and added exactly. */
-__device__ __forceinline__ void deposit8(const Geo &g, unsigned long long *acc, const double x[3],
-                                         double value, double fx) {
-    double lc[3];
-    xtol(g, x, lc);
-    int i = clamp_cell((int)lc[0], g.ni), j = clamp_cell((int)lc[1], g.nj), k = clamp_cell((int)lc[2], g.nk);
-    double di = lc[0] - i, dj = lc[1] - j, dk = lc[2] - k;
-    int64_t n0 = node_of(g, i, j, k);
-    int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    double w[8];
-    w[0] = value * (1 - di) * (1 - dj) * (1 - dk);
-    w[1] = value * (di) * (1 - dj) * (1 - dk);
-    w[2] = value * (di) * (dj) * (1 - dk);
-    w[3] = value * (1 - di) * (dj) * (1 - dk);
-    w[4] = value * (1 - di) * (1 - dj) * (dk);
-    w[5] = value * (di) * (1 - dj) * (dk);
-    w[6] = value * (di) * (dj) * (dk);
-    w[7] = value * (1 - di) * (dj) * (dk);
-    int64_t idx[8] = {n0, n0 + 1, n0 + 1 + sy, n0 + sy, n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
+/* Field_::scatter of `value` at logical coordinates lc as 64-bit fixed point
+ * (scatter8) */
+__device__ __forceinline__ void deposit8(const Geo &g, unsigned long long *acc, const double lc[3], double value,
+                                         double fx) {
+    int c[3];
+    double off[3];
+    const bool unit = cells_of(g, lc, c, off);
+    scatter8(acc, node_of(g, c[0], c[1], c[2]), g.ni, (int64_t)g.ni * g.nj, off, value, fx, unit);
+}
+
+/* A float test that x lies surely outside the sphere, so that most warps
+ * skip the float64 one: rej2 is above the squared radius by more than the
+ * float distance's error (host side, sphere_reject); negative without a
+ * sphere. */
+__device__ __forceinline__ bool surely_outside(const float cf[3], float rej2, const double x[3]) {
+    float d2 = 0.f;
+    bool fits = true;
 #pragma unroll
-    for (int m = 0; m < 8; m++) {
-        long long q = __double2ll_rn(w[m] * fx);
-        if (q != 0) atomicAdd(acc + idx[m], (unsigned long long)q);
+    for (int d = 0; d < 3; d++) {
+        float xf;
+        fits = cut_float(x[d], xf) && fits;
+        const float r = xf - cf[d];
+        d2 += r * r;
     }
+    return fits && d2 > rej2;
+}
+
+struct SphereReject {
+    float c[3], rej2;
+};
+
+static double3 rcp_dh(const World &w) {
+    return make_double3(1.0 / w.g.dh[0], 1.0 / w.g.dh[1], 1.0 / w.g.dh[2]);
+}
+
+static SphereReject sphere_reject(const World &w) {
+    /* coordinates within L of the origin; x and the centre to float and the
+     * difference cost 2^-21 L each at most, the squares and sums 2^-22 of
+     * the squared distance */
+    SphereReject s;
+    double L = 0;
+    for (int d = 0; d < 3; d++) {
+        s.c[d] = (float)w.sphere[d];
+        L = fmax(L, fmax(fabs(w.sphere[d]), fmax(fabs(w.g.x0[d]), fabs(w.g.xm[d]))));
+    }
+    const double r = w.has_sphere ? sqrt(w.sphere[3]) + 8 * ldexp(1.0, -21) * (L + sqrt(w.sphere[3])) : 0;
+    s.rej2 = w.has_sphere ? (float)(r * r * 1.00001) : -1.f;
+    return s;
 }
 
 /* ------------------------------------------------------------------------ */
 /* Species::advance, fused with Species::computeNumberDensity of the moved
  * particles.  One thread per particle; a warp writes one word of the dead
- * mask and adds its dead count to the particle tile's counter. */
+ * mask and adds its dead count to the particle tile's counter.  Bound by the
+ * float64 pipe: 93 of its float64 instructions are the reference's three
+ * left-to-right gathers; quotients by dh come from its rounded reciprocal,
+ * bounds, truncations and the far sphere test from integers and floats.
+ * 4M ions on 64x64x128 nodes: 1.68 ms with divisions, float64 compares and
+ * a conversion per corner weight, 1.28 ms now. */
 template <int WALLS, bool DEPOSIT, bool UNIFORM>
 __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restrict__ ef, double s,
                                                    double dt, double *P, int64_t stride,
                                                    const int64_t *__restrict__ d_count, double4 sph,
-                                                   uint32_t *deadmask, int32_t *tiledead,
-                                                   unsigned long long *acc, double fx, double w0,
-                                                   int *err) {
+                                                   SphereReject far, double3 rdh, uint32_t *deadmask,
+                                                   int32_t *tiledead, unsigned long long *acc, double fx,
+                                                   double w0, int *err) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t n = d_count[0];
     bool dead = false;
@@ -158,7 +187,7 @@ __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restri
         double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
         double v[3] = {P[3 * stride + p], P[4 * stride + p], P[5 * stride + p]};
         double lc[3], e[3];
-        xtol(g, x, lc);
+        xtol_rcp(g, rdh, x, lc);
         gather3(g, ef, lc, e);
 #pragma unroll
         for (int d = 0; d < 3; d++) v[d] += e[d] * s;
@@ -167,19 +196,27 @@ __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restri
         if (WALLS == REFLECT) {
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                if (x[d] < g.x0[d]) {
+                const long long k = order_key(x[d]);
+                if (k < order_key(g.x0[d])) {
                     x[d] = 2 * g.x0[d] - x[d];
                     v[d] *= -1.0;
-                } else if (x[d] >= g.xm[d]) {
+                } else if (k >= order_key(g.xm[d]) && finite_bits(x[d])) {
                     x[d] = 2 * g.xm[d] - x[d];
                     v[d] *= -1.0;
                 }
             }
         } else {
-            double sp[4] = {sph.x, sph.y, sph.z, sph.w};
-            dead = in_sphere(sp, x) || !in_bounds(g, x);
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const long long k = order_key(x[d]);
+                dead = dead || k < order_key(g.x0[d]) || k >= order_key(g.xm[d]);
+            }
+            if (!dead && !surely_outside(far.c, far.rej2, x)) {
+                const double sp[4] = {sph.x, sph.y, sph.z, sph.w};
+                dead = in_sphere(sp, x);
+            }
         }
-        if (!(isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]))) {
+        if (!(finite_bits(x[0]) && finite_bits(x[1]) && finite_bits(x[2]))) {
             atomicOr(err, DERR_NONFINITE);
             dead = true;
         }
@@ -190,7 +227,8 @@ __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restri
         }
         if (DEPOSIT && !dead) {
             double w = UNIFORM ? w0 : P[6 * stride + p];
-            deposit8(g, acc, x, w, fx);
+            xtol_rcp(g, rdh, x, lc);
+            deposit8(g, acc, lc, w, fx);
         }
     }
     if (WALLS == ABSORB) {
@@ -204,13 +242,14 @@ __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restri
 
 template <bool UNIFORM>
 __global__ void __launch_bounds__(256) k_deposit_fp64(Geo g, const double *__restrict__ P, int64_t stride,
-                                                      const int64_t *__restrict__ d_count,
+                                                      const int64_t *__restrict__ d_count, double3 rdh,
                                                       unsigned long long *acc, double fx, double w0) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= d_count[0]) return;
-    double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
+    double x[3] = {P[p], P[stride + p], P[2 * stride + p]}, lc[3];
     double w = UNIFORM ? w0 : P[6 * stride + p];
-    deposit8(g, acc, x, w, fx);
+    xtol_rcp(g, rdh, x, lc);
+    deposit8(g, acc, lc, w, fx);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1407,7 +1446,7 @@ static void push_fp64_as(World &w, Species &s, int blocks) {
     double sc = w.dt * s.charge / s.mass;
     double4 sph = make_double4(w.sphere[0], w.sphere[1], w.sphere[2], w.has_sphere ? w.sphere[3] : -1.0);
     k_push_fp64<WALLS, DEP, UNI><<<blocks, 256, 0, w.stream>>>(w.g, w.ef, sc, w.dt, s.P, s.cap, s.d_count, sph,
-                                                              s.deadmask, s.tiledead, s.acc, s.fx, s.mpw0, w.d_err);
+                                                              sphere_reject(w), rcp_dh(w), s.deadmask, s.tiledead, s.acc, s.fx, s.mpw0, w.d_err);
     w.nlaunch++;
 }
 
@@ -1437,11 +1476,11 @@ void launch_deposit_fp64(World &w, Species &s) {
     int64_t n = s.host_bound;
     if (n <= 0) return;
     if (s.uniform_w)
-        k_deposit_fp64<true><<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, s.acc, s.fx,
-                                                                       s.mpw0);
+        k_deposit_fp64<true><<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, rcp_dh(w),
+                                                                       s.acc, s.fx, s.mpw0);
     else
-        k_deposit_fp64<false><<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, s.acc, s.fx,
-                                                                        s.mpw0);
+        k_deposit_fp64<false><<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, rcp_dh(w),
+                                                                        s.acc, s.fx, s.mpw0);
     w.nlaunch++;
 }
 
@@ -1659,19 +1698,18 @@ struct DsmcAxis {
     int nc;
 };
 
-__device__ __forceinline__ int dsmc_coord(double x, double x0, double dh, DsmcAxis ax) {
-    const int hi = __double2hiint(x);
-    const unsigned lo = (unsigned)__double2loint(x);
-    const int fe = ((hi >> 20) & 0x7ff) - 896; /* float exponent field */
-    float xf = 0.0f;                            /* |x| < 2^-126: zero */
-    if (fe >= 1) xf = __int_as_float((hi & (int)0x80000000) | (fe << 23) | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
+/* below: the index of a quotient in (-1, 0), which truncates to 0 */
+__device__ __forceinline__ int dsmc_coord(double x, double x0, double dh, DsmcAxis ax, int below = 0) {
+    float xf;
+    const bool fits = cut_float(x, xf);
     const float q = (xf - ax.x0f) * ax.invf;
-    if (fe <= 254 && q >= 0.0f && q < (float)ax.nc) {
+    if (fits && q >= 0.0f && q < (float)ax.nc) {
         const int k = (int)q;
         const float fr = q - (float)k; /* exact: k <= q < k + 1 */
         if (fr > ax.tol && fr < 1.0f - ax.tol) return k;
     }
-    return (int)((x - x0) / dh);
+    const double lc = (x - x0) / dh;
+    return lc < 0 ? (lc > -1 ? below : (int)lc) : (int)lc;
 }
 
 static DsmcAxis dsmc_axis(double x0, double xm, double dh, int nc) {
@@ -2042,34 +2080,67 @@ __device__ __forceinline__ void mom_values(const double *__restrict__ P, int64_t
 }
 
 /* largest |value| of each sum over the particles, as float64 bits (the bits
- * of non-negative values order like the values: integer max, no float64) */
-__global__ void __launch_bounds__(256) k_mom_bound(const double *__restrict__ P, int64_t stride, double w0,
-                                                   const int64_t *__restrict__ d_count, unsigned long long *bound) {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long b[NMOM];
-    for (int q = 0; q < NMOM; q++) b[q] = 0;
-    if (p < d_count[0]) {
+ * of non-negative values order like the values: integer max, no float64).
+ * UNIFORM (one weight w0 > 0): a product rounded is monotone in |u|, so the
+ * largest |u|, |v|, |w| are enough; they go to bound[1..3], and k_mom_scale
+ * forms the products.  A block strides over the particles and adds one
+ * atomic per value: with a thread per particle the seven addresses took 1.4M
+ * atomics and the call 943 us for 6.4M atoms (28 us now). */
+constexpr int BOUND_THREADS = 256;
+
+template <bool UNIFORM>
+__global__ void __launch_bounds__(BOUND_THREADS) k_mom_bound(const double *__restrict__ P, int64_t stride,
+                                                             const int64_t *__restrict__ d_count,
+                                                             unsigned long long *bound) {
+    constexpr int NB = UNIFORM ? 3 : NMOM;
+    __shared__ unsigned long long sh[NB][BOUND_THREADS / 32];
+    unsigned long long b[NB];
+    for (int q = 0; q < NB; q++) b[q] = 0;
+    const int64_t n = d_count[0];
+    for (int64_t p = (int64_t)blockIdx.x * BOUND_THREADS + threadIdx.x; p < n;
+         p += (int64_t)gridDim.x * BOUND_THREADS) {
         double v[NMOM];
-        mom_values(P, stride, p, w0, v);
-        for (int q = 0; q < NMOM; q++) b[q] = (unsigned long long)__double_as_longlong(v[q]) & 0x7fffffffffffffffull;
+        if (UNIFORM)
+            for (int q = 0; q < 3; q++) v[q] = P[(3 + q) * stride + p];
+        else
+            mom_values(P, stride, p, 0.0, v);
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            const unsigned long long x = (unsigned long long)__double_as_longlong(v[q]) & 0x7fffffffffffffffull;
+            b[q] = x > b[q] ? x : b[q];
+        }
     }
-    for (int q = 0; q < NMOM; q++) {
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
         unsigned long long x = b[q];
         for (int o = 16; o; o >>= 1) {
             const unsigned long long y = __shfl_xor_sync(0xffffffffu, x, o);
             x = y > x ? y : x;
         }
-        if ((threadIdx.x & 31) == 0 && x) atomicMax(bound + q, x);
+        if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < NB) {
+        unsigned long long x = 0;
+        for (int k = 0; k < BOUND_THREADS / 32; k++) x = sh[threadIdx.x][k] > x ? sh[threadIdx.x][k] : x;
+        if (x) atomicMax(bound + (UNIFORM ? 1 + threadIdx.x : threadIdx.x), x);
     }
 }
 
 /* scale[q] = 2^S_q with count * max_q * 2^S_q < 2^62 (no node overflows)
  * and max_q * 2^S_q < 2^51 (each product converts by one FMA, see
  * fix_round); scale[NMOM + q] = 2^-S_q */
-__global__ void k_mom_scale(const unsigned long long *bound, const int64_t *d_count, double *scale, int *err) {
+__global__ void k_mom_scale(const unsigned long long *bound, double w0, const int64_t *d_count, double *scale,
+                            int *err) {
     const int q = threadIdx.x;
     if (q >= NMOM) return;
-    const double b = __longlong_as_double((long long)bound[q]);
+    double b;
+    if (w0 > 0) { /* the largest |u|, |v|, |w| (k_mom_bound<true>) */
+        const double u = __longlong_as_double((long long)bound[q == 0 ? 1 : 1 + (q - 1) % 3]);
+        b = q == 0 ? (d_count[0] > 0 ? w0 : 0.0) : (q < 4 ? w0 * u : w0 * u * u);
+    } else {
+        b = __longlong_as_double((long long)bound[q]);
+    }
     const double t = b * (double)(d_count[0] > 0 ? d_count[0] : 1);
     int S = 0;
     if (!isfinite(t)) {
@@ -2121,14 +2192,17 @@ __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const d
     const double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
     double lc[3];
     xtol_rcp(g, rdh, x, lc);
-    if (!(lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && lc[0] <= g.ni - 1 && lc[1] <= g.nj - 1 && lc[2] <= g.nk - 1)) {
+    int cl[3];
+    double off[3];
+    /* offsets in [0, 1) imply the range */
+    if (!cells_of(g, lc, cl, off) &&
+        !(lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && lc[0] <= g.ni - 1 && lc[1] <= g.nj - 1 && lc[2] <= g.nk - 1)) {
         atomicOr(err, DERR_NEUTRAL);
         return;
     }
-    const int i = clamp_cell((int)lc[0], g.ni), j = clamp_cell((int)lc[1], g.nj), k = clamp_cell((int)lc[2], g.nk);
     double W[8];
-    corner_weights(lc[0] - i, lc[1] - j, lc[2] - k, W);
-    const int64_t n0 = node_of(g, i, j, k), sy = g.ni, sz = (int64_t)g.ni * g.nj;
+    corner_weights(off[0], off[1], off[2], W);
+    const int64_t n0 = node_of(g, cl[0], cl[1], cl[2]), sy = g.ni, sz = (int64_t)g.ni * g.nj;
     const int64_t idx[8] = {n0, n0 + 1, n0 + 1 + sy, n0 + sy, n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
     double v[NMOM];
     mom_values(P, stride, p, w0, v);
@@ -2181,16 +2255,21 @@ __global__ void __launch_bounds__(256) k_gas_props(int64_t nn, double mass, cons
 }
 
 /* Species::computeMPC (ch4/Species.cpp:228-235): macroparticles per cell
- * (World::XtoIJK); counts below 2^53 are exact in float64 */
-__global__ void __launch_bounds__(256) k_mpc(Geo g, const double *__restrict__ P, int64_t stride,
+ * (World::XtoIJK); counts below 2^53 are exact in float64.  The cell comes
+ * from the float estimate of the collisions' grouping (dsmc_coord); a
+ * position in front of the first cell, which truncates to it, is refused.
+ * With three float64 divisions per particle the kernel took 382 us for 6.4M
+ * atoms, 55 us now. */
+__global__ void __launch_bounds__(256) k_mpc(Geo g, DsmcAxis ax, DsmcAxis ay, DsmcAxis az,
+                                             const double *__restrict__ P, int64_t stride,
                                              const int64_t *__restrict__ d_count, double *mpc, int *err) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= d_count[0]) return;
     const double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
-    double lc[3];
-    xtol(g, x, lc);
-    const int i = (int)lc[0], j = (int)lc[1], k = (int)lc[2];
-    if (!(lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && i < g.ni - 1 && j < g.nj - 1 && k < g.nk - 1)) {
+    const int i = dsmc_coord(x[0], g.x0[0], g.dh[0], ax, -1), j = dsmc_coord(x[1], g.x0[1], g.dh[1], ay, -1),
+              k = dsmc_coord(x[2], g.x0[2], g.dh[2], az, -1);
+    if (!(finite_bits(x[0]) && finite_bits(x[1]) && finite_bits(x[2])) || i < 0 || j < 0 || k < 0 || i >= g.ni - 1 ||
+        j >= g.nj - 1 || k >= g.nk - 1) {
         atomicOr(err, DERR_NEUTRAL);
         return;
     }
@@ -2265,16 +2344,19 @@ __global__ void __launch_bounds__(256) k_mcc_cex(Geo g, double3 rdh, double *P, 
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(ncol, (unsigned long long)__popc(m));
 }
 
-static double3 rcp_dh(const World &w) {
-    return make_double3(1.0 / w.g.dh[0], 1.0 / w.g.dh[1], 1.0 / w.g.dh[2]);
-}
-
 void launch_moments(World &w, Species &s) {
     const int64_t n = s.host_bound;
     cudaMemsetAsync(s.mom_bound, 0, NMOM * sizeof(unsigned long long), w.stream);
     const double w0 = s.uniform_w ? s.mpw0 : 0.0;
-    if (n > 0) k_mom_bound<<<blocks_for(n, 256), 256, 0, w.stream>>>(s.P, s.cap, w0, s.d_count, s.mom_bound);
-    k_mom_scale<<<1, 32, 0, w.stream>>>(s.mom_bound, s.d_count, s.mom_scale, w.d_err);
+    if (n > 0) {
+        int nb = blocks_for(n, BOUND_THREADS);
+        if (nb > 8 * w.sm_count) nb = 8 * w.sm_count;
+        if (w0 > 0)
+            k_mom_bound<true><<<nb, BOUND_THREADS, 0, w.stream>>>(s.P, s.cap, s.d_count, s.mom_bound);
+        else
+            k_mom_bound<false><<<nb, BOUND_THREADS, 0, w.stream>>>(s.P, s.cap, s.d_count, s.mom_bound);
+    }
+    k_mom_scale<<<1, 32, 0, w.stream>>>(s.mom_bound, w0, s.d_count, s.mom_scale, w.d_err);
     if (n > 0)
         k_mom_scatter<<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, rcp_dh(w), s.P, s.cap, w0, s.d_count,
                                                                  s.mom_scale, s.mom_acc, w.nn, w.d_err);
@@ -2292,7 +2374,10 @@ void launch_mpc(World &w, Species &s) {
     const int64_t n_cells = (int64_t)(w.g.ni - 1) * (w.g.nj - 1) * (w.g.nk - 1);
     cudaMemsetAsync(s.mpc, 0, n_cells * sizeof(double), w.stream);
     if (n > 0) {
-        k_mpc<<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, s.mpc, w.d_err);
+        const DsmcAxis ax = dsmc_axis(w.g.x0[0], w.g.xm[0], w.g.dh[0], w.g.ni - 1);
+        const DsmcAxis ay = dsmc_axis(w.g.x0[1], w.g.xm[1], w.g.dh[1], w.g.nj - 1);
+        const DsmcAxis az = dsmc_axis(w.g.x0[2], w.g.xm[2], w.g.dh[2], w.g.nk - 1);
+        k_mpc<<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, ax, ay, az, s.P, s.cap, s.d_count, s.mpc, w.d_err);
         w.nlaunch++;
     }
 }
@@ -2340,7 +2425,8 @@ struct Ch4Uniforms {
     }
 };
 
-__global__ void __launch_bounds__(256) k_advance_ch4(Ch4Geo G, double mass, double dt, double *P, int64_t stride,
+__global__ void __launch_bounds__(256) k_advance_ch4(Ch4Geo G, SphereReject far, double mass, double dt, double *P,
+                                                     int64_t stride,
                                                      const int64_t *__restrict__ d_count,
                                                      const int64_t *__restrict__ d_settled,
                                                      const double *__restrict__ pdt, const double *__restrict__ u,
@@ -2357,9 +2443,25 @@ __global__ void __launch_bounds__(256) k_advance_ch4(Ch4Geo G, double mass, doub
         const double t = (pdt ? pdt[p] : (p >= d_settled[0] ? dt : 0.0)) + dt;
         Ch4Uniforms U{u, nu, u ? p_off[p] : 0, seed, stream, (uint64_t)p << 10, false};
         bool alive = true;
-        b = ch4_advance_one(G, mass, t, x, v, U, alive, 64);
+        /* most particles move once and strike nothing: the bounds by integer
+         * keys and the sphere by a float distance; the others, and those
+         * near the sphere, take the whole step from where they were */
+        double y[3];
+        bool simple = order_key(t) > 0 && finite_bits(t);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            y[d] = x[d] + v[d] * t;
+            const long long k = order_key(y[d]);
+            simple = simple && k >= order_key(G.x0[d]) && k < order_key(G.xm[d]);
+        }
+        if (simple && surely_outside(far.c, far.rej2, y)) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) x[d] = y[d];
+        } else {
+            b = ch4_advance_one(G, mass, t, x, v, U, alive, 64);
+        }
         if (U.bad) atomicOr(err, DERR_NEUTRAL);
-        if (!(isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]))) {
+        if (!(finite_bits(x[0]) && finite_bits(x[1]) && finite_bits(x[2]))) {
             atomicOr(err, DERR_NONFINITE);
             alive = false;
         }
@@ -2397,7 +2499,7 @@ void launch_advance_ch4(World &w, Species &s, double dt, const double *d_pdt, co
         /* one stream per (species, call) */
         const uint64_t stream = (0xC4ull << 56) | ((uint64_t)(s.id & 0xff) << 48) |
                                 (s.ch4_calls & 0xffffffffffffull);
-        k_advance_ch4<<<blocks_for(n, 256), 256, 0, w.stream>>>(G, s.mass, dt, s.P, s.cap, s.d_count, s.ch4_settled,
+        k_advance_ch4<<<blocks_for(n, 256), 256, 0, w.stream>>>(G, sphere_reject(w), s.mass, dt, s.P, s.cap, s.d_count, s.ch4_settled,
                                                                  d_pdt, d_u, nu, d_off, w.seed, stream, s.deadmask,
                                                                  s.tiledead, s.ch4_bounces, w.d_err);
         w.nlaunch++;

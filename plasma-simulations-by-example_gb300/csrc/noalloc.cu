@@ -29,6 +29,7 @@
 
 #include <mutex>
 
+#include "cic64.h"
 #include "espic.h"
 
 namespace {
@@ -37,63 +38,76 @@ __device__ __align__(256) unsigned long long g_noalloc_acc[ESPIC_NOALLOC_MAX_NOD
 
 struct NaGeo {
     int ni, nj, nk;
-    double x0[3], dh[3];
+    double x0[3], dh[3], rdh[3]; /* rdh = RN(1 / dh) */
 };
 
 __device__ __forceinline__ int na_clamp(int i, int n) { return i < 0 ? 0 : (i > n - 2 ? n - 2 : i); }
 
-__global__ void k_na_clear(unsigned long long *acc, int64_t nn, int *flags) {
-    int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+/* The three kernels of a call are launched so that each may start while the
+ * one before drains (programmatic dependent launch): the waits hide the
+ * launches and, in the deposit, the particle's arithmetic.  next_may_start
+ * lets the next kernel be scheduled once every block of this one runs;
+ * wait_for_previous returns when the kernel before has finished and its
+ * writes are visible. */
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__global__ void __launch_bounds__(256) k_na_clear(unsigned long long *acc, uint32_t nn, int *flags) {
+    next_may_start();
+    const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u < nn) acc[u] = 0ull;
     if (u == 0 && flags) *flags = 0;
 }
 
 /* A particle whose position is not finite, or whose weight is not within
  * [-weight_bound, weight_bound] (so that its corner counts could wrap the
- * int64 sums), deposits nothing and sets a bit of *flags. */
-__global__ void k_na_deposit(NaGeo g, const double *__restrict__ P, int64_t stride, int64_t n, double fx,
-                             double weight_bound, unsigned long long *acc, int *flags) {
+ * int64 sums), deposits nothing and sets a bit of the flags.  Bound by the
+ * float64 pipe, which runs the three differences, nine operations of the
+ * quotients by dh, the offsets and the weights (6M particles on 97x89x117
+ * nodes: 827 us with divisions and a conversion per weight, 507 us now). */
+__global__ void __launch_bounds__(256) k_na_deposit(NaGeo g, const double *__restrict__ P, int64_t stride, int64_t n,
+                                                    double fx, double weight_bound, unsigned long long *acc,
+                                                    int *flags) {
+    next_may_start();
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
-    double lc[3];
-    for (int d = 0; d < 3; d++) lc[d] = (P[d * stride + p] - g.x0[d]) / g.dh[d];
-    double value = P[6 * stride + p];
-    const bool finite = isfinite(lc[0]) && isfinite(lc[1]) && isfinite(lc[2]);
-    const bool in_range = fabs(value) <= weight_bound; /* false for NaN */
+    double lc[3], off[3];
+    for (int d = 0; d < 3; d++) lc[d] = espic::div_rcp(P[d * stride + p] - g.x0[d], g.dh[d], g.rdh[d]);
+    const double value = P[6 * stride + p];
+    const bool finite = espic::finite_bits(lc[0]) && espic::finite_bits(lc[1]) && espic::finite_bits(lc[2]);
+    /* false for NaN, whose key lies beyond infinity's */
+    const bool in_range = espic::order_key(fabs(value)) <= espic::order_key(weight_bound);
     if (!(finite && in_range)) {
+        wait_for_previous();
         if (flags) atomicOr(flags, (finite ? 0 : ESPIC_NOALLOC_NONFINITE) | (in_range ? 0 : ESPIC_NOALLOC_RANGE));
         return;
     }
-    int i = na_clamp((int)lc[0], g.ni), j = na_clamp((int)lc[1], g.nj), k = na_clamp((int)lc[2], g.nk);
-    double di = lc[0] - i, dj = lc[1] - j, dk = lc[2] - k;
-    int64_t n0 = ((int64_t)k * g.nj + j) * g.ni + i;
-    int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    double w[8];
-    w[0] = value * (1 - di) * (1 - dj) * (1 - dk);
-    w[1] = value * (di) * (1 - dj) * (1 - dk);
-    w[2] = value * (di) * (dj) * (1 - dk);
-    w[3] = value * (1 - di) * (dj) * (1 - dk);
-    w[4] = value * (1 - di) * (1 - dj) * (dk);
-    w[5] = value * (di) * (1 - dj) * (dk);
-    w[6] = value * (di) * (dj) * (dk);
-    w[7] = value * (1 - di) * (dj) * (dk);
-    int64_t idx[8] = {n0, n0 + 1, n0 + 1 + sy, n0 + sy, n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
-    for (int m = 0; m < 8; m++) {
-        long long q = __double2ll_rn(w[m] * fx);
-        if (q != 0) atomicAdd(acc + idx[m], (unsigned long long)q);
-    }
+    const int nn3[3] = {g.ni, g.nj, g.nk};
+    int c[3];
+    bool unit = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        if (!espic::cell_of(lc[d], nn3[d], c[d], off[d])) {
+            c[d] = na_clamp((int)lc[d], nn3[d]);
+            off[d] = lc[d] - c[d];
+            unit = false;
+        }
+    const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
+    wait_for_previous();
+    espic::scatter8(acc, c[2] * sz + c[1] * sy + c[0], sy, sz, off, value, fx, unit);
 }
 
-__global__ void k_na_density(NaGeo g, const unsigned long long *__restrict__ acc, double unit, double *den) {
-    int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t nn = (int64_t)g.ni * g.nj * g.nk;
-    if (u >= nn) return;
-    int i = (int)(u % g.ni), j = (int)((u / g.ni) % g.nj), k = (int)(u / ((int64_t)g.ni * g.nj));
+__global__ void __launch_bounds__(256) k_na_density(NaGeo g, const unsigned long long *acc, double unit, double *den) {
+    wait_for_previous();
+    const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= (uint32_t)(g.ni * g.nj * g.nk)) return;
+    const uint32_t row = u / (uint32_t)g.ni;
+    const int i = (int)(u - row * (uint32_t)g.ni), j = (int)(row % (uint32_t)g.nj), k = (int)(row / (uint32_t)g.nj);
     double V = g.dh[0] * g.dh[1] * g.dh[2];
     if (i == 0 || i == g.ni - 1) V *= 0.5;
     if (j == 0 || j == g.nj - 1) V *= 0.5;
     if (k == 0 || k == g.nk - 1) V *= 0.5;
-    double d = __ll2double_rn((long long)acc[u]) * unit;
+    const double d = __ll2double_rn((long long)acc[u]) * unit;
     den[u] = (V != 0) ? d / V : 0.0;
 }
 
@@ -126,6 +140,22 @@ static int na_scratch(unsigned long long **out) {
     }
     *out = (unsigned long long *)g_na_addr[dev];
     return ESPIC_OK;
+}
+
+/* a launch of 256-thread blocks that may overlap the tail of the kernel before
+ * it on the stream (the kernel itself waits for its results) */
+template <class... P, class... A>
+static cudaError_t launch_early(unsigned blocks, cudaStream_t st, void (*fn)(P...), A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
 extern "C" int espic_deposit_noalloc(const double *d_P, int64_t stride, int64_t n, int ni, int nj, int nk,
@@ -161,6 +191,7 @@ extern "C" int espic_deposit_noalloc(const double *d_P, int64_t stride, int64_t 
     for (int d = 0; d < 3; d++) {
         g.x0[d] = x0[d];
         g.dh[d] = (xm[d] - x0[d]) / (nn3[d] - 1);
+        g.rdh[d] = 1.0 / g.dh[d];
     }
     /* the fixed-point scale of a species of capacity n with this weight bound */
     int64_t cap = n < 1 ? 1 : n;
@@ -170,11 +201,13 @@ extern "C" int espic_deposit_noalloc(const double *d_P, int64_t stride, int64_t 
     int S = ex - 1 > 52 ? 52 : ex - 1;
     double fx = ldexp(1.0, S);
     cudaStream_t st = (cudaStream_t)stream;
-    k_na_clear<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, nn, d_flags);
-    if (n > 0)
-        k_na_deposit<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, d_P, stride, n, fx, weight_bound, acc, d_flags);
-    k_na_density<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(g, acc, 1.0 / fx, d_den);
+    k_na_clear<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, (uint32_t)nn, d_flags);
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && n > 0)
+        e = launch_early((unsigned)((n + 255) / 256), st, k_na_deposit, g, d_P, stride, n, fx, weight_bound, acc, d_flags);
+    if (e == cudaSuccess)
+        e = launch_early((unsigned)((nn + 255) / 256), st, k_na_density, g, (const unsigned long long *)acc, 1.0 / fx,
+                         d_den);
     if (e != cudaSuccess) {
         char buf[200];
         snprintf(buf, sizeof buf, "espic_deposit_noalloc: launch: %s", cudaGetErrorString(e));
