@@ -1498,13 +1498,13 @@ static int ensure_ch4(World &w, Species &s) {
     if (s.ch4_on) return ESPIC_OK;
     if (s.form != 0) return fail(ESPIC_ERR_ARG, "moments and MCC work on a species in the float64 form");
     const int64_t n_cells = (int64_t)(w.g.ni - 1) * (w.g.nj - 1) * (w.g.nk - 1);
-    if (dalloc(&s.mom, NMOM * w.nn) != ESPIC_OK || dalloc(&s.mom_acc, NMOM * w.nn) != ESPIC_OK ||
+    if (dalloc(&s.mom, NMOM * w.nn) != ESPIC_OK || dalloc(&s.mom_acc, MOM_STRIDE * w.nn) != ESPIC_OK ||
         dalloc(&s.mom_scale, 2 * NMOM) != ESPIC_OK || dalloc(&s.mom_bound, NMOM) != ESPIC_OK ||
         dalloc(&s.gvel, 3 * w.nn) != ESPIC_OK || dalloc(&s.gtemp, w.nn) != ESPIC_OK ||
         dalloc(&s.mpc, n_cells) != ESPIC_OK || dalloc(&s.mcc_ncol, 1) != ESPIC_OK)
         return ESPIC_ERR_CUDA;
     CK(cudaMemsetAsync(s.mom, 0, NMOM * w.nn * sizeof(double), w.stream));
-    CK(cudaMemsetAsync(s.mom_acc, 0, NMOM * w.nn * sizeof(unsigned long long), w.stream));
+    CK(cudaMemsetAsync(s.mom_acc, 0, MOM_STRIDE * w.nn * sizeof(unsigned long long), w.stream));
     CK(cudaMemsetAsync(s.gvel, 0, 3 * w.nn * sizeof(double), w.stream));
     CK(cudaMemsetAsync(s.gtemp, 0, w.nn * sizeof(double), w.stream));
     CK(cudaMemsetAsync(s.mpc, 0, n_cells * sizeof(double), w.stream));

@@ -48,6 +48,8 @@ __host__ __device__ inline int tile_count(int ncell) { return (ncell + TILE_CELL
 
 /* sampled velocity moments of a ch4 species: n, n u, n v, n w, n u u, n v v, n w w */
 constexpr int NMOM = 7;
+/* a node's integer sums of a call lie side by side, NMOM of MOM_STRIDE used */
+constexpr int MOM_STRIDE = 8;
 
 struct SolveStatus {
     int converged;

@@ -2182,39 +2182,65 @@ __device__ __forceinline__ void corner_weights(double di, double dj, double dk, 
 
 /* each sum's 8 corner contributions value * W_m, rounded once (from the exact
  * product) to a count of 2^-S_q and added exactly; within one weight
- * rounding of the reference's left-to-right product */
+ * rounding of the reference's left-to-right product.  The seven sums of a
+ * node lie side by side (acc[node][MOM_STRIDE]), and a warp turns its 32
+ * particles' counts of a corner around in shared memory, so that eight lanes
+ * add to one node's 64 bytes: with a plane per sum and every lane at its own
+ * node, an atomic instruction touched 32 sectors instead of 16 (1592 us for
+ * 6.4M atoms; 1264 us now, of which the ~100 float64 instructions per
+ * atom are 1070). */
 __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const double *__restrict__ P, int64_t stride,
                                                      double w0, const int64_t *__restrict__ d_count,
                                                      const double *__restrict__ scale, unsigned long long *acc,
-                                                     int64_t nn, int *err) {
+                                                     int *err) {
+    __shared__ longlong2 turn[8][32 * 4];
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= d_count[0]) return;
-    const double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
-    double lc[3];
-    xtol_rcp(g, rdh, x, lc);
-    int cl[3];
-    double off[3];
-    /* offsets in [0, 1) imply the range */
-    if (!cells_of(g, lc, cl, off) &&
-        !(lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && lc[0] <= g.ni - 1 && lc[1] <= g.nj - 1 && lc[2] <= g.nk - 1)) {
-        atomicOr(err, DERR_NEUTRAL);
-        return;
-    }
-    double W[8];
-    corner_weights(off[0], off[1], off[2], W);
-    const int64_t n0 = node_of(g, cl[0], cl[1], cl[2]), sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    const int64_t idx[8] = {n0, n0 + 1, n0 + 1 + sy, n0 + sy, n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
-    double v[NMOM];
-    mom_values(P, stride, p, w0, v);
+    const int lane = threadIdx.x & 31;
+    longlong2 *buf = turn[threadIdx.x >> 5];
+    double v[NMOM] = {0, 0, 0, 0, 0, 0, 0}, W[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int32_t n0 = -1; /* no particle */
+    if (p < d_count[0]) {
+        const double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
+        double lc[3], off[3];
+        int cl[3];
+        xtol_rcp(g, rdh, x, lc);
+        /* offsets in [0, 1) imply the range */
+        if (cells_of(g, lc, cl, off) || (lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && lc[0] <= g.ni - 1 &&
+                                         lc[1] <= g.nj - 1 && lc[2] <= g.nk - 1)) {
+            n0 = (int32_t)node_of(g, cl[0], cl[1], cl[2]);
+            corner_weights(off[0], off[1], off[2], W);
+            mom_values(P, stride, p, w0, v);
 #pragma unroll
-    for (int q = 0; q < NMOM; q++) {
-        const double vf = v[q] * scale[q]; /* exact: a power of two */
-        unsigned long long *a = acc + q * nn;
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const long long c = fix_round(vf, W[m]);
-            if (c) atomicAdd(a + idx[m], (unsigned long long)c);
+            for (int q = 0; q < NMOM; q++) v[q] *= scale[q]; /* exact: a power of two */
+        } else {
+            atomicOr(err, DERR_NEUTRAL);
         }
+    }
+    if (!__any_sync(0xffffffffu, n0 >= 0)) return;
+    const int32_t sy = g.ni, sz = g.ni * g.nj;
+    const int32_t shift[8] = {0, 1, 1 + sy, sy, sz, 1 + sz, 1 + sy + sz, sy + sz};
+    /* 16-byte slot j of particle l sits at l * 4 + (j ^ (l / 2 & 3)): no bank
+     * conflicts in either direction */
+    const int swz = (lane >> 1) & 3, q = lane & 7;
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+        long long c[MOM_STRIDE];
+#pragma unroll
+        for (int k = 0; k < NMOM; k++) c[k] = fix_round(v[k], W[m]);
+        c[NMOM] = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) buf[lane * 4 + (k ^ swz)] = make_longlong2(c[2 * k], c[2 * k + 1]);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int l = r * 4 + (lane >> 3);
+            const longlong2 t = buf[l * 4 + ((q >> 1) ^ ((l >> 1) & 3))];
+            const long long val = (q & 1) ? t.y : t.x;
+            const int32_t node = __shfl_sync(0xffffffffu, n0, l);
+            if (node >= 0 && val != 0)
+                atomicAdd(acc + (int64_t)(node + shift[m]) * MOM_STRIDE + q, (unsigned long long)val);
+        }
+        __syncwarp();
     }
 }
 
@@ -2222,11 +2248,12 @@ __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const d
 __global__ void __launch_bounds__(256) k_mom_fold(int64_t nn, unsigned long long *acc, const double *scale,
                                                   double *mom) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= NMOM * nn) return;
-    const int q = (int)(t / nn);
+    const int q = (int)(t % MOM_STRIDE);
+    const int64_t u = t / MOM_STRIDE;
+    if (u >= nn || q >= NMOM) return;
     const long long c = (long long)acc[t];
     if (c) {
-        mom[t] += (double)c * scale[NMOM + q];
+        mom[q * nn + u] += (double)c * scale[NMOM + q];
         acc[t] = 0;
     }
 }
@@ -2359,8 +2386,8 @@ void launch_moments(World &w, Species &s) {
     k_mom_scale<<<1, 32, 0, w.stream>>>(s.mom_bound, w0, s.d_count, s.mom_scale, w.d_err);
     if (n > 0)
         k_mom_scatter<<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, rcp_dh(w), s.P, s.cap, w0, s.d_count,
-                                                                 s.mom_scale, s.mom_acc, w.nn, w.d_err);
-    k_mom_fold<<<blocks_for(NMOM * w.nn, 256), 256, 0, w.stream>>>(w.nn, s.mom_acc, s.mom_scale, s.mom);
+                                                                 s.mom_scale, s.mom_acc, w.d_err);
+    k_mom_fold<<<blocks_for(MOM_STRIDE * w.nn, 256), 256, 0, w.stream>>>(w.nn, s.mom_acc, s.mom_scale, s.mom);
     w.nlaunch += 2 + 2 * (n > 0);
 }
 
@@ -2425,59 +2452,110 @@ struct Ch4Uniforms {
     }
 };
 
+/* LATER: particles whose whole step may be needed (near the sphere, no time
+ * left, not finite) are listed and k_advance_ch4_rest takes them; one of
+ * them in a warp would make the warp issue a bounce's float64 work (sines,
+ * roots, quotients) for one lane.  Without it (the caller gives times or
+ * uniforms) every particle takes the whole step here.  6.4M atoms around
+ * the sphere: 587 us a call in one kernel, 239 us now. */
+template <bool LATER>
 __global__ void __launch_bounds__(256) k_advance_ch4(Ch4Geo G, SphereReject far, double mass, double dt, double *P,
-                                                     int64_t stride,
-                                                     const int64_t *__restrict__ d_count,
+                                                     int64_t stride, const int64_t *__restrict__ d_count,
                                                      const int64_t *__restrict__ d_settled,
                                                      const double *__restrict__ pdt, const double *__restrict__ u,
                                                      int64_t nu, const int64_t *__restrict__ p_off, uint64_t seed,
                                                      uint64_t stream, uint32_t *deadmask, int32_t *tiledead,
-                                                     unsigned long long *nbounce, int *err) {
+                                                     unsigned long long *nbounce, int32_t *later,
+                                                     unsigned long long *nlater, int *err) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n = d_count[0];
-    bool dead = false;
+    const int lane = threadIdx.x & 31;
+    bool dead = false, wait = false;
     int b = 0;
     if (p < n) {
         double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
         double v[3] = {P[3 * stride + p], P[4 * stride + p], P[5 * stride + p]};
         const double t = (pdt ? pdt[p] : (p >= d_settled[0] ? dt : 0.0)) + dt;
-        Ch4Uniforms U{u, nu, u ? p_off[p] : 0, seed, stream, (uint64_t)p << 10, false};
-        bool alive = true;
-        /* most particles move once and strike nothing: the bounds by integer
-         * keys and the sphere by a float distance; the others, and those
-         * near the sphere, take the whole step from where they were */
-        double y[3];
-        bool simple = order_key(t) > 0 && finite_bits(t);
+        if (LATER) {
+            /* most particles move once: the bounds by integer keys, the
+             * sphere by a float distance */
+            bool fine = order_key(t) > 0 && finite_bits(t);
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            y[d] = x[d] + v[d] * t;
-            const long long k = order_key(y[d]);
-            simple = simple && k >= order_key(G.x0[d]) && k < order_key(G.xm[d]);
-        }
-        if (simple && surely_outside(far.c, far.rej2, y)) {
-#pragma unroll
-            for (int d = 0; d < 3; d++) x[d] = y[d];
+            for (int d = 0; d < 3; d++) {
+                x[d] += v[d] * t;
+                const long long k = order_key(x[d]);
+                fine = fine && finite_bits(x[d]);
+                dead = dead || k < order_key(G.x0[d]) || k >= order_key(G.xm[d]);
+            }
+            wait = !fine || (!dead && !surely_outside(far.c, far.rej2, x));
+            dead = dead && !wait;
+            if (!wait)
+                for (int d = 0; d < 3; d++) P[d * stride + p] = x[d];
         } else {
+            Ch4Uniforms U{u, nu, u ? p_off[p] : 0, seed, stream, (uint64_t)p << 10, false};
+            bool alive = true;
             b = ch4_advance_one(G, mass, t, x, v, U, alive, 64);
+            if (U.bad) atomicOr(err, DERR_NEUTRAL);
+            if (!(finite_bits(x[0]) && finite_bits(x[1]) && finite_bits(x[2]))) {
+                atomicOr(err, DERR_NONFINITE);
+                alive = false;
+            }
+            dead = !alive;
+            for (int d = 0; d < 3; d++) {
+                P[d * stride + p] = x[d];
+                P[(3 + d) * stride + p] = v[d];
+            }
         }
-        if (U.bad) atomicOr(err, DERR_NEUTRAL);
+    }
+    if (LATER) {
+        const unsigned w = __ballot_sync(0xffffffffu, wait);
+        unsigned long long base = 0;
+        if (lane == 0 && w) base = atomicAdd(nlater, (unsigned long long)__popc(w));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (wait) later[base + __popc(w & ((1u << lane) - 1u))] = (int32_t)p;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, dead);
+    int bs = b;
+    if (!LATER)
+        for (int o = 16; o; o >>= 1) bs += __shfl_xor_sync(0xffffffffu, bs, o);
+    if (lane == 0 && p < n) {
+        deadmask[p >> 5] = m;
+        if (m) atomicAdd(tiledead + (p / TILE_PARTICLES), __popc(m));
+        if (bs) atomicAdd(nbounce, (unsigned long long)bs);
+    }
+}
+
+/* the whole step of the particles that k_advance_ch4 listed, which it left
+ * where they were; the order of the list does not matter (each particle
+ * draws from its own counters) */
+__global__ void __launch_bounds__(256) k_advance_ch4_rest(Ch4Geo G, double mass, double dt, double *P, int64_t stride,
+                                                          const int64_t *__restrict__ d_settled, uint64_t seed,
+                                                          uint64_t stream, uint32_t *deadmask, int32_t *tiledead,
+                                                          unsigned long long *nbounce,
+                                                          const int32_t *__restrict__ later,
+                                                          const unsigned long long *__restrict__ nlater, int *err) {
+    const int64_t n = (int64_t)nlater[0];
+    for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t0 < n; t0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = later[t0];
+        double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
+        double v[3] = {P[3 * stride + p], P[4 * stride + p], P[5 * stride + p]};
+        const double t = (p >= d_settled[0] ? dt : 0.0) + dt;
+        Ch4Uniforms U{nullptr, 0, 0, seed, stream, (uint64_t)p << 10, false};
+        bool alive = true;
+        const int b = ch4_advance_one(G, mass, t, x, v, U, alive, 64);
         if (!(finite_bits(x[0]) && finite_bits(x[1]) && finite_bits(x[2]))) {
             atomicOr(err, DERR_NONFINITE);
             alive = false;
         }
-        dead = !alive;
         for (int d = 0; d < 3; d++) {
             P[d * stride + p] = x[d];
             P[(3 + d) * stride + p] = v[d];
         }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, dead);
-    int bs = b;
-    for (int o = 16; o; o >>= 1) bs += __shfl_xor_sync(0xffffffffu, bs, o);
-    if ((threadIdx.x & 31) == 0 && p < n) {
-        deadmask[p >> 5] = m;
-        if (m) atomicAdd(tiledead + (p / TILE_PARTICLES), __popc(m));
-        if (bs) atomicAdd(nbounce, (unsigned long long)bs);
+        if (!alive) {
+            atomicOr(deadmask + (p >> 5), 1u << (p & 31));
+            atomicAdd(tiledead + (p / TILE_PARTICLES), 1);
+        }
+        if (b) atomicAdd(nbounce, (unsigned long long)b);
     }
 }
 
@@ -2499,10 +2577,19 @@ void launch_advance_ch4(World &w, Species &s, double dt, const double *d_pdt, co
         /* one stream per (species, call) */
         const uint64_t stream = (0xC4ull << 56) | ((uint64_t)(s.id & 0xff) << 48) |
                                 (s.ch4_calls & 0xffffffffffffull);
-        k_advance_ch4<<<blocks_for(n, 256), 256, 0, w.stream>>>(G, sphere_reject(w), s.mass, dt, s.P, s.cap, s.d_count, s.ch4_settled,
-                                                                 d_pdt, d_u, nu, d_off, w.seed, stream, s.deadmask,
-                                                                 s.tiledead, s.ch4_bounces, w.d_err);
-        w.nlaunch++;
+        const bool later = !d_pdt && !d_u;
+        /* the compaction's hole list and the count's fourth word are free here */
+        unsigned long long *nlater = (unsigned long long *)(s.d_count + 3);
+        if (later) cudaMemsetAsync(nlater, 0, sizeof *nlater, w.stream);
+        auto *fn = later ? k_advance_ch4<true> : k_advance_ch4<false>;
+        fn<<<blocks_for(n, 256), 256, 0, w.stream>>>(G, sphere_reject(w), s.mass, dt, s.P, s.cap, s.d_count,
+                                                     s.ch4_settled, d_pdt, d_u, nu, d_off, w.seed, stream, s.deadmask,
+                                                     s.tiledead, s.ch4_bounces, s.holes, nlater, w.d_err);
+        if (later)
+            k_advance_ch4_rest<<<2 * w.sm_count, 256, 0, w.stream>>>(G, s.mass, dt, s.P, s.cap, s.ch4_settled, w.seed,
+                                                                     stream, s.deadmask, s.tiledead, s.ch4_bounces,
+                                                                     s.holes, nlater, w.d_err);
+        w.nlaunch += later ? 2 : 1;
         launch_compact(w, s);
     }
     k_ch4_settle<<<1, 1, 0, w.stream>>>(s.d_count, s.ch4_settled);
