@@ -135,6 +135,7 @@ struct World {
     int64_t mg_block_nodes = 4096; /* multigrid levels smaller than this run on one block */
     int64_t mg_dense_max = 1024;   /* coarsest level solved by its dense inverse when it has at most this
                                       many nodes (0: smoothing sweeps on block 0) */
+    int sor_cluster = -1;   /* whether the device takes k_sor_cluster's cluster (-1: not asked yet) */
     int solver_blocks = 0;  /* cap on cooperative solver blocks (0: occupancy limit) */
     double *phi_prev = nullptr;    /* the potential before the last Newton solve (predictor) */
     bool phi_prev_valid = false;

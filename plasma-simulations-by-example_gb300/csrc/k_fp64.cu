@@ -1029,22 +1029,28 @@ __global__ void __launch_bounds__(RED_THREADS) k_diag_partials(const double *__r
     block_sum_store<5>(acc, partials + 5 * blockIdx.x);
 }
 
-/* final sums by one warp: lane l adds partials l, l+32, ... in order, then a
- * fixed butterfly; the same bits on every run */
-__global__ void k_diag_final(const double *__restrict__ partials, double mass, double *out) {
-    int lane = threadIdx.x & 31;
-    double s[5] = {0, 0, 0, 0, 0};
-    for (int b = lane; b < RED_BLOCKS; b += 32)
-        for (int q = 0; q < 5; q++) s[q] += partials[5 * b + q];
-    for (int q = 0; q < 5; q++)
-        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
-    if (threadIdx.x == 0) {
-        out[0] = s[0];
-        out[1] = s[1] * mass;
-        out[2] = s[2] * mass;
-        out[3] = s[3] * mass;
-        out[4] = 0.5 * mass * s[4];
-    }
+/* A warp's sum of partials[q + nv * b] over the blocks b: lane l adds blocks
+ * l, l+32, ... in order, then a fixed butterfly; the same bits on every run.
+ * Every load is issued before the additions (one memory latency instead of
+ * nineteen: 15 us as a loop). */
+__device__ __forceinline__ double warp_final(const double *__restrict__ partials, int nv, int q) {
+    constexpr int R = (RED_BLOCKS + 31) / 32;
+    const int lane = threadIdx.x & 31;
+    double x[R], s = 0;
+#pragma unroll
+    for (int i = 0; i < R; i++) x[i] = lane + 32 * i < RED_BLOCKS ? partials[nv * (lane + 32 * i) + q] : 0.0;
+#pragma unroll
+    for (int i = 0; i < R; i++)
+        if (lane + 32 * i < RED_BLOCKS) s += x[i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+/* five warps, one per sum */
+__global__ void __launch_bounds__(160) k_diag_final(const double *__restrict__ partials, double mass, double *out) {
+    const int q = threadIdx.x >> 5;
+    const double s = warp_final(partials, 5, q);
+    if ((threadIdx.x & 31) == 0) out[q] = q == 0 ? s : (q == 4 ? 0.5 * mass * s : s * mass);
 }
 
 __global__ void __launch_bounds__(RED_THREADS) k_pe_partials(int64_t nn, const double *__restrict__ ef,
@@ -1074,10 +1080,7 @@ __global__ void __launch_bounds__(1024) k_pe_sum(const double *__restrict__ part
 }
 
 __global__ void k_pe_final(const double *__restrict__ partials, double *out) {
-    int lane = threadIdx.x & 31;
-    double s = 0;
-    for (int b = lane; b < RED_BLOCKS; b += 32) s += partials[b];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const double s = warp_final(partials, 1, 0);
     if (threadIdx.x == 0) out[0] = 0.5 * EPS_0 * s;
 }
 
@@ -1127,46 +1130,128 @@ __device__ __forceinline__ bool colour_node(const Geo &g, const ColourRange &cr,
     return i <= g.ni - 2;
 }
 
-__global__ void __launch_bounds__(256) k_sor_box(Geo g, double *phi, const double *__restrict__ rho, int max_it,
-                                                 double tol, double *partials, SolveStatus *st, int *err) {
+/* What a node of the linear box needs in every sweep: its index and rho /
+ * eps0, read once. */
+struct SorNode {
+    int32_t u; /* -1: none */
+    double b;
+};
+
+/* constants of the sweeps; rD = RN(1 / D), D the divisor of the node formula */
+struct SorConst {
+    double idx2, idy2, idz2, D, rD, eps0, reps0;
+};
+
+static SorConst sor_const(const Geo &g) {
+    SorConst c;
+    c.idx2 = 1.0 / (g.dh[0] * g.dh[0]);
+    c.idy2 = 1.0 / (g.dh[1] * g.dh[1]);
+    c.idz2 = 1.0 / (g.dh[2] * g.dh[2]);
+    c.D = 2 * c.idx2 + 2 * c.idy2 + 2 * c.idz2;
+    c.rD = 1.0 / c.D;
+    c.eps0 = EPS_0;
+    c.reps0 = 1.0 / EPS_0;
+    return c;
+}
+
+/* entry t (below n) of colour c's enumeration */
+__device__ __forceinline__ SorNode sor_node(const Geo &g, const SorConst &k, uint32_t hx, uint32_t t, uint32_t n,
+                                            int c, const double *__restrict__ rho) {
+    SorNode s = {-1, 0.0};
+    if (t >= n) return s;
+    const uint32_t row = div_small(t, hx, 1.f / (float)hx);
+    const uint32_t kk = div_small(row, (uint32_t)(g.nj - 2), 1.f / (float)(g.nj - 2));
+    const int j = 1 + (int)(row - kk * (uint32_t)(g.nj - 2)), z = 1 + (int)kk;
+    const int i = 1 + 2 * (int)(t - row * hx) + ((1 + j + z + c) & 1);
+    if (i > g.ni - 2) return s;
+    s.u = (z * g.nj + j) * g.ni + i;
+    s.b = div_rcp(rho[s.u], k.eps0, k.reps0);
+    return s;
+}
+
+/* the updated value of a node (operand order of ch2/PotentialSolver.cpp:27-42) */
+template <class P>
+__device__ __forceinline__ double sor_value(const SorConst &k, const P *phi, const SorNode &s, int32_t sy, int32_t sz) {
+    const double x = phi[s.u];
+    const double num = s.b + k.idx2 * (phi[s.u - 1] + phi[s.u + 1]) + k.idy2 * (phi[s.u - sy] + phi[s.u + sy]) +
+                       k.idz2 * (phi[s.u - sz] + phi[s.u + sz]);
+    return x + 1.4 * (div_rcp(num, k.D, k.rD) - x);
+}
+
+/* the square of a node's residual (ch2/PotentialSolver.cpp:44-61) */
+template <class P>
+__device__ __forceinline__ double sor_residual2(const SorConst &k, const P *phi, const SorNode &s, int32_t sy,
+                                                int32_t sz) {
+    if (s.u < 0) return 0.0;
+    const double R = -phi[s.u] * k.D + s.b + k.idx2 * (phi[s.u - 1] + phi[s.u + 1]) +
+                     k.idy2 * (phi[s.u - sy] + phi[s.u + sy]) + k.idz2 * (phi[s.u - sz] + phi[s.u + sz]);
+    return R * R;
+}
+
+__device__ __forceinline__ void sor_status(SolveStatus *st, int conv, int it, double L2) {
+    st->converged = conv;
+    st->iterations = conv ? it + 1 : it;
+    st->inner_iterations = 0;
+    st->residual = L2;
+    st->solves += 1;
+    st->outer_total += st->iterations;
+}
+
+/* The sweeps on the whole grid.  Up to SOR_HELD nodes of a colour per thread
+ * are held in registers (index and rho / eps0); beyond, they are found
+ * again in every sweep.  Bound by the barrier after each half sweep (1.3 us)
+ * and the memory latency behind it (23x47x37: 4.6 us a sweep).  With 64-bit
+ * integer divisions and two float64 divisions per node a sweep of the 21^3
+ * box took 7.5 us on 15 SMs. */
+constexpr int SOR_HELD = 2;
+
+__global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi, const double *__restrict__ rho,
+                                                 int max_it, double tol, double *partials, SolveStatus *st,
+                                                 int *err) {
     cg::grid_group grid = cg::this_grid();
-    const double idx2 = 1.0 / (g.dh[0] * g.dh[0]);
-    const double idy2 = 1.0 / (g.dh[1] * g.dh[1]);
-    const double idz2 = 1.0 / (g.dh[2] * g.dh[2]);
-    const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    ColourRange cr;
-    cr.hx = (g.ni - 2 + 1) / 2;
-    cr.count = (int64_t)cr.hx * (g.nj - 2) * (g.nk - 2);
-    const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t gsize = (int64_t)gridDim.x * blockDim.x;
-    const int64_t interior = (int64_t)(g.ni - 2) * (g.nj - 2) * (g.nk - 2);
+    const int32_t sy = g.ni, sz = g.ni * g.nj;
+    const uint32_t hx = (uint32_t)(g.ni - 1) / 2;
+    const uint32_t count = hx * (uint32_t)(g.nj - 2) * (uint32_t)(g.nk - 2);
+    const uint32_t gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool held = count <= SOR_HELD * gsize;
+    SorNode node[2][SOR_HELD];
+    if (held)
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int h = 0; h < SOR_HELD; h++) node[c][h] = sor_node(g, k, hx, gtid + h * gsize, count, c, rho);
     double L2 = 0;
     int conv = 0, it, round = 0;
     for (it = 0; it < max_it; it++) {
+#pragma unroll
         for (int c = 0; c < 2; c++) {
-            for (int64_t t = gtid; t < cr.count; t += gsize) {
-                int i, j, k;
-                if (!colour_node(g, cr, t, c, i, j, k)) continue;
-                int64_t u = node_of(g, i, j, k);
-                double phi_new = (rho[u] / EPS_0 + idx2 * (phi[u - 1] + phi[u + 1]) +
-                                  idy2 * (phi[u - sy] + phi[u + sy]) + idz2 * (phi[u - sz] + phi[u + sz])) /
-                                 (2 * idx2 + 2 * idy2 + 2 * idz2);
-                phi[u] = phi[u] + 1.4 * (phi_new - phi[u]);
+            if (held) {
+                double v[SOR_HELD];
+#pragma unroll
+                for (int h = 0; h < SOR_HELD; h++)
+                    if (node[c][h].u >= 0) v[h] = sor_value(k, phi, node[c][h], sy, sz);
+#pragma unroll
+                for (int h = 0; h < SOR_HELD; h++)
+                    if (node[c][h].u >= 0) phi[node[c][h].u] = v[h];
+            } else {
+                for (uint32_t t = gtid; t < count; t += gsize) {
+                    const SorNode s = sor_node(g, k, hx, t, count, c, rho);
+                    if (s.u >= 0) phi[s.u] = sor_value(k, phi, s, sy, sz);
+                }
             }
             grid.sync();
         }
         if (it % 25 == 0) {
             double sum = 0;
-            for (int64_t t = gtid; t < interior; t += gsize) {
-                int i = 1 + (int)(t % (g.ni - 2));
-                int64_t r = t / (g.ni - 2);
-                int j = 1 + (int)(r % (g.nj - 2));
-                int k = 1 + (int)(r / (g.nj - 2));
-                int64_t u = node_of(g, i, j, k);
-                double R = -phi[u] * (2 * idx2 + 2 * idy2 + 2 * idz2) + rho[u] / EPS_0 +
-                           idx2 * (phi[u - 1] + phi[u + 1]) + idy2 * (phi[u - sy] + phi[u + sy]) +
-                           idz2 * (phi[u - sz] + phi[u + sz]);
-                sum += R * R;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                if (held) {
+#pragma unroll
+                    for (int h = 0; h < SOR_HELD; h++) sum += sor_residual2(k, phi, node[c][h], sy, sz);
+                } else {
+                    for (uint32_t t = gtid; t < count; t += gsize)
+                        sum += sor_residual2(k, phi, sor_node(g, k, hx, t, count, c, rho), sy, sz);
+                }
             }
             double tot = grid_sum(grid, sum, partials, round);
             L2 = sqrt(tot / ((double)g.ni * g.nj * g.nk));
@@ -1180,14 +1265,79 @@ __global__ void __launch_bounds__(256) k_sor_box(Geo g, double *phi, const doubl
             }
         }
     }
-    if (gtid == 0) {
-        st->converged = conv;
-        st->iterations = conv ? it + 1 : it;
-        st->inner_iterations = 0;
-        st->residual = L2;
-        st->solves += 1;
-        st->outer_total += st->iterations;
+    if (gtid == 0) sor_status(st, conv, it, L2);
+}
+
+/* The sweeps of a small box in one cluster of SOR_CTAS blocks: each holds the
+ * potential in shared memory, works an even share of each colour's nodes and
+ * writes every new value into the blocks whose nodes may read it (reach
+ * blocks on either side: a node's neighbours lie at most a plane of entries
+ * away), so that a half sweep costs a cluster barrier (0.3 us) and no
+ * memory latency.  The shares' float64 work bounds it (15 instructions a
+ * node on SOR_CTAS SMs).  A sweep of the 21^3 box: 4.8 us, 5.2 us on the
+ * whole grid, 7.5 us before either; of 17x17x15: 2.4 and 3.5 us. */
+constexpr int SOR_CTAS = 16, SOR_CTA_NODES = 384;
+
+__global__ void __launch_bounds__(SOR_CTA_NODES) k_sor_cluster(Geo g, SorConst k, double *phi,
+                                                               const double *__restrict__ rho, int max_it, double tol,
+                                                               uint32_t per, int reach, SolveStatus *st, int *err) {
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) double sor_phi[];
+    __shared__ double part[2][SOR_CTAS];
+    __shared__ double warp_sum[SOR_CTA_NODES / 32];
+    const int rank = (int)cl.block_rank();
+    const int32_t sy = g.ni, sz = g.ni * g.nj, nn = sz * g.nk;
+    const uint32_t hx = (uint32_t)(g.ni - 1) / 2;
+    const uint32_t count = hx * (uint32_t)(g.nj - 2) * (uint32_t)(g.nk - 2);
+    const uint32_t t = (uint32_t)rank * per + threadIdx.x;
+    const uint32_t top = threadIdx.x < per ? count : 0u;
+    const SorNode node[2] = {sor_node(g, k, hx, t, top, 0, rho), sor_node(g, k, hx, t, top, 1, rho)};
+    for (int32_t u = threadIdx.x; u < nn; u += blockDim.x) sor_phi[u] = phi[u];
+    cl.sync();
+    double L2 = 0;
+    int conv = 0, it, round = 0;
+    for (it = 0; it < max_it; it++) {
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            if (node[c].u >= 0) {
+                const double v = sor_value(k, sor_phi, node[c], sy, sz);
+                sor_phi[node[c].u] = v;
+                for (int d = 1; d <= reach; d++) {
+                    if (rank - d >= 0) cl.map_shared_rank(sor_phi, rank - d)[node[c].u] = v;
+                    if (rank + d < SOR_CTAS) cl.map_shared_rank(sor_phi, rank + d)[node[c].u] = v;
+                }
+            }
+            cl.sync();
+        }
+        if (it % 25 == 0) {
+            double sum = sor_residual2(k, sor_phi, node[0], sy, sz) + sor_residual2(k, sor_phi, node[1], sy, sz);
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+            __syncthreads();
+            if (threadIdx.x < SOR_CTAS) {
+                double s = 0;
+                for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += warp_sum[w];
+                cl.map_shared_rank(&part[round & 1][0], threadIdx.x)[rank] = s;
+            }
+            cl.sync();
+            double tot = 0;
+            for (int r = 0; r < SOR_CTAS; r++) tot += part[round & 1][r];
+            round++;
+            L2 = sqrt(tot / ((double)g.ni * g.nj * g.nk));
+            if (!isfinite(L2)) {
+                if (t == 0) atomicOr(err, DERR_NONFINITE);
+                break;
+            }
+            if (L2 < tol) {
+                conv = 1;
+                break;
+            }
+        }
     }
+    for (int c = 0; c < 2; c++)
+        if (node[c].u >= 0) phi[node[c].u] = sor_phi[node[c].u];
+    if (t == 0) sor_status(st, conv, it, L2);
+    cl.sync(); /* no block leaves while another may still write into it */
 }
 
 /* Red-black form of solveGS: red then black interior non-Dirichlet nodes with
@@ -1654,7 +1804,7 @@ void launch_diag(World &w, Species &s, double *d_out5) {
     }
     k_diag_partials<0><<<RED_BLOCKS, RED_THREADS, 0, w.stream>>>(s.P, nullptr, s.cap, s.d_count, s.uniform_w,
                                                                  s.mpw0, w.d_partials);
-    k_diag_final<<<1, 32, 0, w.stream>>>(w.d_partials, s.mass, d_out5);
+    k_diag_final<<<1, 160, 0, w.stream>>>(w.d_partials, s.mass, d_out5);
     w.nlaunch += 2;
 }
 
@@ -1997,18 +2147,70 @@ static int coop_grid(World &w, const void *fn, int threads, int64_t work) {
     return g;
 }
 
+/* The cluster form fits when a block's share is one node of each colour per
+ * thread, the potential fits its shared memory, and the device takes such a
+ * cluster (asked once per world; an upper bound on the solver's blocks below
+ * the cluster's size asks for the grid form). */
+static bool sor_cluster_fits(World &w, uint32_t per, size_t smem) {
+    if (per > SOR_CTA_NODES || smem > 200 * 1024) return false;
+    if (w.solver_blocks > 0 && w.solver_blocks < SOR_CTAS) return false;
+    if (w.sor_cluster < 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(SOR_CTAS);
+        cfg.blockDim = dim3(SOR_CTA_NODES);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute a;
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = SOR_CTAS;
+        a.val.clusterDim.y = a.val.clusterDim.z = 1;
+        cfg.attrs = &a;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const bool ok =
+            cudaFuncSetAttribute(k_sor_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(k_sor_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&n, k_sor_cluster, &cfg) == cudaSuccess;
+        if (!ok) (void)cudaGetLastError();
+        w.sor_cluster = ok && n > 0;
+    }
+    return w.sor_cluster == 1;
+}
+
 int launch_sor_box(World &w, int max_it, double tol) {
-    int64_t work = (int64_t)((w.g.ni - 1) / 2) * (w.g.nj - 2) * (w.g.nk - 2);
-    int grid = coop_grid(w, (const void *)k_sor_box, 256, work);
+    const uint32_t plane = (uint32_t)((w.g.ni - 1) / 2) * (uint32_t)(w.g.nj - 2);
+    int64_t work = (int64_t)plane * (w.g.nk - 2);
     Geo g = w.g;
+    SorConst k = sor_const(g);
     double *phi = w.phi;
     const double *rho = w.rho;
     double *part = w.d_partials;
     SolveStatus *st = w.d_status;
     int *err = w.d_err;
-    void *args[] = {&g, &phi, &rho, &max_it, &tol, &part, &st, &err};
     w.nlaunch++;
-    return (int)cudaLaunchCooperativeKernel((const void *)k_sor_box, grid, 256, args, 0, w.stream);
+    const uint32_t per = (uint32_t)((work + SOR_CTAS - 1) / SOR_CTAS);
+    const size_t smem = (size_t)w.nn * sizeof(double);
+    if (work <= (int64_t)SOR_CTAS * SOR_CTA_NODES && sor_cluster_fits(w, per, smem)) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(SOR_CTAS);
+        cfg.blockDim = dim3((per + 31u) & ~31u);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = w.stream;
+        cudaLaunchAttribute a;
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = SOR_CTAS;
+        a.val.clusterDim.y = a.val.clusterDim.z = 1;
+        cfg.attrs = &a;
+        cfg.numAttrs = 1;
+        const int reach = (int)((per + plane) / per);
+        return (int)cudaLaunchKernelEx(&cfg, k_sor_cluster, g, k, phi, rho, max_it, tol, per, reach, st, err);
+    }
+    /* a node of a colour per thread over all SMs, before blocks grow */
+    int threads = (int)((work + w.sm_count - 1) / w.sm_count + 31) & ~31;
+    threads = threads < 64 ? 64 : (threads > 256 ? 256 : threads);
+    int grid = coop_grid(w, (const void *)k_sor_box, threads, work);
+    void *args[] = {&g, &k, &phi, &rho, &max_it, &tol, &part, &st, &err};
+    return (int)cudaLaunchCooperativeKernel((const void *)k_sor_box, grid, threads, args, 0, w.stream);
 }
 
 int launch_gs_sphere(World &w, int max_it, double tol) {
