@@ -623,6 +623,35 @@ __global__ void __launch_bounds__(256) k_deposit_mixed(MixArgs a, const int32_t 
 }
 
 /* ---------------------------------------------------------------------- */
+/* The eight corner counts of a warp's particles into acc by 64-bit atomics,
+ * two neighbouring lanes to the two x corners of one particle: they lie side
+ * by side, mostly in one 32-byte sector, so an atomic instruction touches
+ * about 20 sectors instead of 32 (30M particles of 64 boxes, push and
+ * deposit: 1.80 ms with a lane's own eight corners, 1.19 ms now).  n0: the cell's first node; a particle that
+ * is not live deposits nothing.  Every lane of the warp calls it. */
+__device__ __forceinline__ void deposit_pairs(unsigned long long *acc, int32_t n0, int64_t sy, int64_t sz, bool live,
+                                              float fx, float fy, float fz) {
+    const unsigned FULL = 0xffffffffu;
+    const bool odd = threadIdx.x & 1;
+    float w[8];
+    cic_w(fx, fy, fz, w);
+    const int32_t mate = __shfl_xor_sync(FULL, n0, 1);
+    const int64_t ne = odd ? mate : n0, no = odd ? n0 : mate; /* the even and the odd lane's particle */
+    /* corner pairs (low x, high x) of Field_::gather's order, by row */
+    const int lo[4] = {0, 3, 4, 7}, hi[4] = {1, 2, 5, 6};
+    const int64_t row[4] = {0, sy, sz, sy + sz};
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const unsigned ql = live ? __float2uint_rn(w[lo[r]] * MIX_Q) : 0u;
+        const unsigned qh = live ? __float2uint_rn(w[hi[r]] * MIX_Q) : 0u;
+        /* the even lane takes low corners, the odd lane high ones */
+        const unsigned got = __shfl_xor_sync(FULL, odd ? ql : qh, 1);
+        const unsigned even_count = odd ? got : ql, odd_count = odd ? qh : got;
+        if (even_count) atomicAdd(acc + ne + row[r] + odd, (unsigned long long)even_count);
+        if (odd_count) atomicAdd(acc + no + row[r] + odd, (unsigned long long)odd_count);
+    }
+}
+
 /* Batched ensemble: push (reflecting walls, the ch2 box) and CIC deposit of
  * every box and species in one launch over a flattened work list.  Work item
  * w = (segment, first particle, count) lies inside one species of one box;
@@ -654,35 +683,32 @@ __global__ void __launch_bounds__(512) k_ens_push(const EnsBox *__restrict__ box
         const float4 *E = ef4 + B.node0;
         unsigned long long *A = acc + (int64_t)sg.sp * total_nodes + B.node0;
         const int64_t sy = a.ni, sz = (int64_t)a.ni * a.nj;
-        for (int q = threadIdx.x; q < W.z; q += blockDim.x) {
+        for (int base = threadIdx.x & ~31; base < W.z; base += blockDim.x) { /* whole warps */
+            const int q = base + (threadIdx.x & 31);
             const int64_t p = sg.p0 + W.y + q;
-            int32_t key = cell[p];
-            float fx = off[p], fy = off[stride + p], fz = off[2 * stride + p];
-            bool dead = false;
-            if (PUSH) {
-                float vx = vel[p], vy = vel[stride + p], vz = vel[2 * stride + p];
-                dead = push_particle_mixed<M_REFLECT>(a, E, key, fx, fy, fz, vx, vy, vz, err);
-                cell[p] = key;
-                off[p] = fx;
-                off[stride + p] = fy;
-                off[2 * stride + p] = fz;
-                vel[p] = vx;
-                vel[stride + p] = vy;
-                vel[2 * stride + p] = vz;
+            int32_t key = 0;
+            float fx = 0.f, fy = 0.f, fz = 0.f;
+            bool live = q < W.z;
+            if (live) {
+                key = cell[p];
+                fx = off[p];
+                fy = off[stride + p];
+                fz = off[2 * stride + p];
+                if (PUSH) {
+                    float vx = vel[p], vy = vel[stride + p], vz = vel[2 * stride + p];
+                    live = !push_particle_mixed<M_REFLECT>(a, E, key, fx, fy, fz, vx, vy, vz, err);
+                    cell[p] = key;
+                    off[p] = fx;
+                    off[stride + p] = fy;
+                    off[2 * stride + p] = fz;
+                    vel[p] = vx;
+                    vel[stride + p] = vy;
+                    vel[2 * stride + p] = vz;
+                }
             }
-            if (dead) continue;
             int i, j, k;
             unpack(key, i, j, k);
-            const int64_t n0 = (int64_t)k * sz + (int64_t)j * sy + i;
-            const int64_t idx[8] = {n0,      n0 + 1,      n0 + 1 + sy,      n0 + sy,
-                                    n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
-            float w[8];
-            cic_w(fx, fy, fz, w);
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                unsigned qc = __float2uint_rn(w[c] * MIX_Q);
-                if (qc) atomicAdd(A + idx[c], (unsigned long long)qc);
-            }
+            deposit_pairs(A, (k * a.nj + j) * a.ni + i, sy, sz, live, fx, fy, fz);
         }
     }
 }

@@ -219,3 +219,41 @@ def test_sharded_ensemble_matches_whole(espic):
     for b in range(nb):
         for a, c in zip(whole[b], parts[b]):
             assert np.array_equal(a, c), b
+
+
+@pytest.mark.parametrize("cluster", [1, 8])
+@pytest.mark.parametrize("nodes", [(3, 3, 3), (4, 5, 3), (16, 64, 9), (64, 17, 10), (17, 16, 64), (61, 64, 64),
+                                   (120, 118, 20)])
+def test_solve_routes_by_box_shape(espic, po, nodes, cluster):
+    """Boxes at the edges of the shared-memory sweeps: fewer planes than CTAs,
+    rows that fill no whole float4, the correction alone in shared memory,
+    and one too large for it.  The solve meets the reference's test and does
+    not depend on the cluster's size."""
+    x0, xm = [-0.1, -0.1, 0.0], [0.1, 0.1, 0.2]
+    n = 5000
+    mpw = [[1e11 * 0.008 / n, 1e11 * 0.001 / n]]
+
+    def solved(cl):
+        E = espic.Ensemble([list(nodes)], x0, xm, MASS, CHARGE, mpw, [[n, n]], 2e-10)
+        with E:
+            E.set_launch(4096, 256, 1024, cl)
+            for sp in range(2):
+                P = box_state(x0, xm, n, 5 + sp, octant=sp == 1)
+                P[6] = mpw[0][sp]
+                E.set_particles(0, sp, P)
+            E.set_solver(20000, 1e-4, 0.0)
+            E.prepare()
+            E.step(1)
+            E.sync()
+            _, conv, _ = E.status()
+            return E.read(0, espic.FIELD_PHI), E.read(0, espic.FIELD_RHO), E.read(0, espic.FIELD_EF), conv
+
+    phi, rho, ef, conv = solved(cluster)
+    assert conv.all()
+    g = po.grid(nodes, x0, xm)
+    assert np.array_equal(ef, po.efield(g, phi))
+    tight, ok, _, _ = po.sor_box(g, phi, rho, 20000, 1e-9, "rb")
+    assert ok and np.max(np.abs(phi - tight)) <= 1e-5 * np.max(np.abs(tight))
+    other = solved(2)
+    for a, b in zip((phi, rho, ef), other):
+        assert np.array_equal(a, b)
