@@ -766,10 +766,20 @@ __global__ void __launch_bounds__(256) k_efield(Geo g, double3 y2, const double 
  * computeEF).  World::getPE's sum of |E|^2 vol over the nodes rides along
  * from the same q, in double-float (each term within 2^-44 of the float64
  * term, far inside the 1e-13 to which the sum's order already defines it).
- * Each thread takes EF_KPT planes of its (i, j) column, so the block sum is
- * paid once per EF_KPT nodes: one partial per block, [plane group][block of
+ * Each thread takes kpt planes of its (i, j) column, so the block sum is
+ * paid once per kpt nodes: one partial per block, [plane group][block of
  * the plane]. */
-constexpr int EF_KPT = 8; /* planes per thread of k_efield4 */
+/* Most planes per thread of k_efield4.  A smaller grid takes fewer, down to
+ * one, until it has four blocks per SM: with eight, 64x64x128 nodes made 256
+ * blocks of eight float64 nodes one after the other (65 us a call, 41 now;
+ * 33x29x65: 28 and 12 us). */
+constexpr int EF_KPT = 8;
+
+static int ef_planes_per_thread(const World &w) {
+    const int64_t columns = blocks_for((int64_t)w.g.ni * w.g.nj, 256);
+    int64_t kpt = columns * w.g.nk / (4 * (int64_t)w.sm_count);
+    return (int)(kpt < 1 ? 1 : (kpt > EF_KPT ? EF_KPT : kpt));
+}
 
 struct EfConst {
     double3 y2, d2; /* RN(1 / 2dh) and 2 dh per axis */
@@ -798,7 +808,7 @@ __device__ __noinline__ double ef_node_exact(const double *__restrict__ phi, dou
 
 __global__ void __launch_bounds__(256) k_efield4(Geo g, EfConst ec, const double *__restrict__ phi, double *ef,
                                                  float4 *ef4, const double *__restrict__ vol, double *pe_part,
-                                                 double *phi_ef) {
+                                                 double *phi_ef, int kpt) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t ni = (uint32_t)g.ni, nj = (uint32_t)g.nj, nplane = ni * nj;
     double pe = 0;         /* the nodes of ef_node_exact */
@@ -828,8 +838,8 @@ __global__ void __launch_bounds__(256) k_efield4(Geo g, EfConst ec, const double
         const uint32_t pl = j * ni + i;
         const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
         const bool in_ij = t < nin;
-        const int k0 = blockIdx.y * EF_KPT;
-        for (int kk = 0; kk < EF_KPT; kk++) {
+        const int k0 = blockIdx.y * kpt;
+        for (int kk = 0; kk < kpt; kk++) {
             const int k = k0 + kk;
             if (k >= g.nk) break;
             const int64_t u = (int64_t)k * sz + pl;
@@ -1547,7 +1557,8 @@ void launch_efield(World &w, bool full) {
     /* RN(1 / (2 dh)) per axis, for div_rcp */
     double3 y2 = make_double3(1.0 / (2 * w.g.dh[0]), 1.0 / (2 * w.g.dh[1]), 1.0 / (2 * w.g.dh[2]));
     dim3 grid((unsigned)blocks_for((int64_t)w.g.ni * w.g.nj, 256), (unsigned)w.g.nk);
-    dim3 grid4(grid.x, (unsigned)((w.g.nk + EF_KPT - 1) / EF_KPT));
+    const int kpt = ef_planes_per_thread(w);
+    dim3 grid4(grid.x, (unsigned)((w.g.nk + kpt - 1) / kpt));
     const int64_t nparts = (int64_t)grid4.x * grid4.y;
     if (!full && mixed && !fp64 && !w.phi_ef) {
         /* allocated once per world on the first such call */
@@ -1567,7 +1578,7 @@ void launch_efield(World &w, bool full) {
             const float h = (float)ny[c];
             ec.ny[c] = make_float2(h, (float)(ny[c] - (double)h));
         }
-        k_efield4<<<grid4, 256, 0, w.stream>>>(w.g, ec, w.phi, w.ef, w.ef4, w.vol, w.pe_part, w.phi_ef);
+        k_efield4<<<grid4, 256, 0, w.stream>>>(w.g, ec, w.phi, w.ef, w.ef4, w.vol, w.pe_part, w.phi_ef, kpt);
         w.nlaunch++;
         w.ef4_valid = true;
         w.ef64_valid = false;
@@ -1591,11 +1602,17 @@ void ensure_ef64(World &w) {
     w.ef64_valid = true;
 }
 
+/* Threads per block of the particle kernels whose float64 work an SM runs one
+ * instruction after the other: small counts in small blocks, so that the SMs'
+ * shares differ little (80,000 ions: 313 blocks of 256 put three on some of
+ * 152 SMs and two on most). */
+static int fp64_threads(const World &w, int64_t n) { return n < 4096 * (int64_t)w.sm_count ? 64 : 256; }
+
 template <int WALLS, bool DEP, bool UNI>
-static void push_fp64_as(World &w, Species &s, int blocks) {
+static void push_fp64_as(World &w, Species &s, int blocks, int threads) {
     double sc = w.dt * s.charge / s.mass;
     double4 sph = make_double4(w.sphere[0], w.sphere[1], w.sphere[2], w.has_sphere ? w.sphere[3] : -1.0);
-    k_push_fp64<WALLS, DEP, UNI><<<blocks, 256, 0, w.stream>>>(w.g, w.ef, sc, w.dt, s.P, s.cap, s.d_count, sph,
+    k_push_fp64<WALLS, DEP, UNI><<<blocks, threads, 0, w.stream>>>(w.g, w.ef, sc, w.dt, s.P, s.cap, s.d_count, sph,
                                                               sphere_reject(w), rcp_dh(w), s.deadmask, s.tiledead, s.acc, s.fx, s.mpw0, w.d_err);
     w.nlaunch++;
 }
@@ -1604,32 +1621,33 @@ void launch_push_fp64(World &w, Species &s, bool deposit) {
     int64_t n = s.host_bound;
     if (n <= 0) return;
     ensure_ef64(w);
-    int blocks = blocks_for(n, 256);
+    const int threads = fp64_threads(w, n), blocks = blocks_for(n, threads);
     if (s.walls == 0) {
         if (!deposit)
-            push_fp64_as<REFLECT, false, true>(w, s, blocks);
+            push_fp64_as<REFLECT, false, true>(w, s, blocks, threads);
         else if (s.uniform_w)
-            push_fp64_as<REFLECT, true, true>(w, s, blocks);
+            push_fp64_as<REFLECT, true, true>(w, s, blocks, threads);
         else
-            push_fp64_as<REFLECT, true, false>(w, s, blocks);
+            push_fp64_as<REFLECT, true, false>(w, s, blocks, threads);
     } else {
         if (!deposit)
-            push_fp64_as<ABSORB, false, true>(w, s, blocks);
+            push_fp64_as<ABSORB, false, true>(w, s, blocks, threads);
         else if (s.uniform_w)
-            push_fp64_as<ABSORB, true, true>(w, s, blocks);
+            push_fp64_as<ABSORB, true, true>(w, s, blocks, threads);
         else
-            push_fp64_as<ABSORB, true, false>(w, s, blocks);
+            push_fp64_as<ABSORB, true, false>(w, s, blocks, threads);
     }
 }
 
 void launch_deposit_fp64(World &w, Species &s) {
     int64_t n = s.host_bound;
     if (n <= 0) return;
+    const int threads = fp64_threads(w, n), blocks = blocks_for(n, threads);
     if (s.uniform_w)
-        k_deposit_fp64<true><<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, rcp_dh(w),
+        k_deposit_fp64<true><<<blocks, threads, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, rcp_dh(w),
                                                                        s.acc, s.fx, s.mpw0);
     else
-        k_deposit_fp64<false><<<blocks_for(n, 256), 256, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, rcp_dh(w),
+        k_deposit_fp64<false><<<blocks, threads, 0, w.stream>>>(w.g, s.P, s.cap, s.d_count, rcp_dh(w),
                                                                         s.acc, s.fx, s.mpw0);
     w.nlaunch++;
 }

@@ -144,13 +144,13 @@ static int na_scratch(unsigned long long **out) {
     return ESPIC_OK;
 }
 
-/* a launch of 256-thread blocks that may overlap the tail of the kernel before
- * it on the stream (the kernel itself waits for its results) */
+/* a launch that may overlap the tail of the kernel before it on the stream
+ * (the kernel itself waits for its results) */
 template <class... P, class... A>
-static cudaError_t launch_early(unsigned blocks, cudaStream_t st, void (*fn)(P...), A... args) {
+static cudaError_t launch_early(unsigned blocks, unsigned threads, cudaStream_t st, void (*fn)(P...), A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(threads);
     cfg.stream = st;
     cudaLaunchAttribute early;
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -207,12 +207,14 @@ extern "C" int espic_deposit_noalloc(const double *d_P, int64_t stride, int64_t 
     int S = ex - 1 > 52 ? 52 : ex - 1;
     double fx = ldexp(1.0, S);
     cudaStream_t st = (cudaStream_t)stream;
+    /* small blocks for few particles: an even share of float64 work per SM */
+    const unsigned nt = n < 600000 ? 64 : 256;
     k_na_clear<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, (uint32_t)nn, d_flags);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && n > 0)
-        e = launch_early((unsigned)((n + 255) / 256), st, k_na_deposit, g, d_P, stride, n, fx, weight_bound, acc, d_flags);
+        e = launch_early((unsigned)((n + nt - 1) / nt), nt, st, k_na_deposit, g, d_P, stride, n, fx, weight_bound, acc, d_flags);
     if (e == cudaSuccess)
-        e = launch_early((unsigned)((nn + 255) / 256), st, k_na_density, g, (const unsigned long long *)acc, 1.0 / fx,
+        e = launch_early((unsigned)((nn + 255) / 256), 256, st, k_na_density, g, (const unsigned long long *)acc, 1.0 / fx,
                          d_den);
     if (e != cudaSuccess) {
         char buf[200];
