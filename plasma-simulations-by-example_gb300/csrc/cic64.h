@@ -69,32 +69,90 @@ __device__ __forceinline__ bool cut_float(double x, float &xf) {
     return fe <= 254;
 }
 
-/* Field_::scatter of `value` at cell offsets d, each corner weight
+/* RN(x) as an integer for |x| < 2^62 with integer operations alone (x cut
+ * into mantissa and exponent; ties to even): ~18 of them for one float64
+ * addition, which costs the SM 64 issue slots */
+__device__ __forceinline__ long long round_bits(double x) {
+    const long long b = __double_as_longlong(x);
+    const int s = 1075 - ((int)(b >> 52) & 0x7ff); /* x = m 2^-s */
+    const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | 0x10000000000000ull;
+    unsigned long long q;
+    if (s > 0) {
+        const int t = s > 62 ? 62 : s; /* m < 2^53: 0 beyond */
+        q = (m + ((1ull << (t - 1)) - 1ull) + ((m >> t) & 1ull)) >> t;
+    } else {
+        q = m << -s;
+    }
+    return b < 0 ? -(long long)q : (long long)q;
+}
+
+/* A double's magnitude for round_product: its 53-bit mantissa 10 bits up, and
+ * its exponent field (numbers below 2^-1022 count as 0). */
+struct Mantissa {
+    unsigned long long m;
+    int f;
+};
+
+__device__ __forceinline__ Mantissa mantissa_of(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int f = (int)(b >> 52) & 0x7ff;
+    return {f ? ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10 : 0ull, f};
+}
+
+/* The magnitude of the exact product of two such numbers, rounded to the
+ * nearest integer (ties to even), for products below 2^51: the 128-bit
+ * product of the mantissas (one shifted 11 bits instead of 10, which makes
+ * 21), its lower half folded into a sticky bit.  About 30 integer
+ * operations, half the time of the one float64 FMA that does the same
+ * (RN(a b + 1.5 2^52)). */
+__device__ __forceinline__ unsigned long long round_product(Mantissa a, Mantissa b) {
+    const unsigned long long bm = b.m << 1;
+    unsigned long long h = __umul64hi(a.m, bm);
+    h |= (a.m * bm) != 0ull;
+    const int t = 2107 - (a.f + b.f);
+    if (t > 63) return 0ull;
+    return (h + ((1ull << (t - 1)) - 1ull) + ((h >> t) & 1ull)) >> t;
+}
+
+/* The warp's Field_::scatter of `value` at cell offsets d, each corner weight
  * value*(1-di)*(1-dj)*(1-dk) (the reference's operand order) rounded once to
  * an integer count of 1/fx and added to acc.  fx is a power of two, so it
  * multiplies the value once instead of eight weights.  unit_cell: d lies in
- * [0, 1), so that no weight exceeds the value; a count below 2^50 is then
- * rounded by adding 1.5 * 2^52, which leaves it in the low bits, instead of
- * by a conversion. */
-__device__ __forceinline__ void scatter8(unsigned long long *acc, int64_t n0, int64_t sy, int64_t sz,
-                                         const double d[3], double value, double fx, bool unit_cell) {
-    const double magic = 6755399441055744.0;
+ * [0, 1), so that no weight exceeds the value, whose count below 2^61 is then
+ * rounded by integer operations.  Two neighbouring lanes add to the two x
+ * corners of one particle, which mostly lie in one 32-byte sector.  Every
+ * lane of the warp calls it; n0: the cell's first node; a particle that is
+ * not live adds nothing. */
+__device__ __forceinline__ void scatter8(unsigned long long *acc, uint32_t n0, int64_t sy, int64_t sz,
+                                         const double d[3], double value, double fx, bool unit_cell, bool live) {
+    const unsigned FULL = 0xffffffffu;
+    const bool odd = threadIdx.x & 1;
     const double v = value * fx;
     const double a0 = v * (1 - d[0]), a1 = v * d[0], gj = 1 - d[1], gk = 1 - d[2];
     const double b0 = a0 * gj, b1 = a1 * gj, b2 = a1 * d[1], b3 = a0 * d[1];
-    const double w[8] = {b0 * gk, b1 * gk, b2 * gk, b3 * gk, b0 * d[2], b1 * d[2], b2 * d[2], b3 * d[2]};
-    const int64_t idx[8] = {n0, n0 + 1, n0 + 1 + sy, n0 + sy, n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};
-    if (unit_cell && (__double2hiint(v) & 0x7fffffff) < 0x43100000) { /* |v| < 2^50 */
+    /* rows of low and high x corners */
+    const double lo[4] = {b0 * gk, b3 * gk, b0 * d[2], b3 * d[2]}, hi[4] = {b1 * gk, b2 * gk, b1 * d[2], b2 * d[2]};
+    const int64_t row[4] = {0, sy, sz, sy + sz};
+    /* |v| < 2^61; decided for the warp, so that the conversions, which run on
+     * the float64 pipe, sit behind a branch */
+    const bool small = __all_sync(FULL, !live || (unit_cell && (__double2hiint(v) & 0x7fffffff) < 0x43c00000));
+    const uint32_t mate = __shfl_xor_sync(FULL, n0, 1);
+    unsigned long long *even = acc + (odd ? mate : n0) + odd, *other = acc + (odd ? n0 : mate) + odd;
 #pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const long long q = __double_as_longlong(w[m] + magic) - __double_as_longlong(magic);
-            if (q != 0) atomicAdd(acc + idx[m], (unsigned long long)q);
+    for (int r = 0; r < 4; r++) {
+        long long ql, qh;
+        if (small) {
+            ql = round_bits(lo[r]);
+            qh = round_bits(hi[r]);
+        } else {
+            ql = __double2ll_rn(lo[r]);
+            qh = __double2ll_rn(hi[r]);
         }
-    } else {
-        for (int m = 0; m < 8; m++) {
-            const long long q = __double2ll_rn(w[m]);
-            if (q != 0) atomicAdd(acc + idx[m], (unsigned long long)q);
-        }
+        if (!live) ql = qh = 0;
+        const long long got = __shfl_xor_sync(FULL, odd ? ql : qh, 1);
+        const long long ce = odd ? got : ql, co = odd ? qh : got;
+        if (ce) atomicAdd(even + row[r], (unsigned long long)ce);
+        if (co) atomicAdd(other + row[r], (unsigned long long)co);
     }
 }
 

@@ -114,14 +114,15 @@ __device__ __forceinline__ bool in_sphere(const double s[4], const double x[3]) 
     return rm2 <= s[3];
 }
 
-/* Field_::scatter of `value` at logical coordinates lc as 64-bit fixed point
- * (scatter8) */
+/* the warp's Field_::scatter of `value` at logical coordinates lc as 64-bit
+ * fixed point (scatter8) */
 __device__ __forceinline__ void deposit8(const Geo &g, unsigned long long *acc, const double lc[3], double value,
-                                         double fx) {
-    int c[3];
-    double off[3];
-    const bool unit = cells_of(g, lc, c, off);
-    scatter8(acc, node_of(g, c[0], c[1], c[2]), g.ni, (int64_t)g.ni * g.nj, off, value, fx, unit);
+                                         double fx, bool live) {
+    int c[3] = {0, 0, 0};
+    double off[3] = {0, 0, 0};
+    bool unit = true;
+    if (live) unit = cells_of(g, lc, c, off);
+    scatter8(acc, (uint32_t)node_of(g, c[0], c[1], c[2]), g.ni, (int64_t)g.ni * g.nj, off, value, fx, unit, live);
 }
 
 /* A float test that x lies surely outside the sphere, so that most warps
@@ -172,7 +173,7 @@ static SphereReject sphere_reject(const World &w) {
  * left-to-right gathers; quotients by dh come from its rounded reciprocal,
  * bounds, truncations and the far sphere test from integers and floats.
  * 4M ions on 64x64x128 nodes: 1.68 ms with divisions, float64 compares and
- * a conversion per corner weight, 1.28 ms now. */
+ * a conversion per corner weight, 1.26 ms now. */
 template <int WALLS, bool DEPOSIT, bool UNIFORM>
 __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restrict__ ef, double s,
                                                    double dt, double *P, int64_t stride,
@@ -183,10 +184,11 @@ __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restri
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t n = d_count[0];
     bool dead = false;
+    double lc[3] = {0, 0, 0}, w = 0;
     if (p < n) {
         double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
         double v[3] = {P[3 * stride + p], P[4 * stride + p], P[5 * stride + p]};
-        double lc[3], e[3];
+        double e[3];
         xtol_rcp(g, rdh, x, lc);
         gather3(g, ef, lc, e);
 #pragma unroll
@@ -226,11 +228,11 @@ __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restri
             P[(3 + d) * stride + p] = v[d];
         }
         if (DEPOSIT && !dead) {
-            double w = UNIFORM ? w0 : P[6 * stride + p];
+            w = UNIFORM ? w0 : P[6 * stride + p];
             xtol_rcp(g, rdh, x, lc);
-            deposit8(g, acc, lc, w, fx);
         }
     }
+    if (DEPOSIT) deposit8(g, acc, lc, w, fx, p < n && !dead);
     if (WALLS == ABSORB) {
         unsigned m = __ballot_sync(0xffffffffu, dead);
         if ((threadIdx.x & 31) == 0 && p < n) {
@@ -245,11 +247,14 @@ __global__ void __launch_bounds__(256) k_deposit_fp64(Geo g, const double *__res
                                                       const int64_t *__restrict__ d_count, double3 rdh,
                                                       unsigned long long *acc, double fx, double w0) {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= d_count[0]) return;
-    double x[3] = {P[p], P[stride + p], P[2 * stride + p]}, lc[3];
-    double w = UNIFORM ? w0 : P[6 * stride + p];
-    xtol_rcp(g, rdh, x, lc);
-    deposit8(g, acc, lc, w, fx);
+    const bool live = p < d_count[0];
+    double lc[3] = {0, 0, 0}, w = 0;
+    if (live) {
+        const double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
+        w = UNIFORM ? w0 : P[6 * stride + p];
+        xtol_rcp(g, rdh, x, lc);
+    }
+    deposit8(g, acc, lc, w, fx, live);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -2407,8 +2412,14 @@ __device__ __forceinline__ void corner_weights(double di, double dj, double dk, 
  * particles' counts of a corner around in shared memory, so that eight lanes
  * add to one node's 64 bytes: with a plane per sum and every lane at its own
  * node, an atomic instruction touched 32 sectors instead of 16 (1592 us for
- * 6.4M atoms; 1264 us now, of which the ~100 float64 instructions per
- * atom are 1070). */
+ * 6.4M atoms, 1264 us turned).  What remained were ~100 float64 operations per
+ * atom on a pipe that takes a warp's in 16 clocks, 56 of them the counts'
+ * FMAs: five sums of seven are rounded by integer operations instead, which
+ * balances the two pipes (865 us; a 41^3 gas step of two populations takes
+ * 2.40 ms with all seven by FMA, 2.13 ms with four, 2.06 ms with two, 2.25 ms
+ * with none). */
+constexpr int MOM_FMA = 2; /* sums rounded by an FMA; the others by round_product */
+
 __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const double *__restrict__ P, int64_t stride,
                                                      double w0, const int64_t *__restrict__ d_count,
                                                      const double *__restrict__ scale, unsigned long long *acc,
@@ -2442,11 +2453,23 @@ __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const d
     /* 16-byte slot j of particle l sits at l * 4 + (j ^ (l / 2 & 3)): no bank
      * conflicts in either direction */
     const int swz = (lane >> 1) & 3, q = lane & 7;
+    Mantissa mv[NMOM];
+#pragma unroll
+    for (int k = 0; k < NMOM; k++) mv[k] = mantissa_of(v[k]);
 #pragma unroll
     for (int m = 0; m < 8; m++) {
         long long c[MOM_STRIDE];
+        const Mantissa mw = mantissa_of(W[m]);
+        /* the integer and the float64 pipes share the products */
 #pragma unroll
-        for (int k = 0; k < NMOM; k++) c[k] = fix_round(v[k], W[m]);
+        for (int k = 0; k < NMOM; k++) {
+            if (k < MOM_FMA) {
+                c[k] = fix_round(v[k], W[m]);
+            } else {
+                const long long r = (long long)round_product(mv[k], mw);
+                c[k] = __double2hiint(v[k]) < 0 ? -r : r;
+            }
+        }
         c[NMOM] = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) buf[lane * 4 + (k ^ swz)] = make_longlong2(c[2 * k], c[2 * k + 1]);

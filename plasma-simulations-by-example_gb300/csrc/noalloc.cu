@@ -65,37 +65,39 @@ __global__ void __launch_bounds__(256) k_na_clear(unsigned long long *acc, uint3
  * int64 sums), deposits nothing and sets a bit of the flags.  Bound by the
  * float64 pipe, which runs the three differences, nine operations of the
  * quotients by dh, the offsets and the weights (6M particles on 97x89x117
- * nodes: 827 us with divisions and a conversion per weight, 506 us now). */
+ * nodes: 827 us with divisions and a conversion per weight, 475 us now). */
 __global__ void __launch_bounds__(256) k_na_deposit(NaGeo g, const double *__restrict__ P, int64_t stride, int64_t n,
                                                     double fx, double weight_bound, unsigned long long *acc,
                                                     int *flags) {
     next_may_start();
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    double lc[3], off[3];
-    for (int d = 0; d < 3; d++) lc[d] = espic::div_rcp(P[d * stride + p] - g.x0[d], g.dh[d], g.rdh[d]);
-    const double value = P[6 * stride + p];
-    const bool finite = espic::finite_bits(lc[0]) && espic::finite_bits(lc[1]) && espic::finite_bits(lc[2]);
-    /* false for NaN, whose key lies beyond infinity's */
-    const bool in_range = espic::order_key(fabs(value)) <= espic::order_key(weight_bound);
-    if (!(finite && in_range)) {
-        wait_for_previous();
-        if (flags) atomicOr(flags, (finite ? 0 : ESPIC_NOALLOC_NONFINITE) | (in_range ? 0 : ESPIC_NOALLOC_RANGE));
-        return;
-    }
     const int nn3[3] = {g.ni, g.nj, g.nk};
-    int c[3];
-    bool unit = true;
+    double off[3] = {0, 0, 0}, value = 0;
+    int c[3] = {0, 0, 0};
+    bool unit = true, finite = true, in_range = true;
+    const bool there = p < n;
+    if (there) {
+        double lc[3];
+        for (int d = 0; d < 3; d++) lc[d] = espic::div_rcp(P[d * stride + p] - g.x0[d], g.dh[d], g.rdh[d]);
+        value = P[6 * stride + p];
+        finite = espic::finite_bits(lc[0]) && espic::finite_bits(lc[1]) && espic::finite_bits(lc[2]);
+        /* false for NaN, whose key lies beyond infinity's */
+        in_range = espic::order_key(fabs(value)) <= espic::order_key(weight_bound);
+        if (finite && in_range)
 #pragma unroll
-    for (int d = 0; d < 3; d++)
-        if (!espic::cell_of(lc[d], nn3[d], c[d], off[d])) {
-            c[d] = na_clamp((int)lc[d], nn3[d]);
-            off[d] = lc[d] - c[d];
-            unit = false;
-        }
-    const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
+            for (int d = 0; d < 3; d++)
+                if (!espic::cell_of(lc[d], nn3[d], c[d], off[d])) {
+                    c[d] = na_clamp((int)lc[d], nn3[d]);
+                    off[d] = lc[d] - c[d];
+                    unit = false;
+                }
+    }
     wait_for_previous();
-    espic::scatter8(acc, c[2] * sz + c[1] * sy + c[0], sy, sz, off, value, fx, unit);
+    if (!(finite && in_range) && flags)
+        atomicOr(flags, (finite ? 0 : ESPIC_NOALLOC_NONFINITE) | (in_range ? 0 : ESPIC_NOALLOC_RANGE));
+    const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
+    espic::scatter8(acc, (uint32_t)(c[2] * sz + c[1] * sy + c[0]), sy, sz, off, value, fx, unit,
+                    there && finite && in_range);
 }
 
 __global__ void __launch_bounds__(256) k_na_density(NaGeo g, const unsigned long long *acc, double unit, double *den) {
