@@ -188,14 +188,25 @@ constexpr size_t PCG_SMEM_MAX = 160 * 1024; /* shared memory for block 0's coars
 
 template <typename T>
 struct MgLevel {
-    int nx, ny, nz, pad;
+    int nx, ny, nz;
+    int merge; /* MERGE_PRE | MERGE_POST: half sweeps of the whole grid in one phase */
     int64_t n;
     T *diag, *w, *b, *e; /* w: 6 weights per node, [m][n] */
+    T *f;                /* the level's final correction: its own array with MERGE_POST, else e */
     T *id;               /* 1 / diag, 0 where diag is 0 (an aggregate without unknowns) */
 };
 
+/* MERGE_PRE: the black half sweep before the restriction runs inside the
+ * restriction (restrict_through); MERGE_POST: the two half sweeps after the
+ * prolongation run as one (coarse_post).  Neighbouring work items then
+ * relax the same black nodes again, which costs little where a level has
+ * fewer nodes than the grid has threads, and saves a phase, that is a grid
+ * barrier (1.29 us) and an L2 latency. */
+enum { MERGE_PRE = 1, MERGE_POST = 2 };
+
 template <typename T>
 struct MgArgs {
+    int fine_pre;    /* MERGE_PRE for the node grid */
     int nlev;        /* coarse levels (0: Jacobi preconditioner) */
     int grid_levels; /* coarse levels 1..grid_levels-1 run on the whole grid */
     int nu_coarse;   /* sweeps each way on the coarsest level */
@@ -267,7 +278,7 @@ __device__ __forceinline__ void shared_init(const Fine<T> &F, const MgArgs<T> &A
             st.B.L[i].diag = st.B.L[i].id = (T *)(base + off); /* the one that the sweeps read */
             st.B.L[i].w = (T *)(base + off + a);
             st.B.L[i].b = (T *)(base + off + 7 * a);
-            st.B.L[i].e = (T *)(base + off + 8 * a);
+            st.B.L[i].e = st.B.L[i].f = (T *)(base + off + 8 * a);
             off += 9 * a;
         }
     }
@@ -424,7 +435,7 @@ __device__ __forceinline__ Dots<T> fine_half() {
                  * the next aggregate on the side of the node's parity */
                 const MgLevel<T> &C = shared_of<T>().A.L[0];
                 const int32_t cy = C.nx, cz = C.nx * C.ny;
-                const T *e = C.e + ((k >> 1) * cz + (j >> 1) * cy + (i >> 1));
+                const T *e = C.f + ((k >> 1) * cz + (j >> 1) * cy + (i >> 1));
                 par[q] = (i & 1) | ((j & 1) << 1) | ((k & 1) << 2);
                 ea[q] = e[0];
                 en[q][0] = e[(i & 1) ? 1 : -1];
@@ -479,51 +490,42 @@ __device__ __forceinline__ Dots<T> fine_half() {
     return {rz, zz};
 }
 
-/* one half sweep of colour c on level l (0: the first coarse one), by the
- * grid or by block 0 on its own view; POST reads the neighbours with the next
- * level's correction added (per axis one neighbour
- * shares the node's aggregate, the other is in the next one) */
+/* A node of a coarse level: all loads first (a missing neighbour reads a
+ * clamped node; its zero weight deselects it), then its relaxation, (b + sum
+ * w e_nb) / diag.  POST reads the neighbours with the next level's correction
+ * added (per axis one neighbour shares the node's aggregate, the other is in
+ * the next one). */
 template <typename T, bool POST>
-__device__ __forceinline__ void coarse_half(int l, int c, bool whole) {
-    const MgArgs<T> &A = whole ? shared_of<T>().A : shared_of<T>().B;
-    const MgLevel<T> L = A.L[l];
-    const int hx = (L.nx + 1) / 2;
-    const int32_t offs[6] = {-1, 1, -L.nx, L.nx, -L.nx * L.ny, L.nx * L.ny};
-    const float inv_hx = 1.f / (float)hx, inv_ny = 1.f / (float)L.ny;
-    const Span S = span(whole, (uint32_t)(hx * L.ny * L.nz));
-#pragma unroll 1
-    for (uint32_t t = S.t; t < S.end; t += S.step) {
-        const uint32_t rr = div_small(t, (uint32_t)hx, inv_hx);
-        const uint32_t kk = div_small(rr, (uint32_t)L.ny, inv_ny);
-        const int i2 = (int)(t - rr * (uint32_t)hx);
-        const int j = (int)(rr - kk * (uint32_t)L.ny);
-        const int k = (int)kk;
-        const int i = 2 * i2 + ((j + k + c) & 1);
-        if (i >= L.nx) continue;
+struct CoarseNode {
+    T d, s, wm[6], en[6];
+    __device__ __forceinline__ void load_self(const MgLevel<T> &L, int32_t I) {
+        d = LIGHT<T> ? L.id[I] : L.diag[I];
+        s = L.b[I];
+#pragma unroll
+        for (int m = 0; m < 6; m++) wm[m] = L.w[m * L.n + I];
+    }
+    __device__ __forceinline__ void load(const MgArgs<T> &A, int l, int i, int j, int k) {
+        const MgLevel<T> &L = A.L[l];
+        const int32_t offs[6] = {-1, 1, -L.nx, L.nx, -L.nx * L.ny, L.nx * L.ny};
         const int32_t I = (k * L.ny + j) * L.nx + i;
-        /* all loads first (a missing neighbour reads a clamped node; its zero
-         * weight deselects it), then the arithmetic */
-        const T d = LIGHT<T> ? L.id[I] : L.diag[I];
-        T s = L.b[I];
-        T wm[6], en[6];
+        load_self(L, I);
 #pragma unroll
         for (int m = 0; m < 6; m++) {
             int32_t nb = I + offs[m];
             nb = nb < 0 ? 0 : (nb >= (int32_t)L.n ? (int32_t)L.n - 1 : nb);
-            wm[m] = L.w[m * L.n + I];
             en[m] = L.e[nb];
         }
         if (POST) {
-            const MgLevel<T> *C = &A.L[l + 1];
+            const MgLevel<T> &C = A.L[l + 1];
             const T scale = A.scale;
-            const int g = ((k >> 1) * C->ny + (j >> 1)) * C->nx + (i >> 1);
+            const int g = ((k >> 1) * C.ny + (j >> 1)) * C.nx + (i >> 1);
             /* the next aggregate along each axis; a neighbour off the level
              * has weight 0 and may read the node's own */
             const int ax = (i & 1) ? (i + 1 < L.nx ? g + 1 : g) : (i > 0 ? g - 1 : g);
-            const int ay = (j & 1) ? (j + 1 < L.ny ? g + C->nx : g) : (j > 0 ? g - C->nx : g);
-            const int az = (k & 1) ? (k + 1 < L.nz ? g + C->nx * C->ny : g) : (k > 0 ? g - C->nx * C->ny : g);
-            const T ea = C->e[g];
-            const T ex[3] = {C->e[ax], C->e[ay], C->e[az]};
+            const int ay = (j & 1) ? (j + 1 < L.ny ? g + C.nx : g) : (j > 0 ? g - C.nx : g);
+            const int az = (k & 1) ? (k + 1 < L.nz ? g + C.nx * C.ny : g) : (k > 0 ? g - C.nx * C.ny : g);
+            const T ea = C.f[g];
+            const T ex[3] = {C.f[ax], C.f[ay], C.f[az]};
             const bool odd[3] = {(bool)(i & 1), (bool)(j & 1), (bool)(k & 1)};
 #pragma unroll
             for (int m = 0; m < 6; m++) en[m] += scale * (odd[m >> 1] != (bool)(m & 1) ? ea : ex[m >> 1]);
@@ -531,10 +533,84 @@ __device__ __forceinline__ void coarse_half(int l, int c, bool whole) {
         pin(s);
         pin(wm);
         pin(en);
-        if (d == (T)0) continue;
+    }
+    __device__ __forceinline__ T relax() const {
+        T t = s;
 #pragma unroll
-        for (int m = 0; m < 6; m++) s += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
-        L.e[I] = LIGHT<T> ? s * d : s / d;
+        for (int m = 0; m < 6; m++) t += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
+        return LIGHT<T> ? t * d : t / d;
+    }
+};
+
+/* entry t of the x pairs of a level's rows (hx of them a row) */
+__device__ __forceinline__ void pair_coords(uint32_t t, uint32_t hx, uint32_t ny, float inv_hx, float inv_ny, int &i2,
+                                            int &j, int &k) {
+    const uint32_t rr = div_small(t, hx, inv_hx);
+    const uint32_t kk = div_small(rr, ny, inv_ny);
+    i2 = (int)(t - rr * hx);
+    j = (int)(rr - kk * ny);
+    k = (int)kk;
+}
+
+/* one half sweep of colour c on level l (0: the first coarse one), by the
+ * grid or by block 0 on its own view */
+template <typename T, bool POST>
+__device__ __forceinline__ void coarse_half(int l, int c, bool whole) {
+    const MgArgs<T> &A = whole ? shared_of<T>().A : shared_of<T>().B;
+    const MgLevel<T> &L = A.L[l];
+    const int hx = (L.nx + 1) / 2;
+    const float inv_hx = 1.f / (float)hx, inv_ny = 1.f / (float)L.ny;
+    const Span S = span(whole, (uint32_t)(hx * L.ny * L.nz));
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
+        int i2, j, k;
+        pair_coords(t, (uint32_t)hx, (uint32_t)L.ny, inv_hx, inv_ny, i2, j, k);
+        const int i = 2 * i2 + ((j + k + c) & 1);
+        if (i >= L.nx) continue;
+        CoarseNode<T, POST> x;
+        x.load(A, l, i, j, k);
+        if (x.d == (T)0) continue;
+        L.e[(k * L.ny + j) * L.nx + i] = x.relax();
+    }
+}
+
+/* Both half sweeps after the prolongation, black then red, by the whole grid
+ * (MERGE_POST).  Eight lanes take an x pair of nodes: six relax the black
+ * neighbours of its red node, which they hand to the first, and one of them
+ * is the pair's black node.  The results go to f, since other lanes still
+ * read the red values of e. */
+template <typename T>
+__device__ __forceinline__ void coarse_post(int l) {
+    const MgArgs<T> &A = shared_of<T>().A;
+    const MgLevel<T> &L = A.L[l];
+    const uint32_t hx = (uint32_t)(L.nx + 1) / 2;
+    const float inv_hx = 1.f / (float)hx, inv_ny = 1.f / (float)L.ny;
+    const uint32_t total = 8 * hx * (uint32_t)(L.ny * L.nz);
+    const int m0 = (int)(threadIdx.x & 7);
+    const int step = (m0 & 1) ? 1 : -1;
+    const Span S = span(true, (total + 31u) & ~31u);
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
+        const bool valid = t < total;
+        int i2, j, k;
+        pair_coords(valid ? t >> 3 : 0u, hx, (uint32_t)L.ny, inv_hx, inv_ny, i2, j, k);
+        const int odd = (j + k) & 1;
+        const int i = 2 * i2 + odd; /* the red node */
+        const int bi = i + (m0 < 2 ? step : 0), bj = j + (m0 == 2 || m0 == 3 ? step : 0),
+                  bk = k + (m0 == 4 || m0 == 5 ? step : 0);
+        const bool in = valid && m0 < 6 && bi >= 0 && bj >= 0 && bk >= 0 && bi < L.nx && bj < L.ny && bk < L.nz;
+        const bool red = valid && m0 == 0 && i < L.nx;
+        CoarseNode<T, true> x;
+        CoarseNode<T, false> y;
+        const int32_t I = red ? (k * L.ny + j) * L.nx + i : 0;
+        y.load_self(L, I);
+        x.load(A, l, in ? bi : 0, in ? bj : 0, in ? bk : 0);
+        const bool on = in && x.d != (T)0;
+        const T v = on ? x.relax() : (T)0;
+        if (on && m0 == 1 - odd) L.f[(bk * L.ny + bj) * L.nx + bi] = v;
+#pragma unroll
+        for (int m = 0; m < 6; m++) y.en[m] = __shfl_sync(0xffffffffu, v, m, 8);
+        if (red && y.d != (T)0) L.f[I] = y.relax();
     }
 }
 
@@ -590,7 +666,7 @@ template <typename T>
 struct FineChild {
     T id, r, dg, z, zn[6];
     uint16_t cc;
-    __device__ __forceinline__ void load(const Fine<T> &F, int32_t sy, int32_t sz, uint32_t u, bool in) {
+    __device__ __forceinline__ void load_self(const Fine<T> &F, uint32_t u, bool in) {
         if (LIGHT<T>) {
             id = in ? F.id[u] : (T)0;
         } else {
@@ -599,6 +675,9 @@ struct FineChild {
             dg = F.dg[u];
             z = F.z[u];
         }
+    }
+    __device__ __forceinline__ void load(const Fine<T> &F, int32_t sy, int32_t sz, uint32_t u, bool in) {
+        load_self(F, u, in);
         load_neighbours<T>(F.z, u, sy, sz, zn);
     }
     __device__ __forceinline__ void hold() {
@@ -693,6 +772,14 @@ __device__ __forceinline__ void restrict_fine() {
 /* b of level l+1 from level l, laid out like restrict_fine (an aggregate
  * without unknowns has no weights and contributes 0) */
 template <typename T>
+__device__ __forceinline__ T coarse_residual(T bu, T dd, T eu, const T (&wm)[6], const T (&en)[6]) {
+    T res = LIGHT<T> ? (T)0 : bu - dd * eu;
+#pragma unroll
+    for (int m = 0; m < 6; m++) res += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
+    return res;
+}
+
+template <typename T>
 __device__ __forceinline__ T coarse_child_residual(const MgLevel<T> &L, int i, int j, int k, bool in) {
     const int32_t offs[6] = {-1, 1, -L.nx, L.nx, -L.nx * L.ny, L.nx * L.ny};
     in = in && i < L.nx && j < L.ny && k < L.nz;
@@ -709,10 +796,7 @@ __device__ __forceinline__ T coarse_child_residual(const MgLevel<T> &L, int i, i
     pin(wm);
     pin(en);
     if (!in || dd == (T)0) return (T)0;
-    T res = LIGHT<T> ? (T)0 : bu - dd * eu;
-#pragma unroll
-    for (int m = 0; m < 6; m++) res += (wm[m] != (T)0) ? wm[m] * en[m] : (T)0;
-    return res;
+    return coarse_residual(bu, dd, eu, wm, en);
 }
 
 template <typename T>
@@ -754,6 +838,129 @@ __device__ __forceinline__ void restrict_coarse(int l, bool whole) {
         const T res =
             coarse_child_residual(L, 2 * ci + (d & 1), 2 * cj + ((d >> 1) & 1), 2 * ck + (d >> 2), valid);
         restrict_store(C, valid, I, ci, cj, ck, res, cd);
+    }
+}
+
+/* The black half sweep and the restriction in one phase (MERGE_PRE), by the
+ * whole grid: sixteen lanes take a coarse node and relax the sixteen black
+ * nodes around its four red children (four in its 2x2x2 block, twelve just
+ * outside), which the first four lanes then read as their red child's
+ * neighbours.  Nothing else reads the black values of this half sweep (the
+ * black half after the prolongation overwrites them), so they are not
+ * stored. */
+struct Block16 {
+    int dx, dy, dz; /* this lane's black node, -1..2 from the block's corner */
+    int red;        /* red child of lanes 0..3 (bits dx | dy << 1 | dz << 2) */
+    int src[6];     /* lanes of that child's neighbours */
+};
+
+__device__ __forceinline__ Block16 block16() {
+    Block16 B;
+    const int lane = (int)(threadIdx.x & 15);
+    if (lane < 4) {
+        const int mask = lane == 3 ? 7 : 1 << lane;
+        B.dx = mask & 1;
+        B.dy = (mask >> 1) & 1;
+        B.dz = mask >> 2;
+    } else {
+        const int mask = red_child((lane - 4) / 3), a = (lane - 4) % 3;
+        B.dx = mask & 1;
+        B.dy = (mask >> 1) & 1;
+        B.dz = mask >> 2;
+        if (a == 0) B.dx = B.dx ? 2 : -1;
+        if (a == 1) B.dy = B.dy ? 2 : -1;
+        if (a == 2) B.dz = B.dz ? 2 : -1;
+    }
+    const int q = lane & 3;
+    B.red = red_child(q);
+#pragma unroll
+    for (int m = 0; m < 6; m++) {
+        const int a = m >> 1, bit = (B.red >> a) & 1, inner = B.red ^ (1 << a);
+        B.src[m] = (m & 1) != bit ? (inner == 7 ? 3 : inner >> 1) : 4 + 3 * q + a;
+    }
+    return B;
+}
+
+template <typename T>
+__device__ __forceinline__ void restrict_through(int l) {
+    const MgArgs<T> &A = shared_of<T>().A;
+    const MgLevel<T> &L = A.L[l], &C = A.L[l + 1];
+    const float inv_nx = 1.f / (float)C.nx, inv_ny = 1.f / (float)C.ny;
+    const T *__restrict__ diag = LIGHT<T> ? C.id : C.diag;
+    const Block16 B = block16();
+    const uint32_t total = 16 * (uint32_t)C.n;
+    const Span S = span(true, (total + 31u) & ~31u);
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
+        const bool valid = t < total;
+        const uint32_t I = valid ? (t >> 4) : 0;
+        int ci, cj, ck;
+        coarse_coords(C, I, inv_nx, inv_ny, ci, cj, ck);
+        const int i = 2 * ci + B.dx, j = 2 * cj + B.dy, k = 2 * ck + B.dz;
+        const bool in = i >= 0 && j >= 0 && k >= 0 && i < L.nx && j < L.ny && k < L.nz;
+        const int ri = 2 * ci + (B.red & 1), rj = 2 * cj + ((B.red >> 1) & 1), rk = 2 * ck + (B.red >> 2);
+        const bool rin = (threadIdx.x & 12) == 0 && ri < L.nx && rj < L.ny && rk < L.nz;
+        const int32_t u = rin ? (rk * L.ny + rj) * L.nx + ri : 0;
+        CoarseNode<T, false> x;
+        T wm[6], nb[6], cd = diag[I];
+        const T dd = LIGHT<T> ? (T)1 : L.diag[u], bu = LIGHT<T> ? (T)0 : L.b[u], eu = LIGHT<T> ? (T)0 : L.e[u];
+#pragma unroll
+        for (int m = 0; m < 6; m++) wm[m] = L.w[m * L.n + u];
+        x.load(A, l, in ? i : 0, in ? j : 0, in ? k : 0);
+        pin(wm);
+        pin(cd);
+        const T v = in && x.d != (T)0 ? x.relax() : (T)0;
+#pragma unroll
+        for (int m = 0; m < 6; m++) nb[m] = __shfl_sync(0xffffffffu, v, B.src[m], 16);
+        const T res = rin && dd != (T)0 ? coarse_residual(bu, dd, eu, wm, nb) : (T)0;
+        restrict_store(C, valid && (threadIdx.x & 15) == 0, I, ci, cj, ck, res, cd);
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void restrict_through_fine() {
+    const Fine<T> &F = shared_of<T>().F;
+    const MgLevel<T> &C = shared_of<T>().A.L[0];
+    const Geo g = F.g;
+    const int32_t sy = g.ni, sz = g.ni * g.nj;
+    const float inv_nx = 1.f / (float)C.nx, inv_ny = 1.f / (float)C.ny;
+    const T *__restrict__ diag = LIGHT<T> ? C.id : C.diag;
+    const T *__restrict__ dv = LIGHT<T> ? F.id : F.dg;
+    const Block16 B = block16();
+    const uint32_t total = 16 * (uint32_t)C.n;
+    const Span S = span(true, (total + 31u) & ~31u);
+#pragma unroll 1
+    for (uint32_t t = S.t; t < S.end; t += S.step) {
+        const bool valid = t < total;
+        const uint32_t I = valid ? (t >> 4) : 0;
+        int ci, cj, ck;
+        coarse_coords(C, I, inv_nx, inv_ny, ci, cj, ck);
+        bool in = true, rin = (threadIdx.x & 12) == 0;
+        const uint32_t u = interior_or_safe(g, 2 * ci + B.dx, 2 * cj + B.dy, 2 * ck + B.dz, in);
+        const uint32_t ur = interior_or_safe(g, 2 * ci + (B.red & 1), 2 * cj + ((B.red >> 1) & 1), 2 * ck + (B.red >> 2),
+                                             rin);
+        FineChild<T> ch;
+        T cd = diag[I], ru = F.r[u], du = dv[u], zn[6];
+        const uint16_t cc = LIGHT<T> ? (uint16_t)0 : F.code[u];
+        load_neighbours(F.z, u, sy, sz, zn);
+        ch.load_self(F, ur, rin);
+        pin(cd);
+        pin(ru);
+        pin(du);
+        pin(zn);
+        T v = 0, s = ru;
+        if (LIGHT<T>) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) s += F.ct[a] * (zn[2 * a] + zn[2 * a + 1]);
+            if (in) v = s * du;
+        } else if (in && (cc & SELF)) {
+#pragma unroll
+            for (int m = 0; m < 6; m++) s += (cc & (1u << m)) ? F.ct[m >> 1] * zn[m] : (T)0;
+            v = s / full_diag(cc, du, F.ct);
+        }
+#pragma unroll
+        for (int m = 0; m < 6; m++) ch.zn[m] = __shfl_sync(0xffffffffu, v, B.src[m], 16);
+        restrict_store(C, valid && (threadIdx.x & 15) == 0, I, ci, cj, ck, ch.residual(F), cd);
     }
 }
 
@@ -821,6 +1028,14 @@ template <typename T>
 __device__ __noinline__ void dense_apply_call() {
     dense_apply<T>();
 }
+template <typename T>
+__device__ __noinline__ void coarse_post_call(int l) {
+    coarse_post<T>(l);
+}
+template <typename T>
+__device__ __noinline__ void restrict_through_call(int l) {
+    restrict_through<T>(l);
+}
 
 template <typename T, bool CALL>
 struct Pass {
@@ -846,6 +1061,18 @@ struct Pass {
             restrict_coarse_call<T>(l, whole);
         else
             restrict_coarse<T>(l, whole);
+    }
+    static __device__ __forceinline__ void through_from(int l) {
+        if (CALL)
+            restrict_through_call<T>(l);
+        else
+            restrict_through<T>(l);
+    }
+    static __device__ __forceinline__ void post(int l) {
+        if (CALL)
+            coarse_post_call<T>(l);
+        else
+            coarse_post<T>(l);
     }
     static __device__ __forceinline__ void dense() {
         if (CALL)
@@ -882,15 +1109,23 @@ __device__ __forceinline__ double vcycle_rest(cg::grid_group &grid, double *part
         return v[0];
     }
     const int GL = A.grid_levels;
-    P::template fine<PRE_BLACK>();
-    grid.sync();
-    P::restrict_to_first();
+    if (!CALL && A.fine_pre) {
+        restrict_through_fine<T>();
+    } else {
+        P::template fine<PRE_BLACK>();
+        grid.sync();
+        P::restrict_to_first();
+    }
     grid.sync();
     int l = 1; /* level l lives in A.L[l-1] and its red half was fused */
     for (; l < GL && l < NL; l++) {
-        P::template coarse<false>(l - 1, 1, true);
-        grid.sync();
-        P::restrict_from(l - 1, true);
+        if (A.L[l - 1].merge & MERGE_PRE) {
+            P::through_from(l - 1);
+        } else {
+            P::template coarse<false>(l - 1, 1, true);
+            grid.sync();
+            P::restrict_from(l - 1, true);
+        }
         grid.sync();
     }
     const int lblock = l;
@@ -962,9 +1197,13 @@ __device__ __forceinline__ double vcycle_rest(cg::grid_group &grid, double *part
     }
     const int top = coarsest_whole ? NL - 1 : lblock - 1;
     for (int b = top; b >= 1; b--) {
-        P::template coarse<true>(b - 1, 1, true);
-        grid.sync();
-        P::template coarse<false>(b - 1, 0, true);
+        if (A.L[b - 1].merge & MERGE_POST) {
+            P::post(b - 1);
+        } else {
+            P::template coarse<true>(b - 1, 1, true);
+            grid.sync();
+            P::template coarse<false>(b - 1, 0, true);
+        }
         grid.sync();
     }
     const Dots<T> db = P::template fine<POST_BLACK>();
@@ -1775,7 +2014,7 @@ static size_t mg_layout(World &w, MgArgs<T> &A, char *base) {
         L.nx = nx;
         L.ny = ny;
         L.nz = nz;
-        L.pad = 0;
+        L.merge = 0;
         L.n = (int64_t)nx * ny * nz;
         size_t bytes = ((L.n * sizeof(T) + 255) / 256) * 256;
         L.diag = (T *)(base ? base + off : nullptr);
@@ -1787,6 +2026,8 @@ static size_t mg_layout(World &w, MgArgs<T> &A, char *base) {
         L.b = (T *)(base ? base + off : nullptr);
         off += bytes;
         L.e = (T *)(base ? base + off : nullptr);
+        off += bytes;
+        L.f = (T *)(base ? base + off : nullptr);
         off += bytes;
         nlev++;
         if (L.n >= w.mg_block_nodes) grid_levels = nlev + 1;
@@ -1925,6 +2166,26 @@ static int run_pcg(World &w) {
     int grid = (int)(needb < maxb ? needb : maxb);
     if (grid > w.partial_slots / 4) grid = w.partial_slots / 4;
     if (w.solver_blocks > 0 && grid > w.solver_blocks) grid = w.solver_blocks;
+    /* Half sweeps are merged where the lanes of the merged pass fill the grid
+     * once, and in float the pass before a restriction up to twice: 33x29x65
+     * float sphere run, 20 steps: 16.8 ms unmerged, 14.7 with one, 14.2 with
+     * two; 64x64x128 float: 20.8, 19.7, 19.8 (the post pass of its first
+     * level; 21.8 with all up to eight times).  The float64 pipe, which all
+     * lanes' relaxations queue on, ends the gain earlier: 64x64x128 float64
+     * solve 5.53 ms unmerged, 5.44 with one, 5.78 with two; 32x32x96
+     * differentiable run 193, 180, 188. */
+    const int64_t most = (int64_t)grid * threads, pre_most = sizeof(T) == sizeof(float) ? 2 * most : most;
+    const int whole = A.grid_levels < A.nlev ? A.grid_levels : A.nlev; /* levels 0..whole-2 are the grid's */
+    A.fine_pre = A.nlev > 0 && 16 * A.L[0].n <= pre_most;
+    for (int l = 0; l < A.nlev; l++) {
+        MgLevel<T> &L = A.L[l];
+        L.merge = 0;
+        if (l + 1 < whole) {
+            if (16 * A.L[l + 1].n <= pre_most) L.merge |= MERGE_PRE;
+            if (8 * (int64_t)((L.nx + 1) / 2) * L.ny * L.nz <= most) L.merge |= MERGE_POST;
+        }
+        if (!(L.merge & MERGE_POST)) L.f = L.e;
+    }
     Geo g = w.g;
     double *phi = w.phi;
     const double *rho = w.rho;
