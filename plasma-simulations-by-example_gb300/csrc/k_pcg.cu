@@ -184,6 +184,8 @@ constexpr int MG_MAX = 12;
  * spills (33x29x65 float solve: 0.75 ms with 1024, 0.63 with 512; 64x64x128
  * float64: 7.5 and 6.8 ms a cold solve) */
 constexpr int PCG_THREADS = 1024, PCG_THREADS_SMALL = 512;
+constexpr int GJ_ROWS = 64;                /* rows of the dense inversion per block */
+constexpr size_t GJ_SMEM_MAX = 200 * 1024; /* and the shared memory they may take */
 constexpr size_t PCG_SMEM_MAX = 160 * 1024; /* shared memory for block 0's coarse levels */
 
 template <typename T>
@@ -1954,41 +1956,86 @@ __global__ void k_dense_build(MgLevel<T> L, double *M, double *diag0) {
     if (i == j) diag0[i] = v;
 }
 
-/* In-place Gauss-Jordan inversion without pivoting (the operator is
- * symmetric positive definite), in one cooperative launch: for each k,
- * block 0 saves column k and scales row k by the pivot, then every thread
- * eliminates column k from the other rows.  A pivot that vanished against
- * the original diagonal (a singular operator) clears *ok. */
-__global__ void __launch_bounds__(1024) k_gauss_jordan(double *M, int n, double *col,
-                                                       const double *__restrict__ diag0, int *ok) {
-    cg::grid_group grid = cg::this_grid();
-    __shared__ double piv;
-    for (int k = 0; k < n; k++) {
-        if (blockIdx.x == 0) {
-            if (threadIdx.x == 0) {
-                piv = __ldcg(M + (int64_t)k * n + k);
-                if (!(piv > 1e-9 * diag0[k])) {
-                    *ok = 0;
-                    piv = 1.0;
-                }
-            }
-            for (int i = threadIdx.x; i < n; i += blockDim.x) col[i] = __ldcg(M + (int64_t)i * n + k);
-            __syncthreads();
-            for (int j = threadIdx.x; j < n; j += blockDim.x) {
-                const double a = j == k ? 1.0 : __ldcg(M + (int64_t)k * n + j);
-                M[(int64_t)k * n + j] = a / piv;
-            }
+/* Row k of the inversion, divided by its pivot, for every block to read, and
+ * its place in row: 1 / pivot in column k.  One thread divides 1 by the pivot
+ * and the block's threads multiply (div_rcp; a division where an operand is
+ * too small for it).  A pivot that vanished against the original diagonal (a
+ * singular operator) clears *ok. */
+__device__ __forceinline__ void gj_publish(const double *row, int n, int k, double diag0, double *out, int *ok) {
+    __shared__ double piv, rpiv;
+    if (threadIdx.x == 0) {
+        double p = row[k];
+        if (!(p > 1e-9 * diag0)) {
+            *ok = 0;
+            p = 1.0;
         }
-        grid.sync();
-        for (int i = blockIdx.x; i < n; i += gridDim.x) {
-            if (i == k) continue;
-            const double f = __ldcg(col + i);
-            double *Mi = M + (int64_t)i * n;
-            for (int j = threadIdx.x; j < n; j += blockDim.x)
-                Mi[j] = (j == k ? 0.0 : __ldcg(Mi + j)) - f * __ldcg(M + (int64_t)k * n + j);
+        piv = p;
+        rpiv = 1.0 / p;
+    }
+    __syncthreads();
+    const double p = piv, y = rpiv;
+    const bool normal = p > 1e-100 && p < 1e100;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const double a = j == k ? 1.0 : row[j];
+        out[j] = normal && (fabs(a) > 1e-150 || a == 0.0) && fabs(a) < 1e150 ? div_rcp(a, p, y) : a / p;
+    }
+}
+
+/* In-place Gauss-Jordan inversion without pivoting (the operator is
+ * symmetric positive definite), in one cooperative launch.  A block keeps
+ * every gridDim.x-th row, in shared memory when they fit (staged), else where
+ * they lie.  For each k it reads the scaled row k and eliminates column k
+ * from its rows, the owner of row k + 1 that one first, so that it publishes
+ * the next scaled row while the others still work: one grid barrier a pivot
+ * and only a row of traffic.  With two barriers, a column buffer and the
+ * matrix in global memory 1024 rows took 13.1 ms; 6.6 ms now, of which the
+ * barriers and the row's way through L2 are the most.  pub: two rows of n. */
+__global__ void __launch_bounds__(1024, 1) k_gauss_jordan(double *M, int n, double *pub,
+                                                          const double *__restrict__ diag0, int *ok, int staged) {
+    cg::grid_group grid = cg::this_grid();
+    extern __shared__ __align__(16) double gj_rows[];
+    __shared__ double col[GJ_ROWS];
+    const int G = (int)gridDim.x, b = (int)blockIdx.x;
+    const int cnt = (n - b + G - 1) / G; /* rows b, b + G, ...; G <= n */
+    double *S = staged ? gj_rows : M + (int64_t)b * n;
+    const int64_t ld = staged ? n : (int64_t)G * n;
+    if (staged) {
+        for (int m = 0; m < cnt; m++)
+            for (int j = threadIdx.x; j < n; j += blockDim.x) S[m * ld + j] = M[((int64_t)b + (int64_t)m * G) * n + j];
+        __syncthreads();
+    }
+    if (b == 0) gj_publish(S, n, 0, diag0[0], pub, ok);
+    grid.sync();
+    for (int k = 0; k < n; k++) {
+        const double *R = pub + (k & 1) * n;
+        double r[4]; /* n <= 4096 */
+#pragma unroll
+        for (int q = 0; q < 4; q++) r[q] = threadIdx.x + 1024 * q < n ? __ldcg(R + threadIdx.x + 1024 * q) : 0.0;
+        for (int m = threadIdx.x; m < cnt; m += blockDim.x) col[m] = S[m * ld + k];
+        __syncthreads();
+        const int next = k + 1 < n && (k + 1) % G == b ? (k + 1) / G : -1;
+        for (int t = next >= 0 ? -1 : 0; t < cnt; t++) {
+            const int m = t < 0 ? next : t;
+            if (t >= 0 && t == next) continue;
+            const double f = col[m];
+            const bool own = b + m * G == k;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int j = threadIdx.x + 1024 * q;
+                if (j >= n) break;
+                const double x = j == k ? 0.0 : S[m * ld + j];
+                S[m * ld + j] = own ? r[q] : x - f * r[q];
+            }
+            if (t < 0) {
+                __syncthreads();
+                gj_publish(S + m * ld, n, k + 1, diag0[k + 1], pub + ((k + 1) & 1) * n, ok);
+            }
         }
         grid.sync();
     }
+    if (staged)
+        for (int m = 0; m < cnt; m++)
+            for (int j = threadIdx.x; j < n; j += blockDim.x) M[((int64_t)b + (int64_t)m * G) * n + j] = S[m * ld + j];
 }
 
 /* the inverse in T, symmetrised; rows and columns of aggregates without
@@ -2039,8 +2086,8 @@ static size_t mg_layout(World &w, MgArgs<T> &A, char *base) {
     A.nlev = w.mg_levels_max < nlev ? w.mg_levels_max : nlev;
     /* the first level with at most mg_dense_max nodes becomes the coarsest,
      * solved by its dense inverse on the whole grid (every level above it
-     * runs on the whole grid too); the float64 work matrix of the inversion
-     * and its column buffer follow the levels */
+     * runs on the whole grid too); the float64 work matrix of the inversion,
+     * its two published rows and the diagonal follow the levels */
     A.dense = nullptr;
     A.dense_n = 0;
     if (w.mg_dense_max > 0)
@@ -2055,7 +2102,7 @@ static size_t mg_layout(World &w, MgArgs<T> &A, char *base) {
         const size_t nsq = (size_t)A.dense_n * A.dense_n;
         A.dense = (T *)(base ? base + off : nullptr);
         off += (nsq * sizeof(T) + 255) / 256 * 256;
-        off += (nsq * sizeof(double) + 255) / 256 * 256 + 2 * (((size_t)A.dense_n * sizeof(double) + 255) / 256 * 256);
+        off += (nsq * sizeof(double) + 255) / 256 * 256 + 3 * (((size_t)A.dense_n * sizeof(double) + 255) / 256 * 256);
         A.dense_ok = (const int *)(base ? base + off : nullptr);
         off += 256;
     } else {
@@ -2121,20 +2168,23 @@ static int run_pcg(World &w) {
             const int n = A.dense_n;
             const int64_t nsq = (int64_t)n * n;
             double *M = (double *)((char *)A.dense + (nsq * sizeof(T) + 255) / 256 * 256);
-            double *col = (double *)((char *)M + (nsq * sizeof(double) + 255) / 256 * 256);
-            double *diag0 = col + ((size_t)n * sizeof(double) + 255) / 256 * 256 / sizeof(double);
+            double *pub = (double *)((char *)M + (nsq * sizeof(double) + 255) / 256 * 256);
+            double *diag0 = pub + (2 * (size_t)n * sizeof(double) + 255) / 256 * 256 / sizeof(double);
             int *ok = (int *)A.dense_ok;
             const int one = 1;
             cudaMemcpyAsync(ok, &one, sizeof(int), cudaMemcpyHostToDevice, w.stream);
             const MgLevel<T> &Lc = A.L[A.nlev - 1];
             k_dense_build<T><<<blocks_for(nsq, 256), 256, 0, w.stream>>>(Lc, M, diag0);
-            int gj_per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gj_per_sm, k_gauss_jordan, 1024, 0);
-            int gj_grid = (gj_per_sm < 1 ? 1 : gj_per_sm) * w.sm_count;
-            if (gj_grid > n) gj_grid = n;
-            int nn_ = n;
-            void *gj_args[] = {&M, &nn_, &col, &diag0, &ok};
-            cudaLaunchCooperativeKernel((const void *)k_gauss_jordan, gj_grid, 1024, gj_args, 0, w.stream);
+            /* one block per SM; its share of the rows (n <= 4096 of at least
+             * 64 SMs) */
+            const int gj_grid = w.sm_count < n ? w.sm_count : n;
+            const size_t gj_bytes = (size_t)((n + gj_grid - 1) / gj_grid) * n * sizeof(double);
+            if ((n + gj_grid - 1) / gj_grid > GJ_ROWS) return (int)cudaErrorInvalidValue;
+            int nn_ = n, staged = gj_bytes <= GJ_SMEM_MAX;
+            cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GJ_SMEM_MAX);
+            void *gj_args[] = {&M, &nn_, &pub, &diag0, &ok, &staged};
+            cudaLaunchCooperativeKernel((const void *)k_gauss_jordan, gj_grid, 1024, gj_args, staged ? gj_bytes : 0,
+                                        w.stream);
             k_dense_store<T><<<blocks_for(nsq, 256), 256, 0, w.stream>>>(Lc, M, A.dense);
             w.nlaunch += 3;
         }
