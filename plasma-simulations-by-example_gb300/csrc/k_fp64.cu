@@ -43,16 +43,17 @@ __device__ __forceinline__ int64_t node_of(const Geo &g, int i, int j, int k) {
     return ((int64_t)k * g.nj + j) * g.ni + i;
 }
 
-/* The cell of logical coordinates lc with the index clamp, and the offsets
- * lc - cell; true when every offset lies in [0, 1). */
-__device__ __forceinline__ bool cells_of(const Geo &g, const double lc[3], int c[3], double off[3]) {
+/* The cell of logical coordinates lc with the index clamp, the offsets
+ * off = lc - cell and rest = 1 - off; true when every offset lies in [0, 1). */
+__device__ __forceinline__ bool cells_of(const Geo &g, const double lc[3], int c[3], double off[3], double rest[3]) {
     const int n[3] = {g.ni, g.nj, g.nk};
     bool unit = true;
 #pragma unroll
     for (int d = 0; d < 3; d++)
-        if (!cell_of(lc[d], n[d], c[d], off[d])) {
+        if (!cell_of(lc[d], n[d], c[d], off[d], rest[d])) {
             c[d] = clamp_cell((int)lc[d], n[d]);
             off[d] = lc[d] - c[d];
+            rest[d] = 1 - off[d];
             unit = false;
         }
     return unit;
@@ -65,10 +66,10 @@ __device__ __forceinline__ bool cells_of(const Geo &g, const double lc[3], int c
 __device__ __forceinline__ void gather3(const Geo &g, const double *__restrict__ ef, const double lc[3],
                                         double e[3]) {
     int cell[3];
-    double off[3];
-    cells_of(g, lc, cell, off);
+    double off[3], rest[3];
+    cells_of(g, lc, cell, off, rest);
     const int i = cell[0], j = cell[1], k = cell[2];
-    const double di = off[0], dj = off[1], dk = off[2];
+    const double di = off[0], dj = off[1], dk = off[2], ri = rest[0], rj = rest[1], rk = rest[2];
     int64_t n0 = node_of(g, i, j, k);
     int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
     const double *a = ef + 3 * n0;
@@ -81,10 +82,8 @@ __device__ __forceinline__ void gather3(const Geo &g, const double *__restrict__
     const double *m = ef + 3 * (n0 + sy + sz);
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-        e[q] = a[q] * (1 - di) * (1 - dj) * (1 - dk) + b[q] * (di) * (1 - dj) * (1 - dk) +
-               c[q] * (di) * (dj) * (1 - dk) + d[q] * (1 - di) * (dj) * (1 - dk) +
-               e4[q] * (1 - di) * (1 - dj) * (dk) + f[q] * (di) * (1 - dj) * (dk) +
-               h[q] * (di) * (dj) * (dk) + m[q] * (1 - di) * (dj) * (dk);
+        e[q] = a[q] * ri * rj * rk + b[q] * di * rj * rk + c[q] * di * dj * rk + d[q] * ri * dj * rk +
+               e4[q] * ri * rj * dk + f[q] * di * rj * dk + h[q] * di * dj * dk + m[q] * ri * dj * dk;
     }
 }
 
@@ -119,10 +118,11 @@ __device__ __forceinline__ bool in_sphere(const double s[4], const double x[3]) 
 __device__ __forceinline__ void deposit8(const Geo &g, unsigned long long *acc, const double lc[3], double value,
                                          double fx, bool live) {
     int c[3] = {0, 0, 0};
-    double off[3] = {0, 0, 0};
+    double off[3] = {0, 0, 0}, rest[3] = {1, 1, 1};
     bool unit = true;
-    if (live) unit = cells_of(g, lc, c, off);
-    scatter8(acc, (uint32_t)node_of(g, c[0], c[1], c[2]), g.ni, (int64_t)g.ni * g.nj, off, value, fx, unit, live);
+    if (live) unit = cells_of(g, lc, c, off, rest);
+    scatter8(acc, (uint32_t)node_of(g, c[0], c[1], c[2]), g.ni, (int64_t)g.ni * g.nj, off, rest, value, fx, unit,
+             live);
 }
 
 /* A float test that x lies surely outside the sphere, so that most warps
@@ -173,7 +173,8 @@ static SphereReject sphere_reject(const World &w) {
  * left-to-right gathers; quotients by dh come from its rounded reciprocal,
  * bounds, truncations and the far sphere test from integers and floats.
  * 4M ions on 64x64x128 nodes: 1.68 ms with divisions, float64 compares and
- * a conversion per corner weight, 1.26 ms now. */
+ * a conversion per corner weight, 1.26 ms without, 1.17 ms with the offsets
+ * and the corners' last products made of integers. */
 template <int WALLS, bool DEPOSIT, bool UNIFORM>
 __global__ void __launch_bounds__(256) k_push_fp64(Geo g, const double *__restrict__ ef, double s,
                                                    double dt, double *P, int64_t stride,
@@ -2393,16 +2394,16 @@ __device__ __forceinline__ long long fix_round(double a, double b) {
 
 /* corner weights (1-di)(1-dj)(1-dk), di(1-dj)(1-dk), ... in Field_::scatter's
  * corner order (ch4/Field.h:212-232), the dj, dk factors shared */
-__device__ __forceinline__ void corner_weights(double di, double dj, double dk, double W[8]) {
-    const double a0 = (1 - di) * (1 - dj), a1 = di * (1 - dj), a2 = di * dj, a3 = (1 - di) * dj;
-    W[0] = a0 * (1 - dk);
-    W[1] = a1 * (1 - dk);
-    W[2] = a2 * (1 - dk);
-    W[3] = a3 * (1 - dk);
-    W[4] = a0 * dk;
-    W[5] = a1 * dk;
-    W[6] = a2 * dk;
-    W[7] = a3 * dk;
+__device__ __forceinline__ void corner_weights(const double d[3], const double e[3], double W[8]) {
+    const double a0 = e[0] * e[1], a1 = d[0] * e[1], a2 = d[0] * d[1], a3 = e[0] * d[1];
+    W[0] = a0 * e[2];
+    W[1] = a1 * e[2];
+    W[2] = a2 * e[2];
+    W[3] = a3 * e[2];
+    W[4] = a0 * d[2];
+    W[5] = a1 * d[2];
+    W[6] = a2 * d[2];
+    W[7] = a3 * d[2];
 }
 
 /* each sum's 8 corner contributions value * W_m, rounded once (from the exact
@@ -2432,14 +2433,14 @@ __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const d
     int32_t n0 = -1; /* no particle */
     if (p < d_count[0]) {
         const double x[3] = {P[p], P[stride + p], P[2 * stride + p]};
-        double lc[3], off[3];
+        double lc[3], off[3], rest[3];
         int cl[3];
         xtol_rcp(g, rdh, x, lc);
         /* offsets in [0, 1) imply the range */
-        if (cells_of(g, lc, cl, off) || (lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && lc[0] <= g.ni - 1 &&
-                                         lc[1] <= g.nj - 1 && lc[2] <= g.nk - 1)) {
+        if (cells_of(g, lc, cl, off, rest) || (lc[0] >= 0 && lc[1] >= 0 && lc[2] >= 0 && lc[0] <= g.ni - 1 &&
+                                               lc[1] <= g.nj - 1 && lc[2] <= g.nk - 1)) {
             n0 = (int32_t)node_of(g, cl[0], cl[1], cl[2]);
-            corner_weights(off[0], off[1], off[2], W);
+            corner_weights(off, rest, W);
             mom_values(P, stride, p, w0, v);
 #pragma unroll
             for (int q = 0; q < NMOM; q++) v[q] *= scale[q]; /* exact: a power of two */
@@ -2574,7 +2575,8 @@ __global__ void __launch_bounds__(256) k_mcc_cex(Geo g, double3 rdh, double *P, 
             const int i = clamp_cell((int)lc[0], g.ni), j = clamp_cell((int)lc[1], g.nj),
                       k = clamp_cell((int)lc[2], g.nk);
             double W[8];
-            corner_weights(lc[0] - i, lc[1] - j, lc[2] - k, W);
+            const double off[3] = {lc[0] - i, lc[1] - j, lc[2] - k}, rest[3] = {1 - off[0], 1 - off[1], 1 - off[2]};
+            corner_weights(off, rest, W);
             const int64_t n0 = node_of(g, i, j, k), sy = g.ni, sz = (int64_t)g.ni * g.nj;
             const int64_t idx[8] = {n0,      n0 + 1,      n0 + 1 + sy,      n0 + sy,
                                     n0 + sz, n0 + 1 + sz, n0 + 1 + sy + sz, n0 + sy + sz};

@@ -63,16 +63,17 @@ __global__ void __launch_bounds__(256) k_na_clear(unsigned long long *acc, uint3
 /* A particle whose position is not finite, or whose weight is not within
  * [-weight_bound, weight_bound] (so that its corner counts could wrap the
  * int64 sums), deposits nothing and sets a bit of the flags.  Bound by the
- * float64 pipe, which runs the three differences, nine operations of the
- * quotients by dh, the offsets and the weights (6M particles on 97x89x117
- * nodes: 827 us with divisions and a conversion per weight, 475 us now). */
+ * float64 pipe and the integer work of scatter8 alike: float64 are the three
+ * differences, nine operations of the quotients by dh and seven products (6M
+ * particles on 97x89x117 nodes, the whole call: 869 us with divisions and a
+ * conversion per weight, 401 us now). */
 __global__ void __launch_bounds__(256) k_na_deposit(NaGeo g, const double *__restrict__ P, int64_t stride, int64_t n,
                                                     double fx, double weight_bound, unsigned long long *acc,
                                                     int *flags) {
     next_may_start();
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int nn3[3] = {g.ni, g.nj, g.nk};
-    double off[3] = {0, 0, 0}, value = 0;
+    double off[3] = {0, 0, 0}, rest[3] = {1, 1, 1}, value = 0;
     int c[3] = {0, 0, 0};
     bool unit = true, finite = true, in_range = true;
     const bool there = p < n;
@@ -86,9 +87,10 @@ __global__ void __launch_bounds__(256) k_na_deposit(NaGeo g, const double *__res
         if (finite && in_range)
 #pragma unroll
             for (int d = 0; d < 3; d++)
-                if (!espic::cell_of(lc[d], nn3[d], c[d], off[d])) {
+                if (!espic::cell_of(lc[d], nn3[d], c[d], off[d], rest[d])) {
                     c[d] = na_clamp((int)lc[d], nn3[d]);
                     off[d] = lc[d] - c[d];
+                    rest[d] = 1 - off[d];
                     unit = false;
                 }
     }
@@ -96,8 +98,8 @@ __global__ void __launch_bounds__(256) k_na_deposit(NaGeo g, const double *__res
     if (!(finite && in_range) && flags)
         atomicOr(flags, (finite ? 0 : ESPIC_NOALLOC_NONFINITE) | (in_range ? 0 : ESPIC_NOALLOC_RANGE));
     const int64_t sy = g.ni, sz = (int64_t)g.ni * g.nj;
-    espic::scatter8(acc, (uint32_t)(c[2] * sz + c[1] * sy + c[0]), sy, sz, off, value, fx, unit,
-                    there && finite && in_range);
+    espic::scatter8(acc, (uint32_t)(c[2] * sz + c[1] * sy + c[0]), sy, sz, off, rest, value, fx,
+                    unit, there && finite && in_range);
 }
 
 __global__ void __launch_bounds__(256) k_na_density(NaGeo g, const unsigned long long *acc, double unit, double *den) {
