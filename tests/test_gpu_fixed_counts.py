@@ -16,6 +16,7 @@ count.
 """
 import ctypes as C
 import math
+import sys
 
 import numpy as np
 import pytest
@@ -103,3 +104,13 @@ def test_moment_counts(espic, po, n, uniform):
     values = [P[6]] + [P[6] * P[3 + d] for d in range(3)] + [P[6] * P[3 + d] ** 2 for d in range(3)]
     for q in range(7):
         assert np.max(np.abs(mom[q] - ref[q])) <= n * np.max(np.abs(values[q])) * (2.0 ** -50 + n * 2.0 ** -53), q
+
+
+@pytest.mark.parametrize("n,spread", [(4096, 0), (4099, 30)])
+def test_deposit_counts_below_the_conversions(espic, monkeypatch, n, spread):
+    """Every count below 2^51 (2^40 2^S with S <= 10), cells up to 1023: the
+    products and offsets that are integer operations throughout."""
+    here = sys.modules[__name__]
+    monkeypatch.setattr(here, "GRID", (1025, 3, 5))
+    monkeypatch.setattr(here, "DH", np.array([2.0 ** -10, 0.5, 0.25]))
+    test_deposit_counts(espic, n, spread)
