@@ -134,6 +134,18 @@ __device__ __forceinline__ unsigned long long round_twice(Mantissa a, Mantissa b
     return (r + ((1ull << (t - 1)) - 1ull) + ((r >> t) & 1ull)) >> t;
 }
 
+/* (double)c, rounded to nearest even, by integer operations */
+__device__ __forceinline__ double count_to_double(long long c) {
+    const unsigned long long a = c < 0 ? 0ull - (unsigned long long)c : (unsigned long long)c;
+    const int n = __clzll((long long)a) & 63;
+    const unsigned long long m = a << n, h = m >> 11; /* 53 bits, the leading one on top */
+    const unsigned tail = (unsigned)m & 0x7ffu;
+    const unsigned long long up = tail > 0x400u - (unsigned)(h & 1ull); /* half and odd, or more than half */
+    const unsigned long long b = ((unsigned long long)(1085 - n) << 52) + h + up;
+    const double x = __longlong_as_double((long long)(b | ((unsigned long long)c & 0x8000000000000000ull)));
+    return a ? x : 0.0;
+}
+
 /* The warp's Field_::scatter of `value` at cell offsets d with e = 1 - d, each
  * corner weight value*(1-di)*(1-dj)*(1-dk) (the reference's operand order)
  * rounded once to an integer count of 1/fx and added to acc.  fx is a power

@@ -958,15 +958,29 @@ __global__ void k_targets(Geo g, const int32_t *__restrict__ obj, int32_t *targe
 
 /* ------------------------------------------------------------------------ */
 /* den = acc * unit / node_vol (0 where the volume is 0): the fixed-point sum
- * followed by Field_::operator/=, ch2/Field.h:125-134 */
-__global__ void k_density(int64_t nn, const unsigned long long *__restrict__ acc, double unit,
-                          const double *__restrict__ vol, const double *__restrict__ ivol, double *den) {
-    int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= nn) return;
-    double d = __ll2double_rn((long long)acc[u]) * unit;
-    double v = vol[u];
+ * followed by Field_::operator/=, ch2/Field.h:125-134.  Bound by the float64
+ * pipe, five operations a node, and by the loads in flight: the conversion
+ * of the count is made of integer operations and a thread takes two nodes
+ * with 16-byte loads (ten transport steps of 60M ions on 128x128x256 nodes,
+ * one of these each: 7.74 ms with a node a thread, 7.66 ms now). */
+__device__ __forceinline__ double node_density(unsigned long long count, double unit, double v, double iv) {
+    const double d = count_to_double((long long)count) * unit;
     /* d / v, correctly rounded, from RN(1/v) (the float64 pipe is narrow) */
-    den[u] = !zero_bits(v) ? div_rcp(d, v, ivol[u]) : 0.0;
+    return !zero_bits(v) ? div_rcp(d, v, iv) : 0.0;
+}
+
+__global__ void __launch_bounds__(128) k_density(int64_t nn, const unsigned long long *__restrict__ acc, double unit,
+                                                 const double *__restrict__ vol, const double *__restrict__ ivol,
+                                                 double *den) {
+    const int64_t u = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (u + 1 < nn) { /* the arrays are allocations of their own: u is 16-byte aligned */
+        const ulonglong2 c = *(const ulonglong2 *)(acc + u);
+        const double2 v = *(const double2 *)(vol + u), iv = *(const double2 *)(ivol + u);
+        *(double2 *)(den + u) =
+            make_double2(node_density(c.x, unit, v.x, iv.x), node_density(c.y, unit, v.y, iv.y));
+    } else if (u < nn) {
+        den[u] = node_density(acc[u], unit, vol[u], ivol[u]);
+    }
 }
 
 struct ChargeArgs {
@@ -1675,7 +1689,7 @@ void launch_compact(World &w, Species &s) {
 }
 
 void launch_density(World &w, Species &s) {
-    k_density<<<blocks_for(w.nn, 256), 256, 0, w.stream>>>(w.nn, s.acc, s.unit, w.vol, w.ivol, s.den);
+    k_density<<<blocks_for((w.nn + 1) / 2, 128), 128, 0, w.stream>>>(w.nn, s.acc, s.unit, w.vol, w.ivol, s.den);
     w.nlaunch++;
 }
 
