@@ -959,27 +959,30 @@ __global__ void k_targets(Geo g, const int32_t *__restrict__ obj, int32_t *targe
 /* ------------------------------------------------------------------------ */
 /* den = acc * unit / node_vol (0 where the volume is 0): the fixed-point sum
  * followed by Field_::operator/=, ch2/Field.h:125-134.  Bound by the float64
- * pipe, five operations a node, and by the loads in flight: the conversion
- * of the count is made of integer operations and a thread takes two nodes
- * with 16-byte loads (ten transport steps of 60M ions on 128x128x256 nodes,
- * one of these each: 7.74 ms with a node a thread, 7.66 ms now). */
+ * pipe, five operations a node, and by the loads in flight: on large grids
+ * the conversion of the count is made of integer operations and a thread
+ * takes two nodes with 16-byte loads (ten transport steps of 60M ions on
+ * 128x128x256 nodes, one of these each: 7.74 ms with a node a thread, 7.67 ms
+ * with two). */
+template <int PER>
 __device__ __forceinline__ double node_density(unsigned long long count, double unit, double v, double iv) {
-    const double d = count_to_double((long long)count) * unit;
+    const double c = PER > 1 ? count_to_double((long long)count) : __ll2double_rn((long long)count);
     /* d / v, correctly rounded, from RN(1/v) (the float64 pipe is narrow) */
-    return !zero_bits(v) ? div_rcp(d, v, iv) : 0.0;
+    return !zero_bits(v) ? div_rcp(c * unit, v, iv) : 0.0;
 }
 
-__global__ void __launch_bounds__(128) k_density(int64_t nn, const unsigned long long *__restrict__ acc, double unit,
+template <int PER>
+__global__ void __launch_bounds__(256) k_density(int64_t nn, const unsigned long long *__restrict__ acc, double unit,
                                                  const double *__restrict__ vol, const double *__restrict__ ivol,
                                                  double *den) {
-    const int64_t u = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-    if (u + 1 < nn) { /* the arrays are allocations of their own: u is 16-byte aligned */
+    const int64_t u = PER * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (PER == 2 && u + 1 < nn) { /* the arrays are allocations of their own: u is 16-byte aligned */
         const ulonglong2 c = *(const ulonglong2 *)(acc + u);
         const double2 v = *(const double2 *)(vol + u), iv = *(const double2 *)(ivol + u);
         *(double2 *)(den + u) =
-            make_double2(node_density(c.x, unit, v.x, iv.x), node_density(c.y, unit, v.y, iv.y));
+            make_double2(node_density<PER>(c.x, unit, v.x, iv.x), node_density<PER>(c.y, unit, v.y, iv.y));
     } else if (u < nn) {
-        den[u] = node_density(acc[u], unit, vol[u], ivol[u]);
+        den[u] = node_density<PER>(acc[u], unit, vol[u], ivol[u]);
     }
 }
 
@@ -1035,6 +1038,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_diag_partials(const double *__r
                                                                const int64_t *__restrict__ d_count, int uniform,
                                                                double w0, double *partials) {
     int64_t n = d_count[0];
+    if ((int64_t)blockIdx.x * RED_THREADS >= n) { /* block-uniform: no particle, and no float64 sums of zeros */
+        if (threadIdx.x < 5) partials[5 * blockIdx.x + threadIdx.x] = 0.0;
+        return;
+    }
     double acc[5] = {0, 0, 0, 0, 0};
     for (int64_t p = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; p < n; p += (int64_t)RED_BLOCKS * RED_THREADS) {
         double w, v0, v1, v2;
@@ -1104,7 +1111,7 @@ __global__ void __launch_bounds__(1024) k_pe_sum(const double *__restrict__ part
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0;
-        for (int w32 = 0; w32 < 32; w32++) t += ws[w32];
+        for (int w32 = 0; w32 < (int)(blockDim.x >> 5); w32++) t += ws[w32];
         out[0] = 0.5 * EPS_0 * t;
     }
 }
@@ -1689,7 +1696,13 @@ void launch_compact(World &w, Species &s) {
 }
 
 void launch_density(World &w, Species &s) {
-    k_density<<<blocks_for((w.nn + 1) / 2, 128), 128, 0, w.stream>>>(w.nn, s.acc, s.unit, w.vol, w.ivol, s.den);
+    /* two nodes a thread where that still fills every SM (2048 threads); on
+     * smaller grids it gains nothing (10 transport steps on 64x74x126 nodes:
+     * 0.81 ms either way) */
+    if (w.nn >= 2 * 2048 * (int64_t)w.sm_count)
+        k_density<2><<<blocks_for((w.nn + 1) / 2, 256), 256, 0, w.stream>>>(w.nn, s.acc, s.unit, w.vol, w.ivol, s.den);
+    else
+        k_density<1><<<blocks_for(w.nn, 256), 256, 0, w.stream>>>(w.nn, s.acc, s.unit, w.vol, w.ivol, s.den);
     w.nlaunch++;
 }
 
@@ -2162,7 +2175,9 @@ void launch_dsmc(World &w, Species &s, double dt, const double *d_u, int64_t nu,
 
 void launch_pe(World &w, double *d_out1) {
     if (w.pe_parts > 0) { /* the sum k_efield4 left behind */
-        k_pe_sum<<<1, 1024, 0, w.stream>>>(w.pe_part, w.pe_parts, d_out1);
+        /* no warps without a partial: theirs would be float64 sums of zeros */
+        const int threads = w.pe_parts < 1024 ? (int)((w.pe_parts + 31) / 32 * 32) : 1024;
+        k_pe_sum<<<1, threads, 0, w.stream>>>(w.pe_part, w.pe_parts, d_out1);
         w.nlaunch++;
         return;
     }
