@@ -182,8 +182,8 @@ struct World {
 /* n / d for n < 2^24, or n < 2^31 with a quotient below 2^22, without an
  * integer division: the float estimate (n, 1/d and the product each rounded
  * once) is within one of the quotient, and one remainder test corrects it */
-__device__ __forceinline__ uint32_t div_small(uint32_t n, uint32_t d, float inv_d) {
-    uint32_t q = __float2uint_rz((float)n * inv_d);
+__host__ __device__ __forceinline__ uint32_t div_small(uint32_t n, uint32_t d, float inv_d) {
+    uint32_t q = (uint32_t)((float)n * inv_d);
     const int32_t r = (int32_t)(n - q * d);
     if (r < 0) q--;
     else if (r >= (int32_t)d) q++;

@@ -25,6 +25,7 @@
 #include "ch4_push.h"
 #include "dfloat.h"
 #include "espic_world.h"
+#include "sor_box.h"
 
 namespace cg = cooperative_groups;
 
@@ -1169,8 +1170,9 @@ __device__ __forceinline__ bool colour_node(const Geo &g, const ColourRange &cr,
 
 /* What a node of the linear box needs in every sweep: its index and rho /
  * eps0, read once. */
+template <typename I>
 struct SorNode {
-    int32_t u; /* -1: none */
+    I u; /* -1: none */
     double b;
 };
 
@@ -1192,23 +1194,19 @@ static SorConst sor_const(const Geo &g) {
 }
 
 /* entry t (below n) of colour c's enumeration */
-__device__ __forceinline__ SorNode sor_node(const Geo &g, const SorConst &k, uint32_t hx, uint32_t t, uint32_t n,
-                                            int c, const double *__restrict__ rho) {
-    SorNode s = {-1, 0.0};
+template <typename I>
+__device__ __forceinline__ SorNode<I> sor_node(const Geo &g, const SorConst &k, I t, I n, int c,
+                                               const double *__restrict__ rho) {
+    SorNode<I> s = {-1, 0.0};
     if (t >= n) return s;
-    const uint32_t row = div_small(t, hx, 1.f / (float)hx);
-    const uint32_t kk = div_small(row, (uint32_t)(g.nj - 2), 1.f / (float)(g.nj - 2));
-    const int j = 1 + (int)(row - kk * (uint32_t)(g.nj - 2)), z = 1 + (int)kk;
-    const int i = 1 + 2 * (int)(t - row * hx) + ((1 + j + z + c) & 1);
-    if (i > g.ni - 2) return s;
-    s.u = (z * g.nj + j) * g.ni + i;
-    s.b = div_rcp(rho[s.u], k.eps0, k.reps0);
+    s.u = sor_entry<I>(g, t, c);
+    if (s.u >= 0) s.b = div_rcp(rho[s.u], k.eps0, k.reps0);
     return s;
 }
 
 /* the updated value of a node (operand order of ch2/PotentialSolver.cpp:27-42) */
-template <class P>
-__device__ __forceinline__ double sor_value(const SorConst &k, const P *phi, const SorNode &s, int32_t sy, int32_t sz) {
+template <class P, typename I>
+__device__ __forceinline__ double sor_value(const SorConst &k, const P *phi, const SorNode<I> &s, I sy, I sz) {
     const double x = phi[s.u];
     const double num = s.b + k.idx2 * (phi[s.u - 1] + phi[s.u + 1]) + k.idy2 * (phi[s.u - sy] + phi[s.u + sy]) +
                        k.idz2 * (phi[s.u - sz] + phi[s.u + sz]);
@@ -1216,9 +1214,8 @@ __device__ __forceinline__ double sor_value(const SorConst &k, const P *phi, con
 }
 
 /* the square of a node's residual (ch2/PotentialSolver.cpp:44-61) */
-template <class P>
-__device__ __forceinline__ double sor_residual2(const SorConst &k, const P *phi, const SorNode &s, int32_t sy,
-                                                int32_t sz) {
+template <class P, typename I>
+__device__ __forceinline__ double sor_residual2(const SorConst &k, const P *phi, const SorNode<I> &s, I sy, I sz) {
     if (s.u < 0) return 0.0;
     const double R = -phi[s.u] * k.D + s.b + k.idx2 * (phi[s.u - 1] + phi[s.u + 1]) +
                      k.idy2 * (phi[s.u - sy] + phi[s.u + sy]) + k.idz2 * (phi[s.u - sz] + phi[s.u + sz]);
@@ -1239,24 +1236,26 @@ __device__ __forceinline__ void sor_status(SolveStatus *st, int conv, int it, do
  * again in every sweep.  Bound by the barrier after each half sweep (1.3 us)
  * and the memory latency behind it (23x47x37: 4.6 us a sweep).  With 64-bit
  * integer divisions and two float64 divisions per node a sweep of the 21^3
- * box took 7.5 us on 15 SMs. */
+ * box took 7.5 us on 15 SMs.  I: int32_t with sor_short_indices, else
+ * int64_t, which divides by 64-bit integers and holds no nodes (it has 2^24
+ * entries or more). */
 constexpr int SOR_HELD = 2;
 
+template <typename I>
 __global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi, const double *__restrict__ rho,
                                                  int max_it, double tol, double *partials, SolveStatus *st,
                                                  int *err) {
     cg::grid_group grid = cg::this_grid();
-    const int32_t sy = g.ni, sz = g.ni * g.nj;
-    const uint32_t hx = (uint32_t)(g.ni - 1) / 2;
-    const uint32_t count = hx * (uint32_t)(g.nj - 2) * (uint32_t)(g.nk - 2);
-    const uint32_t gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool held = count <= SOR_HELD * gsize;
-    SorNode node[2][SOR_HELD];
+    const I sy = g.ni, sz = (I)g.ni * g.nj;
+    const I count = (I)(sor_row_entries(g) * sor_rows(g));
+    const I gsize = (I)gridDim.x * blockDim.x, gtid = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool held = sizeof(I) == 4 && count <= SOR_HELD * gsize;
+    SorNode<I> node[2][SOR_HELD];
     if (held)
 #pragma unroll
         for (int c = 0; c < 2; c++)
 #pragma unroll
-            for (int h = 0; h < SOR_HELD; h++) node[c][h] = sor_node(g, k, hx, gtid + h * gsize, count, c, rho);
+            for (int h = 0; h < SOR_HELD; h++) node[c][h] = sor_node<I>(g, k, gtid + h * gsize, count, c, rho);
     double L2 = 0;
     int conv = 0, it, round = 0;
     for (it = 0; it < max_it; it++) {
@@ -1271,8 +1270,8 @@ __global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi,
                 for (int h = 0; h < SOR_HELD; h++)
                     if (node[c][h].u >= 0) phi[node[c][h].u] = v[h];
             } else {
-                for (uint32_t t = gtid; t < count; t += gsize) {
-                    const SorNode s = sor_node(g, k, hx, t, count, c, rho);
+                for (I t = gtid; t < count; t += gsize) {
+                    const SorNode<I> s = sor_node<I>(g, k, t, count, c, rho);
                     if (s.u >= 0) phi[s.u] = sor_value(k, phi, s, sy, sz);
                 }
             }
@@ -1286,8 +1285,8 @@ __global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi,
 #pragma unroll
                     for (int h = 0; h < SOR_HELD; h++) sum += sor_residual2(k, phi, node[c][h], sy, sz);
                 } else {
-                    for (uint32_t t = gtid; t < count; t += gsize)
-                        sum += sor_residual2(k, phi, sor_node(g, k, hx, t, count, c, rho), sy, sz);
+                    for (I t = gtid; t < count; t += gsize)
+                        sum += sor_residual2(k, phi, sor_node<I>(g, k, t, count, c, rho), sy, sz);
                 }
             }
             double tot = grid_sum(grid, sum, partials, round);
@@ -1324,11 +1323,10 @@ __global__ void __launch_bounds__(SOR_CTA_NODES) k_sor_cluster(Geo g, SorConst k
     __shared__ double warp_sum[SOR_CTA_NODES / 32];
     const int rank = (int)cl.block_rank();
     const int32_t sy = g.ni, sz = g.ni * g.nj, nn = sz * g.nk;
-    const uint32_t hx = (uint32_t)(g.ni - 1) / 2;
-    const uint32_t count = hx * (uint32_t)(g.nj - 2) * (uint32_t)(g.nk - 2);
-    const uint32_t t = (uint32_t)rank * per + threadIdx.x;
-    const uint32_t top = threadIdx.x < per ? count : 0u;
-    const SorNode node[2] = {sor_node(g, k, hx, t, top, 0, rho), sor_node(g, k, hx, t, top, 1, rho)};
+    const int32_t count = (int32_t)(sor_row_entries(g) * sor_rows(g));
+    const int32_t t = rank * (int32_t)per + (int32_t)threadIdx.x;
+    const int32_t top = threadIdx.x < per ? count : 0;
+    const SorNode<int32_t> node[2] = {sor_node(g, k, t, top, 0, rho), sor_node(g, k, t, top, 1, rho)};
     for (int32_t u = threadIdx.x; u < nn; u += blockDim.x) sor_phi[u] = phi[u];
     cl.sync();
     double L2 = 0;
@@ -2231,8 +2229,7 @@ static bool sor_cluster_fits(World &w, uint32_t per, size_t smem) {
 }
 
 int launch_sor_box(World &w, int max_it, double tol) {
-    const uint32_t plane = (uint32_t)((w.g.ni - 1) / 2) * (uint32_t)(w.g.nj - 2);
-    int64_t work = (int64_t)plane * (w.g.nk - 2);
+    const int64_t work = sor_row_entries(w.g) * sor_rows(w.g);
     Geo g = w.g;
     SorConst k = sor_const(g);
     double *phi = w.phi;
@@ -2255,15 +2252,17 @@ int launch_sor_box(World &w, int max_it, double tol) {
         a.val.clusterDim.y = a.val.clusterDim.z = 1;
         cfg.attrs = &a;
         cfg.numAttrs = 1;
+        const uint32_t plane = (uint32_t)sor_row_entries(w.g) * (uint32_t)(w.g.nj - 2);
         const int reach = (int)((per + plane) / per);
         return (int)cudaLaunchKernelEx(&cfg, k_sor_cluster, g, k, phi, rho, max_it, tol, per, reach, st, err);
     }
     /* a node of a colour per thread over all SMs, before blocks grow */
     int threads = (int)((work + w.sm_count - 1) / w.sm_count + 31) & ~31;
     threads = threads < 64 ? 64 : (threads > 256 ? 256 : threads);
-    int grid = coop_grid(w, (const void *)k_sor_box, threads, work);
+    const void *fn = sor_short_indices(g) ? (const void *)k_sor_box<int32_t> : (const void *)k_sor_box<int64_t>;
+    int grid = coop_grid(w, fn, threads, work);
     void *args[] = {&g, &k, &phi, &rho, &max_it, &tol, &part, &st, &err};
-    return (int)cudaLaunchCooperativeKernel((const void *)k_sor_box, grid, threads, args, 0, w.stream);
+    return (int)cudaLaunchCooperativeKernel(fn, grid, threads, args, 0, w.stream);
 }
 
 int launch_gs_sphere(World &w, int max_it, double tol) {

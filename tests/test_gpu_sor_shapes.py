@@ -26,3 +26,17 @@ def test_sor_routes_match_the_oracle(espic, po, nodes, blocks):
         sol.solve()
         want, _, _, _ = po.sor_box(g, np.zeros(g.nn), rho, its, 0.0, "rb")
         assert np.array_equal(w.phi, want)
+
+
+def test_thin_box_of_many_rows(espic, po):
+    """11.6M interior rows of three entries a colour: the route with 64-bit
+    division (its 46,899 entries that a float estimate would misplace lie at
+    the far end)."""
+    nodes, x0, xm = (7, 3402, 3402), [-0.1, -0.1, 0.0], [0.1, 0.1, 0.2]
+    g = po.grid(nodes, x0, xm)
+    rho = 1.6e-8 * np.random.default_rng(7).standard_normal(g.nn)
+    with espic.World(*nodes, x0, xm) as w:
+        w.write(espic.FIELD_RHO, rho)
+        espic.PotentialSolver(w, espic.SOLVER_SOR, 2, 0.0).solve()
+        want, _, _, _ = po.sor_box(g, np.zeros(g.nn), rho, 2, 0.0, "rb")
+        assert np.array_equal(w.phi, want)
