@@ -825,7 +825,10 @@ static cudaError_t ens_launch_solve(espic_ensemble &E, int solve) {
         const int64_t er = e + 4 * ens_slab_r(b.g.ni, b.g.nj, b.g.nk, E.cluster);
         bytes = std::max(bytes, er <= ENS_SLAB_MAX ? er : (e <= ENS_SLAB_MAX ? e : 0));
     }
-    cudaError_t fe = cudaFuncSetAttribute(k_ens_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    /* the limit belongs to the kernel, not to this ensemble: always the same
+     * value, or another thread's ensemble could lower it before the launch */
+    cudaError_t fe =
+        cudaFuncSetAttribute(k_ens_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ENS_SLAB_MAX);
     if (fe != cudaSuccess) return fe;
     cfg.dynamicSmemBytes = (size_t)bytes;
     cfg.stream = E.stream;

@@ -257,3 +257,40 @@ def test_solve_routes_by_box_shape(espic, po, nodes, cluster):
     other = solved(2)
     for a, b in zip((phi, rho, ef), other):
         assert np.array_equal(a, b)
+
+
+def test_two_ensembles_from_two_threads(espic):
+    """An ensemble whose boxes need no slab in shared memory beside one whose
+    boxes need most of it, each stepped by its own host thread: a launch must
+    not depend on what the other thread set up."""
+    import threading
+
+    def make(nodes):
+        n = 100
+        E = espic.Ensemble([nodes], X0, XM, MASS, CHARGE, [[1e5, 1e5]], [[n, n]], 2e-10)
+        E.set_launch(4096, 256, 1024, 1)
+        for sp in range(2):
+            P = box_state(X0, XM, n, sp)
+            P[6] = 1e5
+            E.set_particles(0, sp, P)
+        E.set_solver(25, 1e-4, 0.0)
+        E.prepare()
+        return E
+
+    errors = []
+
+    def steps(E):
+        try:
+            for _ in range(800):
+                E.step(1, graph=False)
+            E.sync()
+        except Exception as e:
+            errors.append(e)
+
+    with make([120, 118, 20]) as a, make([30, 30, 20]) as b:
+        threads = [threading.Thread(target=steps, args=(E,)) for E in (a, b)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not errors, errors
