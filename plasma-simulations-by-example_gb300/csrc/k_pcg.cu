@@ -2203,7 +2203,9 @@ static int run_pcg(World &w) {
     size_t dyn = 0;
     if (A.smem_from >= 0)
         for (int i = A.smem_from; i < A.nlev; i++) dyn += level_smem_bytes<T>(A.L[i].n);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    /* the kernel's limit, not this world's need: another thread's world must
+     * not lower it before the launch */
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PCG_SMEM_MAX);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn);
     if (per_sm < 1) per_sm = 1;
