@@ -164,6 +164,27 @@ __host__ __device__ inline int64_t ens_slab_r(int ni, int nj, int nk, int C) {
     return 2ll * ens_planes(nk, C).most() * nj * ens_slots(ni);
 }
 
+/* Pieces of the residual's sum, whose bits depend on neither the cluster nor
+ * the block size: a plane's nodes in ENS_PLANE_WARPS virtual warps (ens_warp_sum
+ * of each), their sums in order (ens_plane_sum), and the planes' sums over the
+ * lanes of a warp (ens_planes_total; get(p) is plane p's, all lanes get the
+ * total). */
+__device__ __forceinline__ double ens_warp_sum(double x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+__device__ __forceinline__ double ens_plane_sum(const double *part) {
+    double s = 0;
+    for (int w = 0; w < ENS_PLANE_WARPS; w++) s += part[w];
+    return s;
+}
+template <class F>
+__device__ __forceinline__ double ens_planes_total(int planes, F get) {
+    double s = 0;
+    for (int p = (int)(threadIdx.x & 31); p < planes; p += 32) s += get(p);
+    return ens_warp_sum(s);
+}
+
 /* The sweeps of one box with the correction in shared memory.  Each CTA owns
  * a run of planes; its float32 correction e, and its right-hand side R where
  * that fits too (else R lies in global memory in the same order, a colour
@@ -176,10 +197,9 @@ __host__ __device__ inline int64_t ens_slab_r(int ni, int nj, int nk, int C) {
  * and found its nodes by integer divisions.  Boxes of 16 to 64 nodes an
  * axis, 8 CTAs: a half sweep 1.9 us on average, a step's solve of 64 boxes
  * 5.2 ms before, 2.9 ms now; what is left is a third float64 residuals (14
- * instructions a node).  The residual's sum is taken
- * plane by plane (ENS_PLANE_WARPS virtual warps each, a fixed tree) and the
- * planes' sums by a fixed tree, so it depends on neither the cluster nor the
- * block size.  Returns the sweeps done; conv and L2 as the caller's. */
+ * instructions a node).  The residual's sum is taken as in k_ens_solve, the
+ * planes' sums from the CTAs' shared memory.  Returns the sweeps done; conv
+ * and L2 as the caller's. */
 __device__ __forceinline__ int ens_sor_slab(cg::cluster_group &cl, const EnsBox &B, double *ph,
                                             const double *__restrict__ rh, float *R0, float *R1, int max_it,
                                             double tol, bool r_shared, float *slab, double *part, double *plane_sum, double *total,
@@ -243,26 +263,20 @@ __device__ __forceinline__ int ens_sor_slab(cg::cluster_group &cl, const EnsBox 
                 E[c * ecol + (kk + 1) * plane + o] = 0.f;
                 acc2 += Ru * Ru;
             }
-            for (int o = 16; o > 0; o >>= 1) acc2 += __shfl_xor_sync(0xffffffffu, acc2, o);
+            acc2 = ens_warp_sum(acc2);
             if (lane == 0) part[task] = acc2;
         }
         if (sweeps) /* the halo planes: what the neighbours wrote */
             for (int t = tid; t < plane; t += nt)
                 for (int c = 0; c < 2; c++) E[c * ecol + t] = E[c * ecol + (np + 1) * plane + t] = 0.f;
         __syncthreads();
-        for (int kk = tid; kk < np; kk += nt) {
-            double s = 0;
-            for (int w = 0; w < ENS_PLANE_WARPS; w++) s += part[kk * ENS_PLANE_WARPS + w];
-            plane_sum[kk] = s;
-        }
+        for (int kk = tid; kk < np; kk += nt) plane_sum[kk] = ens_plane_sum(part + kk * ENS_PLANE_WARPS);
         cluster_sync_global(cl);
         if (warp == 0) {
-            double s = 0;
-            for (int p = lane; p < pl.planes; p += 32) {
+            const double s = ens_planes_total(pl.planes, [&](int p) {
                 const int o = pl.owner(p);
-                s += *cl.map_shared_rank(plane_sum + (p - pl.first(o)), o);
-            }
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                return *cl.map_shared_rank(plane_sum + (p - pl.first(o)), o);
+            });
             if (lane == 0) *total = s;
         }
         __syncthreads();
@@ -336,13 +350,12 @@ __device__ __forceinline__ int ens_sor_slab(cg::cluster_group &cl, const EnsBox 
 /* One box per thread-block cluster of C CTAs (C = 1, 2, 4 or 8, chosen at
  * launch): the CTAs split every node pass and every half sweep into
  * contiguous slices and meet at cluster barriers.  Boxes whose slabs fit the
- * launch's shared memory are swept there (ens_sor_slab), the others here.  The box a cluster works
- * on is claimed by CTA 0 and read by the others from its shared memory.  The
- * residual sum uses the fixed layout of ENS_VW virtual threads (node t
- * belongs to virtual thread t mod ENS_VW; CTA r owns a contiguous range of
- * virtual threads); CTA 0 gathers the ENS_VW partials through distributed
- * shared memory and sums them in a fixed tree, so the result depends on
- * neither C nor the block size. */
+ * launch's shared memory are swept there (ens_sor_slab), the others here.  The
+ * box a cluster works on is claimed by CTA 0 and read by the others from its
+ * shared memory.  The residual is summed plane by plane on both routes (see
+ * ens_planes_total), here with the planes' sums in global memory, so the
+ * solve's outcome depends on neither C nor the block size, nor on whether
+ * these let the box's slab fit. */
 __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ boxes, const EnsSeg *__restrict__ segs,
                                                     int nsp, const int *__restrict__ order, int nbox, int *counter,
                                                     double *phi, double *rho, float *ecor, float *res, float4 *ef4,
@@ -357,7 +370,7 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
     __shared__ double total;
     __shared__ int sb;
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int vper = ENS_VW / C, v0 = rank * vper, v1 = v0 + vper;
+    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     for (;;) {
         if (rank == 0 && tid == 0) sb = atomicAdd(counter, 1);
         cluster_sync_global(cl);
@@ -428,31 +441,41 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
         if (solve && slab)
             sweeps = ens_sor_slab(cl, B, ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab, part, plane_sum,
                                   &total, conv, L2, err);
+        constexpr int PLANES = ENS_VW / ENS_PLANE_WARPS; /* planes that part holds */
+        const EnsPlanes pl = ens_planes(nk, C);
+        const int pa = rank < pl.parts ? pl.first(rank) : 0, pb = rank < pl.parts ? pl.first(rank + 1) : 0;
+        const uint32_t in_row = (uint32_t)(ni - 2), in_plane = in_row * (uint32_t)(nj - 2);
+        double *psum = (double *)(ef4 + B.node0); /* the box's E is written after the solve */
         while (solve && !slab) {
-            for (int v = v0 + tid; v < v1; v += nt) {
-                double acc2 = 0;
-                for (int t = v; t < interior; t += ENS_VW) {
-                    const int i = 1 + t % (ni - 2);
-                    const int r = t / (ni - 2);
-                    const int j = 1 + r % (nj - 2);
-                    const int k = 1 + r / (nj - 2);
-                    const int u = (k * nj + j) * ni + i;
-                    const double Ru = -ph[u] * D + div_rcp(rh[u], ENS_EPS_0, yeps) + idx2 * (ph[u - 1] + ph[u + 1]) +
-                                      idy2 * (ph[u - sy] + ph[u + sy]) + idz2 * (ph[u - sz] + ph[u + sz]);
-                    R[u] = (float)Ru;
-                    e[u] = 0.f;
-                    acc2 += Ru * Ru;
+            for (int p0 = pa; p0 < pb; p0 += PLANES) {
+                const int np = pb - p0 < PLANES ? pb - p0 : PLANES;
+                for (int task = warp; task < np * ENS_PLANE_WARPS; task += nw) {
+                    const int k = 1 + p0 + task / ENS_PLANE_WARPS, vw = task % ENS_PLANE_WARPS;
+                    double acc2 = 0;
+                    for (uint32_t t = (uint32_t)(vw * 32 + lane); t < in_plane; t += 32 * ENS_PLANE_WARPS) {
+                        const uint32_t r = t / in_row;
+                        const int u = (k * nj + 1 + (int)r) * ni + 1 + (int)(t - r * in_row);
+                        const double Ru = -ph[u] * D + div_rcp(rh[u], ENS_EPS_0, yeps) +
+                                          idx2 * (ph[u - 1] + ph[u + 1]) + idy2 * (ph[u - sy] + ph[u + sy]) +
+                                          idz2 * (ph[u - sz] + ph[u + sz]);
+                        R[u] = (float)Ru;
+                        e[u] = 0.f;
+                        acc2 += Ru * Ru;
+                    }
+                    acc2 = ens_warp_sum(acc2);
+                    if (lane == 0) part[task] = acc2;
                 }
-                part[v] = acc2;
+                __syncthreads();
+                for (int kk = tid; kk < np; kk += nt) psum[p0 + kk] = ens_plane_sum(part + kk * ENS_PLANE_WARPS);
+                __syncthreads();
             }
             cluster_sync_global(cl);
-            if (rank == 0) {
-                for (int v = vper + tid; v < ENS_VW; v += nt) part[v] = *cl.map_shared_rank(&part[v], v / vper);
-                const double t = ens_tree_sum(part);
-                if (tid == 0) total = t;
+            if (warp == 0) {
+                const double t = ens_planes_total(pl.planes, [&](int p) { return __ldcg(psum + p); });
+                if (lane == 0) total = t;
             }
-            cluster_sync_global(cl);
-            L2 = sqrt(*cl.map_shared_rank(&total, 0) / ((double)ni * nj * nk));
+            __syncthreads();
+            L2 = sqrt(total / ((double)ni * nj * nk));
             if (!isfinite(L2)) {
                 if (rank == 0 && tid == 0) atomicOr(err, DERR_NONFINITE);
                 break;
@@ -512,6 +535,7 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
             }
             cluster_sync_global(cl);
         }
+        if (solve && !slab) cluster_sync_global(cl); /* psum is read before E takes its place */
         /* 3. E = -grad phi, float32 copy for the push */
         /* interior nodes first, the face nodes in passes of their own: a
          * row of at most 64 nodes puts a face lane into every warp, and the

@@ -294,3 +294,27 @@ def test_two_ensembles_from_two_threads(espic):
         for t in threads:
             t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("nodes", [(61, 64, 64), (4, 5, 3), (9, 10, 200)])
+def test_residual_does_not_depend_on_the_cluster(espic, nodes):
+    """The residuals' bits and the sweep counts of sixteen boxes' solves, for
+    cluster sizes and block sizes that sweep a box in shared memory and that
+    do not."""
+    n, nb = 5000, 16
+    mpw = [1e11 * 0.008 / n, 1e11 * 0.001 / n]
+    got = []
+    for cluster, threads in ((1, 1024), (2, 256), (4, 1024), (8, 512)):
+        with espic.Ensemble([list(nodes)] * nb, X0, XM, MASS, CHARGE, mpw, [[n, n]] * nb, 2e-10) as E:
+            E.set_launch(4096, 256, threads, cluster)
+            for b in range(nb):
+                for sp in range(2):
+                    P = box_state(X0, XM, n, 2 * b + sp, octant=sp == 1)
+                    P[6] = mpw[sp]
+                    E.set_particles(b, sp, P)
+            E.set_solver(75, 1e-300, 0.0)
+            E.prepare()
+            sweeps, _, res = E.status()
+            got.append([(int(k), float(r).hex()) for k, r in zip(sweeps, res)])
+    for other in got[1:]:
+        assert other == got[0]
