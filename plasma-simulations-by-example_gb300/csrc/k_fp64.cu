@@ -162,7 +162,9 @@ static SphereReject sphere_reject(const World &w) {
         L = fmax(L, fmax(fabs(w.sphere[d]), fmax(fabs(w.g.x0[d]), fabs(w.g.xm[d]))));
     }
     const double r = w.has_sphere ? sqrt(w.sphere[3]) + 8 * ldexp(1.0, -21) * (L + sqrt(w.sphere[3])) : 0;
-    s.rej2 = w.has_sphere ? (float)(r * r * 1.00001) : -1.f;
+    /* squares near the smallest floats lose their relative accuracy: no
+     * particle then skips the float64 test */
+    s.rej2 = !w.has_sphere ? -1.f : (r * r > 1e-36 ? (float)(r * r * 1.00001) : INFINITY);
     return s;
 }
 
