@@ -185,6 +185,11 @@ __device__ __forceinline__ double ens_planes_total(int planes, F get) {
     return ens_warp_sum(s);
 }
 
+struct EnsSolved {
+    int sweeps, converged;
+    double residual;
+};
+
 /* The sweeps of one box with the correction in shared memory.  Each CTA owns
  * a run of planes; its float32 correction e, and its right-hand side R where
  * that fits too (else R lies in global memory in the same order, a colour
@@ -198,12 +203,11 @@ __device__ __forceinline__ double ens_planes_total(int planes, F get) {
  * axis, 8 CTAs: a half sweep 1.9 us on average, a step's solve of 64 boxes
  * 5.2 ms before, 2.9 ms now; what is left is a third float64 residuals (14
  * instructions a node).  The residual's sum is taken as in k_ens_solve, the
- * planes' sums from the CTAs' shared memory.  Returns the sweeps done; conv
- * and L2 as the caller's. */
-__device__ __forceinline__ int ens_sor_slab(cg::cluster_group &cl, const EnsBox &B, double *ph,
-                                            const double *__restrict__ rh, float *R0, float *R1, int max_it,
-                                            double tol, bool r_shared, float *slab, double *part, double *plane_sum, double *total,
-                                            int &conv, double &L2, int *err) {
+ * planes' sums from the CTAs' shared memory. */
+__device__ __noinline__ EnsSolved ens_sor_slab(const EnsBox &B, double *ph, const double *__restrict__ rh, float *R0,
+                                               float *R1, int max_it, double tol, bool r_shared, float *slab,
+                                               double *part, double *plane_sum, double *total, int *err) {
+    cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
     const Geo &g = B.g;
     const int ni = g.ni, nj = g.nj, nk = g.nk, sy = ni, sz = ni * nj;
@@ -233,7 +237,8 @@ __device__ __forceinline__ int ens_sor_slab(cg::cluster_group &cl, const EnsBox 
     const int below_top = rank > 0 && on ? (pl.first(rank) - pl.first(rank - 1) + 1) * plane : 0;
     for (int t = tid; t < 2 * ecol; t += nt) E[t] = 0.f;
     __syncthreads();
-    int sweeps = 0;
+    int sweeps = 0, conv = 0;
+    double L2 = 0;
     /* with R in shared memory the work arrays hold the halves of rho / eps0,
      * written in the first residual pass */
     int *b_hi = (int *)R0, *b_lo = (int *)R1;
@@ -344,7 +349,140 @@ __device__ __forceinline__ int ens_sor_slab(cg::cluster_group &cl, const EnsBox 
         cluster_sync_global(cl);
     }
     cluster_sync_global(cl); /* plane_sum and the halo planes are free again */
-    return sweeps;
+    return {sweeps, conv, L2};
+}
+
+/* The sweeps of one box whose slab does not fit the launch's shared memory:
+ * e and R in global memory, every half sweep's nodes an even share of each
+ * CTA.  psum: the planes' sums, one double a plane of the box.  A function of
+ * its own, like ens_sor_slab: inlined into one kernel the two spilled. */
+__device__ __noinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, const double *__restrict__ rh, float *R,
+                                                 float *e, int max_it, double tol, double *psum, double *part,
+                                                 double *total, int *err) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
+    const Geo &g = B.g;
+    const int ni = g.ni, nj = g.nj, nk = g.nk, sy = ni, sz = ni * nj;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    const double idx2 = 1.0 / (g.dh[0] * g.dh[0]);
+    const double idy2 = 1.0 / (g.dh[1] * g.dh[1]);
+    const double idz2 = 1.0 / (g.dh[2] * g.dh[2]);
+    const double D = 2 * idx2 + 2 * idy2 + 2 * idz2;
+    const float fcx = (float)idx2, fcy = (float)idy2, fcz = (float)idz2, fiD = (float)(1.0 / D);
+    const double yeps = 1.0 / ENS_EPS_0;
+    const float fw = (float)B.omega;
+    const int hx = (ni - 2 + 1) / 2;
+    const int count = hx * (nj - 2) * (nk - 2);
+    const int interior = (ni - 2) * (nj - 2) * (nk - 2);
+    const int c0 = (int)((int64_t)count * rank / C), c1 = (int)((int64_t)count * (rank + 1) / C);
+    const int i0 = (int)((int64_t)interior * rank / C), i1 = (int)((int64_t)interior * (rank + 1) / C);
+    constexpr int PLANES = ENS_VW / ENS_PLANE_WARPS; /* planes that part holds */
+    const EnsPlanes pl = ens_planes(nk, C);
+    const int pa = rank < pl.parts ? pl.first(rank) : 0, pb = rank < pl.parts ? pl.first(rank + 1) : 0;
+    const uint32_t in_row = (uint32_t)(ni - 2), in_plane = in_row * (uint32_t)(nj - 2);
+    int sweeps = 0, conv = 0;
+    double L2 = 0;
+    for (;;) {
+        for (int p0 = pa; p0 < pb; p0 += PLANES) {
+            const int np = pb - p0 < PLANES ? pb - p0 : PLANES;
+            for (int task = warp; task < np * ENS_PLANE_WARPS; task += nw) {
+                const int k = 1 + p0 + task / ENS_PLANE_WARPS, vw = task % ENS_PLANE_WARPS;
+                double acc2 = 0;
+                /* two nodes at once, all loads before any store */
+                for (uint32_t t0 = (uint32_t)(vw * 32 + lane); t0 < in_plane; t0 += 64 * ENS_PLANE_WARPS) {
+                    int uq[2];
+                    double Rq[2];
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        const uint32_t t = t0 + q * 32 * ENS_PLANE_WARPS, r = t / in_row;
+                        uq[q] = t < in_plane ? (k * nj + 1 + (int)r) * ni + 1 + (int)(t - r * in_row) : -1;
+                        const int u = uq[q] < 0 ? (k * nj + 1) * ni + 1 : uq[q];
+                        Rq[q] = -ph[u] * D + div_rcp(rh[u], ENS_EPS_0, yeps) + idx2 * (ph[u - 1] + ph[u + 1]) +
+                                idy2 * (ph[u - sy] + ph[u + sy]) + idz2 * (ph[u - sz] + ph[u + sz]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        if (uq[q] < 0) continue;
+                        R[uq[q]] = (float)Rq[q];
+                        e[uq[q]] = 0.f;
+                        acc2 += Rq[q] * Rq[q];
+                    }
+                }
+                acc2 = ens_warp_sum(acc2);
+                if (lane == 0) part[task] = acc2;
+            }
+            __syncthreads();
+            for (int kk = tid; kk < np; kk += nt) psum[p0 + kk] = ens_plane_sum(part + kk * ENS_PLANE_WARPS);
+            __syncthreads();
+        }
+        cluster_sync_global(cl);
+        if (warp == 0) {
+            const double t = ens_planes_total(pl.planes, [&](int p) { return __ldcg(psum + p); });
+            if (lane == 0) *total = t;
+        }
+        __syncthreads();
+        L2 = sqrt(*total / ((double)ni * nj * nk));
+        if (!isfinite(L2)) {
+            if (rank == 0 && tid == 0) atomicOr(err, DERR_NONFINITE);
+            break;
+        }
+        if (L2 < tol) {
+            conv = 1;
+            break;
+        }
+        if (sweeps >= max_it) break;
+        /* ENS_SWEEPS float32 sweeps of L e = -R, then phi += e and the
+         * float64 residual decides again */
+        const int ns = max_it - sweeps < ENS_SWEEPS ? max_it - sweeps : ENS_SWEEPS;
+        for (int s = 0; s < ns; s++) {
+            for (int c = 0; c < 2; c++) {
+                /* four independent nodes of colour c per thread: all
+                 * loads before any store */
+                for (int tb = c0 + tid; tb < c1; tb += 4 * nt) {
+                    int uq[4];
+                    float eo[4], sum[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int t = tb + q * nt;
+                        uq[q] = -1;
+                        eo[q] = 0.f;
+                        sum[q] = 0.f;
+                        if (t >= c1) continue;
+                        const int i2 = t % hx;
+                        const int r = t / hx;
+                        const int j = 1 + r % (nj - 2);
+                        const int k = 1 + r / (nj - 2);
+                        const int i = 1 + 2 * i2 + ((1 + j + k + c) & 1);
+                        if (i > ni - 2) continue;
+                        const int u = (k * nj + j) * ni + i;
+                        uq[q] = u;
+                        eo[q] = e[u];
+                        sum[q] = R[u] + fcx * (e[u - 1] + e[u + 1]) + fcy * (e[u - sy] + e[u + sy]) +
+                                 fcz * (e[u - sz] + e[u + sz]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (uq[q] < 0) continue;
+                        const float en = sum[q] * fiD;
+                        e[uq[q]] = eo[q] + fw * (en - eo[q]);
+                    }
+                }
+                cluster_sync_global(cl);
+            }
+        }
+        sweeps += ns;
+        for (int t = i0 + tid; t < i1; t += nt) {
+            const int i = 1 + t % (ni - 2);
+            const int r = t / (ni - 2);
+            const int j = 1 + r % (nj - 2);
+            const int k = 1 + r / (nj - 2);
+            const int u = (k * nj + j) * ni + i;
+            ph[u] += (double)e[u];
+        }
+        cluster_sync_global(cl);
+    }
+    cluster_sync_global(cl); /* psum is free again */
+    return {sweeps, conv, L2};
 }
 
 /* One box per thread-block cluster of C CTAs (C = 1, 2, 4 or 8, chosen at
@@ -370,7 +508,6 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
     __shared__ double total;
     __shared__ int sb;
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     for (;;) {
         if (rank == 0 && tid == 0) sb = atomicAdd(counter, 1);
         cluster_sync_global(cl);
@@ -423,119 +560,13 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
         cluster_sync_global(cl);
         /* 2. red-black SOR: float32 correction sweeps under the float64
          *    residual */
-        const double idx2 = 1.0 / (g.dh[0] * g.dh[0]);
-        const double idy2 = 1.0 / (g.dh[1] * g.dh[1]);
-        const double idz2 = 1.0 / (g.dh[2] * g.dh[2]);
-        const double D = 2 * idx2 + 2 * idy2 + 2 * idz2;
-        const float fcx = (float)idx2, fcy = (float)idy2, fcz = (float)idz2, fiD = (float)(1.0 / D);
-        const double yeps = 1.0 / ENS_EPS_0;
-        const float fw = (float)B.omega;
         const int sy = ni, sz = ni * nj;
-        const int hx = (ni - 2 + 1) / 2;
-        const int count = hx * (nj - 2) * (nk - 2);
-        const int interior = (ni - 2) * (nj - 2) * (nk - 2);
-        const int c0 = (int)((int64_t)count * rank / C), c1 = (int)((int64_t)count * (rank + 1) / C);
-        const int i0 = (int)((int64_t)interior * rank / C), i1 = (int)((int64_t)interior * (rank + 1) / C);
-        int sweeps = 0, conv = 0;
-        double L2 = 0;
+        EnsSolved done = {0, 0, 0.0};
         if (solve && slab)
-            sweeps = ens_sor_slab(cl, B, ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab, part, plane_sum,
-                                  &total, conv, L2, err);
-        constexpr int PLANES = ENS_VW / ENS_PLANE_WARPS; /* planes that part holds */
-        const EnsPlanes pl = ens_planes(nk, C);
-        const int pa = rank < pl.parts ? pl.first(rank) : 0, pb = rank < pl.parts ? pl.first(rank + 1) : 0;
-        const uint32_t in_row = (uint32_t)(ni - 2), in_plane = in_row * (uint32_t)(nj - 2);
-        double *psum = (double *)(ef4 + B.node0); /* the box's E is written after the solve */
-        while (solve && !slab) {
-            for (int p0 = pa; p0 < pb; p0 += PLANES) {
-                const int np = pb - p0 < PLANES ? pb - p0 : PLANES;
-                for (int task = warp; task < np * ENS_PLANE_WARPS; task += nw) {
-                    const int k = 1 + p0 + task / ENS_PLANE_WARPS, vw = task % ENS_PLANE_WARPS;
-                    double acc2 = 0;
-                    for (uint32_t t = (uint32_t)(vw * 32 + lane); t < in_plane; t += 32 * ENS_PLANE_WARPS) {
-                        const uint32_t r = t / in_row;
-                        const int u = (k * nj + 1 + (int)r) * ni + 1 + (int)(t - r * in_row);
-                        const double Ru = -ph[u] * D + div_rcp(rh[u], ENS_EPS_0, yeps) +
-                                          idx2 * (ph[u - 1] + ph[u + 1]) + idy2 * (ph[u - sy] + ph[u + sy]) +
-                                          idz2 * (ph[u - sz] + ph[u + sz]);
-                        R[u] = (float)Ru;
-                        e[u] = 0.f;
-                        acc2 += Ru * Ru;
-                    }
-                    acc2 = ens_warp_sum(acc2);
-                    if (lane == 0) part[task] = acc2;
-                }
-                __syncthreads();
-                for (int kk = tid; kk < np; kk += nt) psum[p0 + kk] = ens_plane_sum(part + kk * ENS_PLANE_WARPS);
-                __syncthreads();
-            }
-            cluster_sync_global(cl);
-            if (warp == 0) {
-                const double t = ens_planes_total(pl.planes, [&](int p) { return __ldcg(psum + p); });
-                if (lane == 0) total = t;
-            }
-            __syncthreads();
-            L2 = sqrt(total / ((double)ni * nj * nk));
-            if (!isfinite(L2)) {
-                if (rank == 0 && tid == 0) atomicOr(err, DERR_NONFINITE);
-                break;
-            }
-            if (L2 < tol) {
-                conv = 1;
-                break;
-            }
-            if (sweeps >= max_it) break;
-            /* ENS_SWEEPS float32 sweeps of L e = -R, then phi += e and the
-             * float64 residual decides again */
-            const int ns = max_it - sweeps < ENS_SWEEPS ? max_it - sweeps : ENS_SWEEPS;
-            for (int s = 0; s < ns; s++) {
-                for (int c = 0; c < 2; c++) {
-                    /* four independent nodes of colour c per thread: all
-                     * loads before any store */
-                    for (int tb = c0 + tid; tb < c1; tb += 4 * nt) {
-                        int uq[4];
-                        float eo[4], sum[4];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const int t = tb + q * nt;
-                            uq[q] = -1;
-                            eo[q] = 0.f;
-                            sum[q] = 0.f;
-                            if (t >= c1) continue;
-                            const int i2 = t % hx;
-                            const int r = t / hx;
-                            const int j = 1 + r % (nj - 2);
-                            const int k = 1 + r / (nj - 2);
-                            const int i = 1 + 2 * i2 + ((1 + j + k + c) & 1);
-                            if (i > ni - 2) continue;
-                            const int u = (k * nj + j) * ni + i;
-                            uq[q] = u;
-                            eo[q] = e[u];
-                            sum[q] = R[u] + fcx * (e[u - 1] + e[u + 1]) + fcy * (e[u - sy] + e[u + sy]) +
-                                     fcz * (e[u - sz] + e[u + sz]);
-                        }
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            if (uq[q] < 0) continue;
-                            const float en = sum[q] * fiD;
-                            e[uq[q]] = eo[q] + fw * (en - eo[q]);
-                        }
-                    }
-                    cluster_sync_global(cl);
-                }
-            }
-            sweeps += ns;
-            for (int t = i0 + tid; t < i1; t += nt) {
-                const int i = 1 + t % (ni - 2);
-                const int r = t / (ni - 2);
-                const int j = 1 + r % (nj - 2);
-                const int k = 1 + r / (nj - 2);
-                const int u = (k * nj + j) * ni + i;
-                ph[u] += (double)e[u];
-            }
-            cluster_sync_global(cl);
-        }
-        if (solve && !slab) cluster_sync_global(cl); /* psum is read before E takes its place */
+            done = ens_sor_slab(boxes[bid], ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab, part,
+                                plane_sum, &total, err);
+        else if (solve) /* the planes' sums where the box's E will be written */
+            done = ens_sor_global(boxes[bid], ph, rh, R, e, max_it, tol, (double *)(ef4 + B.node0), part, &total, err);
         /* 3. E = -grad phi, float32 copy for the push */
         /* interior nodes first, the face nodes in passes of their own: a
          * row of at most 64 nodes puts a face lane into every warp, and the
@@ -591,9 +622,9 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
             ef4[B.node0 + u] = make_float4((float)e0, (float)e1, (float)e2, 0.f);
         }
         if (rank == 0 && tid == 0) {
-            stat[bid].sweeps = sweeps;
-            stat[bid].converged = conv;
-            stat[bid].residual = L2;
+            stat[bid].sweeps = done.sweeps;
+            stat[bid].converged = done.converged;
+            stat[bid].residual = done.residual;
         }
         cluster_sync_global(cl);
     }
