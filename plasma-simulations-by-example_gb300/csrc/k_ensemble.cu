@@ -862,6 +862,32 @@ static int ens_push_blocks(espic_ensemble &E) {
     return (int)(E.nwork < b ? (E.nwork > 0 ? E.nwork : 1) : b);
 }
 
+/* Shared memory of the solve launch: for the largest slab that fits
+ * (correction and right-hand side, or the correction alone), or none.  A
+ * launch with slabs leaves little L1 to the boxes that do not fit: they take
+ * 5% longer (64 boxes of 16 to 64 nodes an axis with single CTAs of 256
+ * threads, where the largest boxes decide: 124.4 ms without slabs, 130.1
+ * with), the others half as long (8 CTAs of 1024 threads: 15.6 and 7.9 ms).
+ * A box's time goes as its nodes and, through the sweeps, its longest axis;
+ * the launch's is that of the largest box or the sum over the clusters. */
+static int64_t ens_slab_launch(const espic_ensemble &E) {
+    int64_t bytes = 0;
+    double with = 0, without = 0, sum_with = 0, sum_without = 0;
+    for (const EnsBox &b : E.boxes) {
+        const int64_t e = 4 * ens_slab_e(b.g.ni, b.g.nj, b.g.nk, E.cluster);
+        const int64_t er = e + 4 * ens_slab_r(b.g.ni, b.g.nj, b.g.nk, E.cluster);
+        bytes = std::max(bytes, er <= ENS_SLAB_MAX ? er : (e <= ENS_SLAB_MAX ? e : 0));
+        const double t = (double)b.nn * std::max(b.g.ni, std::max(b.g.nj, b.g.nk));
+        const double t_with = e <= ENS_SLAB_MAX ? 0.5 * t : 1.05 * t;
+        with = std::max(with, t_with);
+        without = std::max(without, t);
+        sum_with += t_with;
+        sum_without += t;
+    }
+    const double clusters = std::max(1, E.sm_count / E.cluster);
+    return std::max(with, sum_with / clusters) <= std::max(without, sum_without / clusters) ? bytes : 0;
+}
+
 /* the solve launch: clusters of E.cluster CTAs, as many as can be resident
  * (one box each at a time), at most one per box */
 static cudaError_t ens_launch_solve(espic_ensemble &E, int solve) {
@@ -872,14 +898,7 @@ static cudaError_t ens_launch_solve(espic_ensemble &E, int solve) {
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(E.solve_threads);
-    /* shared memory for the largest slab that fits: correction and right-hand
-     * side, or the correction alone */
-    int64_t bytes = 0;
-    for (const EnsBox &b : E.boxes) {
-        const int64_t e = 4 * ens_slab_e(b.g.ni, b.g.nj, b.g.nk, E.cluster);
-        const int64_t er = e + 4 * ens_slab_r(b.g.ni, b.g.nj, b.g.nk, E.cluster);
-        bytes = std::max(bytes, er <= ENS_SLAB_MAX ? er : (e <= ENS_SLAB_MAX ? e : 0));
-    }
+    const int64_t bytes = ens_slab_launch(E);
     /* the limit belongs to the kernel, not to this ensemble: always the same
      * value, or another thread's ensemble could lower it before the launch */
     cudaError_t fe =
