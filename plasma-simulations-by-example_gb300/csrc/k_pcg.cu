@@ -143,6 +143,9 @@ __device__ __forceinline__ void grid_sum(cg::grid_group &grid, const T (&v)[NV],
         double x[NV];
 #pragma unroll
         for (int q = 0; q < NV; q++) x[q] = 0;
+        /* once for up to 160 blocks: unrolled by the compiler, the passes past
+         * the last block would add zeros in float64 */
+#pragma unroll 1
         for (unsigned b0 = lane; b0 < gridDim.x; b0 += 160) {
             double t[5][NV];
 #pragma unroll
