@@ -2195,7 +2195,26 @@ static int run_pcg(World &w) {
     }
     /* float: up to one node per thread, where both give a warp the same
      * nodes and so the same dot products; float64: up to 2^20 nodes */
-    const bool small = sizeof(T) == sizeof(float) ? w.nn <= (int64_t)PCG_THREADS_SMALL * w.sm_count : w.nn <= 1 << 20;
+    bool small = sizeof(T) == sizeof(float) ? w.nn <= (int64_t)PCG_THREADS_SMALL * w.sm_count : w.nn <= 1 << 20;
+    /* Solves of several worlds run beside each other when each takes a part
+     * of the SMs, which a small grid hardly misses.  Float solves in ms, one
+     * alone and per solve with three worlds in flight: 17x17x33 1.24 and 1.17
+     * on every SM, 1.24 and 0.42 on a third; 24x24x48 1.22 and 1.17, on half
+     * of them 1.31 and 0.64; 28x28x56 1.43 and 1.38, on a third with 1024
+     * threads 1.64 and 0.55 (with a block per 1024 nodes: 2.16 and 0.73, 2.17
+     * and 0.73, 2.30 and 0.80).  A float grid still has one node per thread,
+     * see span.  Float64: 17x17x33 1.41 and 1.32, on half 1.39 and 0.67;
+     * above 512 nodes an SM of a third, the SMs' float64 pipes count. */
+    const int64_t third = w.sm_count / 3, half = w.sm_count / 2;
+    int at_once = 1;
+    if (w.nn <= PCG_THREADS_SMALL * third) {
+        at_once = sizeof(T) == sizeof(float) ? 3 : 2;
+    } else if (sizeof(T) == sizeof(float) && w.nn <= PCG_THREADS_SMALL * half) {
+        at_once = 2;
+    } else if (sizeof(T) == sizeof(float) && w.nn <= PCG_THREADS * third) {
+        at_once = 3;
+        small = false;
+    }
     const int threads = small ? PCG_THREADS_SMALL : PCG_THREADS;
     const void *fn = (const void *)k_newton_pcg<T, PCG_THREADS, true>;
     if (small) fn = (const void *)k_newton_pcg<T, PCG_THREADS_SMALL, false>;
@@ -2212,11 +2231,11 @@ static int run_pcg(World &w) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn);
     if (per_sm < 1) per_sm = 1;
-    int64_t maxb = (int64_t)per_sm * w.sm_count;
-    /* every SM as soon as there is a warp of nodes for each: the phases of a
-     * small grid are bound by the instructions and float64 operations that
-     * one SM issues between two barriers, and a barrier of 152 blocks costs
-     * what one of 16 does (1.29 and 1.30 us) */
+    int64_t maxb = (int64_t)per_sm * (w.sm_count / at_once);
+    /* every SM (of the share) as soon as there is a warp of nodes for each:
+     * the phases of a small grid are bound by the instructions and float64
+     * operations that one SM issues between two barriers, and a barrier of
+     * 152 blocks costs what one of 16 does (1.29 and 1.30 us) */
     int64_t needb = (w.nn + 31) / 32;
     int grid = (int)(needb < maxb ? needb : maxb);
     if (grid > w.partial_slots / 4) grid = w.partial_slots / 4;
