@@ -1196,13 +1196,13 @@ static SorConst sor_const(const Geo &g) {
 }
 
 /* entry t (below n) of colour c's enumeration */
-template <typename I>
-__device__ __forceinline__ SorNode<I> sor_node(const Geo &g, const SorConst &k, I t, I n, int c,
+template <typename I, typename U>
+__device__ __forceinline__ SorNode<I> sor_node(const Geo &g, const SorConst &k, U hx, U t, U n, int c,
                                                const double *__restrict__ rho) {
     SorNode<I> s = {-1, 0.0};
     if (t >= n) return s;
-    s.u = sor_entry<I>(g, t, c);
-    if (s.u >= 0) s.b = div_rcp(rho[s.u], k.eps0, k.reps0);
+    if (!sor_entry(g, hx, t, c, s.u)) return s;
+    s.b = div_rcp(rho[s.u], k.eps0, k.reps0);
     return s;
 }
 
@@ -1248,16 +1248,17 @@ __global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi,
                                                  int max_it, double tol, double *partials, SolveStatus *st,
                                                  int *err) {
     cg::grid_group grid = cg::this_grid();
+    using U = std::make_unsigned_t<I>;
     const I sy = g.ni, sz = (I)g.ni * g.nj;
-    const I count = (I)(sor_row_entries(g) * sor_rows(g));
-    const I gsize = (I)gridDim.x * blockDim.x, gtid = (I)blockIdx.x * blockDim.x + threadIdx.x;
+    const U hx = (U)sor_row_entries(g), count = hx * (U)(g.nj - 2) * (U)(g.nk - 2);
+    const U gsize = (U)gridDim.x * blockDim.x, gtid = (U)blockIdx.x * blockDim.x + threadIdx.x;
     const bool held = sizeof(I) == 4 && count <= SOR_HELD * gsize;
     SorNode<I> node[2][SOR_HELD];
     if (held)
 #pragma unroll
         for (int c = 0; c < 2; c++)
 #pragma unroll
-            for (int h = 0; h < SOR_HELD; h++) node[c][h] = sor_node<I>(g, k, gtid + h * gsize, count, c, rho);
+            for (int h = 0; h < SOR_HELD; h++) node[c][h] = sor_node<I, U>(g, k, hx, gtid + h * gsize, count, c, rho);
     double L2 = 0;
     int conv = 0, it, round = 0;
     for (it = 0; it < max_it; it++) {
@@ -1272,8 +1273,8 @@ __global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi,
                 for (int h = 0; h < SOR_HELD; h++)
                     if (node[c][h].u >= 0) phi[node[c][h].u] = v[h];
             } else {
-                for (I t = gtid; t < count; t += gsize) {
-                    const SorNode<I> s = sor_node<I>(g, k, t, count, c, rho);
+                for (U t = gtid; t < count; t += gsize) {
+                    const SorNode<I> s = sor_node<I>(g, k, hx, t, count, c, rho);
                     if (s.u >= 0) phi[s.u] = sor_value(k, phi, s, sy, sz);
                 }
             }
@@ -1287,8 +1288,8 @@ __global__ void __launch_bounds__(256) k_sor_box(Geo g, SorConst k, double *phi,
 #pragma unroll
                     for (int h = 0; h < SOR_HELD; h++) sum += sor_residual2(k, phi, node[c][h], sy, sz);
                 } else {
-                    for (I t = gtid; t < count; t += gsize)
-                        sum += sor_residual2(k, phi, sor_node<I>(g, k, t, count, c, rho), sy, sz);
+                    for (U t = gtid; t < count; t += gsize)
+                        sum += sor_residual2(k, phi, sor_node<I>(g, k, hx, t, count, c, rho), sy, sz);
                 }
             }
             double tot = grid_sum(grid, sum, partials, round);
@@ -1325,10 +1326,12 @@ __global__ void __launch_bounds__(SOR_CTA_NODES) k_sor_cluster(Geo g, SorConst k
     __shared__ double warp_sum[SOR_CTA_NODES / 32];
     const int rank = (int)cl.block_rank();
     const int32_t sy = g.ni, sz = g.ni * g.nj, nn = sz * g.nk;
-    const int32_t count = (int32_t)(sor_row_entries(g) * sor_rows(g));
-    const int32_t t = rank * (int32_t)per + (int32_t)threadIdx.x;
-    const int32_t top = threadIdx.x < per ? count : 0;
-    const SorNode<int32_t> node[2] = {sor_node(g, k, t, top, 0, rho), sor_node(g, k, t, top, 1, rho)};
+    const uint32_t hx = (uint32_t)sor_row_entries(g);
+    const uint32_t count = hx * (uint32_t)(g.nj - 2) * (uint32_t)(g.nk - 2);
+    const uint32_t t = (uint32_t)rank * per + threadIdx.x;
+    const uint32_t top = threadIdx.x < per ? count : 0u;
+    const SorNode<int32_t> node[2] = {sor_node<int32_t>(g, k, hx, t, top, 0, rho),
+                                      sor_node<int32_t>(g, k, hx, t, top, 1, rho)};
     for (int32_t u = threadIdx.x; u < nn; u += blockDim.x) sor_phi[u] = phi[u];
     cl.sync();
     double L2 = 0;

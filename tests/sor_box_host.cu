@@ -20,7 +20,13 @@ extern "C" int64_t sor_host_misplaced(int ni, int nj, int nk, int64_t first, int
             const int64_t k = 1 + t / hx / (nj - 2), j = 1 + t / hx % (nj - 2);
             const int64_t i = 1 + 2 * (t % hx) + ((1 + j + k + c) & 1);
             const int64_t want = i <= ni - 2 ? (k * nj + j) * ni + i : -1;
-            const int64_t got = brief ? (int64_t)sor_entry<int32_t>(g, (int32_t)t, c) : sor_entry<int64_t>(g, t, c);
+            int64_t got = -1;
+            if (brief) {
+                int32_t u;
+                if (sor_entry(g, (uint32_t)hx, (uint32_t)t, c, u)) got = u;
+            } else {
+                sor_entry(g, (uint64_t)hx, (uint64_t)t, c, got);
+            }
             bad += got != want;
         }
     return bad;
