@@ -164,6 +164,15 @@ __host__ __device__ inline int64_t ens_slab_r(int ni, int nj, int nk, int C) {
     return 2ll * ens_planes(nk, C).most() * nj * ens_slots(ni);
 }
 
+/* whether a box is swept in a launch's shared memory: its correction fits, its
+ * planes' sums fit their arrays, a colour fits a work array, and div_small's
+ * range holds whatever the axes */
+__host__ __device__ inline bool ens_has_slab(int ni, int nj, int nk, int C, int64_t slab_bytes) {
+    const int64_t nn = (int64_t)ni * nj * nk;
+    return nn < (1 << 24) && 4 * ens_slab_e(ni, nj, nk, C) <= slab_bytes &&
+           ens_planes(nk, C).most() <= ENS_VW / ENS_PLANE_WARPS && (int64_t)(nk - 2) * nj * ens_slots(ni) <= nn;
+}
+
 /* Pieces of the residual's sum, whose bits depend on neither the cluster nor
  * the block size: a plane's nodes in ENS_PLANE_WARPS virtual warps (ens_warp_sum
  * of each), their sums in order (ens_plane_sum), and the planes' sums over the
@@ -204,9 +213,10 @@ struct EnsSolved {
  * 5.2 ms before, 2.9 ms now; what is left is a third float64 residuals (14
  * instructions a node).  The residual's sum is taken as in k_ens_solve, the
  * planes' sums from the CTAs' shared memory. */
-__device__ __noinline__ EnsSolved ens_sor_slab(const EnsBox &B, double *ph, const double *__restrict__ rh, float *R0,
-                                               float *R1, int max_it, double tol, bool r_shared, float *slab,
-                                               double *part, double *plane_sum, double *total, int *err) {
+__device__ __forceinline__ EnsSolved ens_sor_slab(const EnsBox &B, double *ph, const double *__restrict__ rh,
+                                                  float *R0, float *R1, int max_it, double tol, bool r_shared,
+                                                  float *slab, double *part, double *plane_sum, double *total,
+                                                  int *err) {
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
     const Geo &g = B.g;
@@ -352,10 +362,15 @@ __device__ __noinline__ EnsSolved ens_sor_slab(const EnsBox &B, double *ph, cons
     return {sweeps, conv, L2};
 }
 
+__device__ __noinline__ EnsSolved ens_sor_slab_call(const EnsBox &B, double *ph, const double *rh, float *R0, float *R1,
+                                                    int max_it, double tol, bool r_shared, float *slab, double *part,
+                                                    double *plane_sum, double *total, int *err) {
+    return ens_sor_slab(B, ph, rh, R0, R1, max_it, tol, r_shared, slab, part, plane_sum, total, err);
+}
+
 /* The sweeps of one box whose slab does not fit the launch's shared memory:
  * e and R in global memory, every half sweep's nodes an even share of each
- * CTA.  psum: the planes' sums, one double a plane of the box.  A function of
- * its own, like ens_sor_slab: inlined into one kernel the two spilled. */
+ * CTA.  psum: the planes' sums, one double a plane of the box. */
 __device__ __noinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, const double *__restrict__ rh, float *R,
                                                  float *e, int max_it, double tol, double *psum, double *part,
                                                  double *total, int *err) {
@@ -493,7 +508,10 @@ __device__ __noinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, co
  * shared memory.  The residual is summed plane by plane on both routes (see
  * ens_planes_total), here with the planes' sums in global memory, so the
  * solve's outcome depends on neither C nor the block size, nor on whether
- * these let the box's slab fit. */
+ * these let the box's slab fit.  ALL_SLABS: every box has its slab, whose
+ * sweeps are then inlined; else both routes are calls, since inlined into one
+ * kernel of 64 registers they spill. */
+template <bool ALL_SLABS>
 __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ boxes, const EnsSeg *__restrict__ segs,
                                                     int nsp, const int *__restrict__ order, int nbox, int *counter,
                                                     double *phi, double *rho, float *ecor, float *res, float4 *ef4,
@@ -531,8 +549,7 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
         const float inv_ni = 1.f / (float)ni, inv_nj = 1.f / (float)nj;
         const bool small = nn < (1 << 24); /* div_small's range, whatever the axes */
         const int64_t slab_e = 4 * ens_slab_e(ni, nj, nk, C), slab_r = 4 * ens_slab_r(ni, nj, nk, C);
-        const bool slab = small && slab_e <= slab_bytes && ens_planes(nk, C).most() <= ENS_VW / ENS_PLANE_WARPS &&
-                          (int64_t)(nk - 2) * nj * ens_slots(ni) <= nn; /* a colour fits a work array */
+        const bool slab = ALL_SLABS || ens_has_slab(ni, nj, nk, C, slab_bytes);
         for (int64_t u = n0 + tid; u < n1; u += nt) {
             int i, j, k;
             if (small) {
@@ -562,9 +579,12 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
          *    residual */
         const int sy = ni, sz = ni * nj;
         EnsSolved done = {0, 0, 0.0};
-        if (solve && slab)
-            done = ens_sor_slab(boxes[bid], ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab, part,
-                                plane_sum, &total, err);
+        if (solve && ALL_SLABS)
+            done = ens_sor_slab(B, ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab, part, plane_sum,
+                                &total, err);
+        else if (solve && slab)
+            done = ens_sor_slab_call(boxes[bid], ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab,
+                                     part, plane_sum, &total, err);
         else if (solve) /* the planes' sums where the box's E will be written */
             done = ens_sor_global(boxes[bid], ph, rh, R, e, max_it, tol, (double *)(ef4 + B.node0), part, &total, err);
         /* 3. E = -grad phi, float32 copy for the push */
@@ -876,9 +896,10 @@ static int64_t ens_slab_launch(const espic_ensemble &E) {
     for (const EnsBox &b : E.boxes) {
         const int64_t e = 4 * ens_slab_e(b.g.ni, b.g.nj, b.g.nk, E.cluster);
         const int64_t er = e + 4 * ens_slab_r(b.g.ni, b.g.nj, b.g.nk, E.cluster);
-        bytes = std::max(bytes, er <= ENS_SLAB_MAX ? er : (e <= ENS_SLAB_MAX ? e : 0));
+        const bool fits = ens_has_slab(b.g.ni, b.g.nj, b.g.nk, E.cluster, ENS_SLAB_MAX);
+        if (fits) bytes = std::max(bytes, er <= ENS_SLAB_MAX ? er : e);
         const double t = (double)b.nn * std::max(b.g.ni, std::max(b.g.nj, b.g.nk));
-        const double t_with = e <= ENS_SLAB_MAX ? 0.5 * t : 1.05 * t;
+        const double t_with = fits ? 0.5 * t : 1.05 * t;
         with = std::max(with, t_with);
         without = std::max(without, t);
         sum_with += t_with;
@@ -899,10 +920,12 @@ static cudaError_t ens_launch_solve(espic_ensemble &E, int solve) {
     attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(E.solve_threads);
     const int64_t bytes = ens_slab_launch(E);
+    bool all = true;
+    for (const EnsBox &b : E.boxes) all = all && ens_has_slab(b.g.ni, b.g.nj, b.g.nk, E.cluster, bytes);
+    auto *fn = all ? k_ens_solve<true> : k_ens_solve<false>;
     /* the limit belongs to the kernel, not to this ensemble: always the same
      * value, or another thread's ensemble could lower it before the launch */
-    cudaError_t fe =
-        cudaFuncSetAttribute(k_ens_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ENS_SLAB_MAX);
+    cudaError_t fe = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ENS_SLAB_MAX);
     if (fe != cudaSuccess) return fe;
     cfg.dynamicSmemBytes = (size_t)bytes;
     cfg.stream = E.stream;
@@ -910,11 +933,11 @@ static cudaError_t ens_launch_solve(espic_ensemble &E, int solve) {
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(E.cluster);
     int ncl = 0;
-    cudaError_t ce = cudaOccupancyMaxActiveClusters(&ncl, (void *)k_ens_solve, &cfg);
+    cudaError_t ce = cudaOccupancyMaxActiveClusters(&ncl, (void *)fn, &cfg);
     if (ce != cudaSuccess || ncl < 1) ncl = E.sm_count / E.cluster > 0 ? E.sm_count / E.cluster : 1;
     if (ncl > E.nbox) ncl = E.nbox;
     cfg.gridDim = dim3(ncl * E.cluster);
-    return cudaLaunchKernelEx(&cfg, k_ens_solve, (const EnsBox *)E.d_boxes, (const EnsSeg *)E.d_segs, E.nsp,
+    return cudaLaunchKernelEx(&cfg, fn, (const EnsBox *)E.d_boxes, (const EnsSeg *)E.d_segs, E.nsp,
                               (const int *)E.d_order, E.nbox, E.d_counter, E.phi, E.rho, E.ecor, E.res, E.ef4, E.acc,
                               E.total_nodes, E.max_it, E.tol, solve, E.d_stat, (int)bytes, E.d_err);
 }
