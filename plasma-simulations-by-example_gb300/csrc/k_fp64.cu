@@ -964,9 +964,9 @@ __global__ void k_targets(Geo g, const int32_t *__restrict__ obj, int32_t *targe
  * followed by Field_::operator/=, ch2/Field.h:125-134.  Bound by the float64
  * pipe, five operations a node, and by the loads in flight: on large grids
  * the conversion of the count is made of integer operations and a thread
- * takes two nodes with 16-byte loads (ten transport steps of 60M ions on
- * 128x128x256 nodes, one of these each: 7.74 ms with a node a thread, 7.67 ms
- * with two). */
+ * takes two nodes with 16-byte loads (the density of 64 ions, clear and
+ * deposit included, on 128x128x256 nodes 55.5 us with a node a thread, 47.3
+ * with two; 256x256x512: 356 and 291 us). */
 template <int PER>
 __device__ __forceinline__ double node_density(unsigned long long count, double unit, double v, double iv) {
     const double c = PER > 1 ? count_to_double((long long)count) : __ll2double_rn((long long)count);
@@ -1699,9 +1699,9 @@ void launch_compact(World &w, Species &s) {
 }
 
 void launch_density(World &w, Species &s) {
-    /* two nodes a thread where that still fills every SM (2048 threads); on
-     * smaller grids it gains nothing (10 transport steps on 64x74x126 nodes:
-     * 0.81 ms either way) */
+    /* two nodes a thread where that still fills every SM (2048 threads): 87x89x91
+     * nodes, just above, 18.6 us with one and 17.9 with two; 64x74x126, just
+     * below, 16.6 us either way */
     if (w.nn >= 2 * 2048 * (int64_t)w.sm_count)
         k_density<2><<<blocks_for((w.nn + 1) / 2, 256), 256, 0, w.stream>>>(w.nn, s.acc, s.unit, w.vol, w.ivol, s.den);
     else
@@ -2206,7 +2206,10 @@ static int coop_grid(World &w, const void *fn, int threads, int64_t work) {
 /* The cluster form fits when a block's share is one node of each colour per
  * thread, the potential fits its shared memory, and the device takes such a
  * cluster (asked once per world; an upper bound on the solver's blocks below
- * the cluster's size asks for the grid form). */
+ * the cluster's size asks for the grid form).  A sweep in the cluster and on
+ * the whole grid: 13^3 2.30 and 4.26 us, 17^3 2.85 and 4.41, 21^3 3.95 and
+ * 4.26, 23^3 (4,851 entries a colour) 4.4-4.6 and 4.37, 26x25x23 (5,796)
+ * 5.5 and 4.35: the last boxes that fit lose by it. */
 static bool sor_cluster_fits(World &w, uint32_t per, size_t smem) {
     if (per > SOR_CTA_NODES || smem > 200 * 1024) return false;
     if (w.solver_blocks > 0 && w.solver_blocks < SOR_CTAS) return false;
@@ -2458,6 +2461,8 @@ __global__ void __launch_bounds__(256) k_mom_scatter(Geo g, double3 rdh, const d
                                                      double w0, const int64_t *__restrict__ d_count,
                                                      const double *__restrict__ scale, unsigned long long *acc,
                                                      int *err) {
+    /* node indices: 32 bits, since 2^31 nodes of moments (120 bytes a node
+     * for these sums alone) do not fit the card */
     __shared__ longlong2 turn[8][32 * 4];
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;

@@ -658,13 +658,6 @@ __device__ __forceinline__ void restrict_store(const MgLevel<T> &C, bool valid, 
     if (((ci + cj + ck) & 1) == 0 && d != (T)0) C.e[I] = LIGHT<T> ? sum * d : sum / d;
 }
 
-/* b of level 1 = sum of the node-grid children's residuals (r - J z).  When
- * the level has fewer nodes than the grid has threads (latency-bound),
- * four consecutive threads take the four red children of a coarse node,
- * each issuing all its loads at once (neighbour indices clamped into the
- * grid; a child that is not an unknown contributes zero); otherwise
- * (bandwidth-bound) a thread takes a coarse node and its four children, so
- * that a warp's loads of one child cover consecutive nodes of a row. */
 /* A red child of the node grid: what its residual needs, loaded at once, and
  * the residual (0 for a node that is not an unknown, or not interior). */
 template <typename T>
@@ -713,6 +706,13 @@ __device__ __forceinline__ uint32_t interior_or_safe(const Geo &g, int i, int j,
     return (kk * (uint32_t)g.nj + jj) * (uint32_t)g.ni + ii;
 }
 
+/* b of level 1 = sum of the node-grid children's residuals (r - J z).  When
+ * the level has fewer nodes than the grid has threads (latency-bound),
+ * four consecutive threads take the four red children of a coarse node,
+ * each issuing all its loads at once (neighbour indices clamped into the
+ * grid; a child that is not an unknown contributes zero); otherwise
+ * (bandwidth-bound) a thread takes a coarse node and its four children, so
+ * that a warp's loads of one child cover consecutive nodes of a row. */
 template <typename T>
 __device__ __forceinline__ void restrict_fine() {
     const Fine<T> &F = shared_of<T>().F;
@@ -2194,7 +2194,10 @@ static int run_pcg(World &w) {
         w.pcg_codes_valid = true;
     }
     /* float: up to one node per thread, where both give a warp the same
-     * nodes and so the same dot products; float64: up to 2^20 nodes */
+     * nodes and so the same dot products; float64: up to 2^20 nodes
+     * (102x102x100, just below: 21.2 ms a cold solve with 512 threads, 25.0
+     * with 1024 and calls; 96x96x192, above: 13.8 and 14.4; 128x128x192: 29.8
+     * either way) */
     bool small = sizeof(T) == sizeof(float) ? w.nn <= (int64_t)PCG_THREADS_SMALL * w.sm_count : w.nn <= 1 << 20;
     /* Solves of several worlds run beside each other when each takes a part
      * of the SMs, which a small grid hardly misses.  Float solves in ms, one
@@ -2218,8 +2221,10 @@ static int run_pcg(World &w) {
     const int threads = small ? PCG_THREADS_SMALL : PCG_THREADS;
     const void *fn = (const void *)k_newton_pcg<T, PCG_THREADS, true>;
     if (small) fn = (const void *)k_newton_pcg<T, PCG_THREADS_SMALL, false>;
-    /* between: the passes inlined (64x64x128 float sphere step: 1.09 ms, 1.12
-     * as calls; 256x256x512: 25.7 ms inlined, 24.9 as calls) */
+    /* between: the passes inlined (a cold solve of 128x128x127 nodes, just
+     * below the line: 10.3 ms, 10.8 as calls; above it the calls are not yet
+     * ahead: 128x128x129 10.5 and 11.0, 160x160x320 16.2 and 16.4; 256x256x512
+     * sphere step: 25.7 ms inlined, 24.9 as calls) */
     if constexpr (sizeof(T) == sizeof(float))
         if (!small && w.nn <= 1 << 21) fn = (const void *)k_newton_pcg<T, PCG_THREADS, false>;
     size_t dyn = 0;

@@ -211,7 +211,8 @@ extern "C" int espic_deposit_noalloc(const double *d_P, int64_t stride, int64_t 
     int S = ex - 1 > 52 ? 52 : ex - 1;
     double fx = ldexp(1.0, S);
     cudaStream_t st = (cudaStream_t)stream;
-    /* small blocks for few particles: an even share of float64 work per SM */
+    /* small blocks for few particles (4096 an SM of 152): an even share of
+     * float64 work per SM */
     const unsigned nt = n < 600000 ? 64 : 256;
     k_na_clear<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, (uint32_t)nn, d_flags);
     cudaError_t e = cudaGetLastError();

@@ -53,3 +53,16 @@ def test_instances_on_either_side_of_their_sizes(espic, fp32, below, above):
     (n0, i0), (n1, i1) = runs
     assert n0 == n1
     assert abs(i0 - i1) <= n0 + 0.25 * i0, runs
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("nodes", [(5, 5, 6), (29, 29, 30), (30, 30, 29), (33, 34, 34), (34, 34, 34), (37, 37, 37),
+                                   (37, 37, 38), (42, 42, 44)])
+def test_small_grids_on_their_share_of_the_sms(espic, nodes, fp32):
+    """Grids at the edges of the shares of the SMs that small solves take (on
+    152 SMs: a node per thread on a third with 512 threads, on half, on a
+    third with 1024, on all)."""
+    nr_tol, pcg_tol = (1e-6, 1e-6) if fp32 else (1e-9, 1e-12)
+    phi, _, _ = solve(espic, nodes, fp32, nr_tol, pcg_tol)
+    want, _, _ = solve(espic, nodes, False, 1e-9, 1e-12, levels=0)
+    assert np.max(np.abs(phi - want)) <= (nr_tol * np.sqrt(phi.size) if fp32 else 2e-6)
