@@ -30,8 +30,8 @@
  * in float64; while L2 >= tol, 25 red-black sweeps solve L e = -R for a
  * float32 correction e (e = 0 on the walls) and phi += e.  The float64
  * residual bounds the error of phi, the float32 sweeps do the work.  Its
- * reduction uses a fixed virtual width of 1024 partial sums and a fixed tree,
- * so results do not depend on the block size the autotuner picks.
+ * sum is taken plane by plane in a fixed order, so results do not depend on
+ * the launch shape the autotuner picks.
  */
 #include <math.h>
 #include <stdarg.h>
@@ -362,18 +362,12 @@ __device__ __forceinline__ EnsSolved ens_sor_slab(const EnsBox &B, double *ph, c
     return {sweeps, conv, L2};
 }
 
-__device__ __noinline__ EnsSolved ens_sor_slab_call(const EnsBox &B, double *ph, const double *rh, float *R0, float *R1,
-                                                    int max_it, double tol, bool r_shared, float *slab, double *part,
-                                                    double *plane_sum, double *total, int *err) {
-    return ens_sor_slab(B, ph, rh, R0, R1, max_it, tol, r_shared, slab, part, plane_sum, total, err);
-}
-
 /* The sweeps of one box whose slab does not fit the launch's shared memory:
  * e and R in global memory, every half sweep's nodes an even share of each
  * CTA.  psum: the planes' sums, one double a plane of the box. */
-__device__ __noinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, const double *__restrict__ rh, float *R,
-                                                 float *e, int max_it, double tol, double *psum, double *part,
-                                                 double *total, int *err) {
+__device__ __forceinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, const double *__restrict__ rh,
+                                                    float *R, float *e, int max_it, double tol, double *psum,
+                                                    double *part, double *total, int *err) {
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
     const Geo &g = B.g;
@@ -500,6 +494,12 @@ __device__ __noinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, co
     return {sweeps, conv, L2};
 }
 
+__device__ __noinline__ EnsSolved ens_sor_global_call(const EnsBox &B, double *ph, const double *rh, float *R, float *e,
+                                                      int max_it, double tol, double *psum, double *part,
+                                                      double *total, int *err) {
+    return ens_sor_global(B, ph, rh, R, e, max_it, tol, psum, part, total, err);
+}
+
 /* One box per thread-block cluster of C CTAs (C = 1, 2, 4 or 8, chosen at
  * launch): the CTAs split every node pass and every half sweep into
  * contiguous slices and meet at cluster barriers.  Boxes whose slabs fit the
@@ -508,10 +508,15 @@ __device__ __noinline__ EnsSolved ens_sor_global(const EnsBox &B, double *ph, co
  * shared memory.  The residual is summed plane by plane on both routes (see
  * ens_planes_total), here with the planes' sums in global memory, so the
  * solve's outcome depends on neither C nor the block size, nor on whether
- * these let the box's slab fit.  ALL_SLABS: every box has its slab, whose
- * sweeps are then inlined; else both routes are calls, since inlined into one
- * kernel of 64 registers they spill. */
-template <bool ALL_SLABS>
+ * these let the box's slab fit.  ROUTES: those of the launch's
+ * boxes.  The shared-memory sweeps are inlined (64 boxes of 16 to 64 nodes
+ * with 8 CTAs, five steps: 22.1 ms, as a call 22.8), the others a call where
+ * they are alone (24 boxes of 80 to 120 nodes an axis with single CTAs of
+ * 1024 threads, three steps: 887 ms, inlined 987) and inlined beside them
+ * (512 boxes, 4 CTAs: 27.2 ms a step, as calls 27.5). */
+enum { ENS_SLAB = 1, ENS_GLOBAL = 2 };
+
+template <int ROUTES>
 __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ boxes, const EnsSeg *__restrict__ segs,
                                                     int nsp, const int *__restrict__ order, int nbox, int *counter,
                                                     double *phi, double *rho, float *ecor, float *res, float4 *ef4,
@@ -549,7 +554,7 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
         const float inv_ni = 1.f / (float)ni, inv_nj = 1.f / (float)nj;
         const bool small = nn < (1 << 24); /* div_small's range, whatever the axes */
         const int64_t slab_e = 4 * ens_slab_e(ni, nj, nk, C), slab_r = 4 * ens_slab_r(ni, nj, nk, C);
-        const bool slab = ALL_SLABS || ens_has_slab(ni, nj, nk, C, slab_bytes);
+        const bool slab = ROUTES == ENS_SLAB || ((ROUTES & ENS_SLAB) && ens_has_slab(ni, nj, nk, C, slab_bytes));
         for (int64_t u = n0 + tid; u < n1; u += nt) {
             int i, j, k;
             if (small) {
@@ -579,14 +584,14 @@ __global__ void __launch_bounds__(1024) k_ens_solve(const EnsBox *__restrict__ b
          *    residual */
         const int sy = ni, sz = ni * nj;
         EnsSolved done = {0, 0, 0.0};
-        if (solve && ALL_SLABS)
+        if (solve && slab)
             done = ens_sor_slab(B, ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab, part, plane_sum,
                                 &total, err);
-        else if (solve && slab)
-            done = ens_sor_slab_call(boxes[bid], ph, rh, R, e, max_it, tol, slab_e + slab_r <= slab_bytes, ens_slab,
-                                     part, plane_sum, &total, err);
         else if (solve) /* the planes' sums where the box's E will be written */
-            done = ens_sor_global(boxes[bid], ph, rh, R, e, max_it, tol, (double *)(ef4 + B.node0), part, &total, err);
+            done = ROUTES == ENS_GLOBAL
+                       ? ens_sor_global_call(boxes[bid], ph, rh, R, e, max_it, tol, (double *)(ef4 + B.node0), part,
+                                             &total, err)
+                       : ens_sor_global(B, ph, rh, R, e, max_it, tol, (double *)(ef4 + B.node0), part, &total, err);
         /* 3. E = -grad phi, float32 copy for the push */
         /* interior nodes first, the face nodes in passes of their own: a
          * row of at most 64 nodes puts a face lane into every warp, and the
@@ -884,10 +889,12 @@ static int ens_push_blocks(espic_ensemble &E) {
 
 /* Shared memory of the solve launch: for the largest slab that fits
  * (correction and right-hand side, or the correction alone), or none.  A
- * launch with slabs leaves little L1 to the boxes that do not fit: they take
- * 5% longer (64 boxes of 16 to 64 nodes an axis with single CTAs of 256
- * threads, where the largest boxes decide: 124.4 ms without slabs, 130.1
- * with), the others half as long (8 CTAs of 1024 threads: 15.6 and 7.9 ms).
+ * launch with slabs leaves little L1, and the slower of its two forms, to the
+ * boxes that do not fit: they take 15% longer (64 boxes of 16 to 64 nodes an
+ * axis with single CTAs of 256 threads, where the largest boxes decide: 114 ms
+ * without slabs, 131 with), the others half as long (8 CTAs of 1024 threads:
+ * 15.5 and 7.7 ms; 512 such boxes with 4 CTAs, of which the largest do not
+ * fit: 39 and 27 ms a step).
  * A box's time goes as its nodes and, through the sweeps, its longest axis;
  * the launch's is that of the largest box or the sum over the clusters. */
 static int64_t ens_slab_launch(const espic_ensemble &E) {
@@ -899,7 +906,7 @@ static int64_t ens_slab_launch(const espic_ensemble &E) {
         const bool fits = ens_has_slab(b.g.ni, b.g.nj, b.g.nk, E.cluster, ENS_SLAB_MAX);
         if (fits) bytes = std::max(bytes, er <= ENS_SLAB_MAX ? er : e);
         const double t = (double)b.nn * std::max(b.g.ni, std::max(b.g.nj, b.g.nk));
-        const double t_with = fits ? 0.5 * t : 1.05 * t;
+        const double t_with = fits ? 0.5 * t : 1.15 * t;
         with = std::max(with, t_with);
         without = std::max(without, t);
         sum_with += t_with;
@@ -920,9 +927,12 @@ static cudaError_t ens_launch_solve(espic_ensemble &E, int solve) {
     attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(E.solve_threads);
     const int64_t bytes = ens_slab_launch(E);
-    bool all = true;
-    for (const EnsBox &b : E.boxes) all = all && ens_has_slab(b.g.ni, b.g.nj, b.g.nk, E.cluster, bytes);
-    auto *fn = all ? k_ens_solve<true> : k_ens_solve<false>;
+    int routes = 0;
+    for (const EnsBox &b : E.boxes)
+        routes |= ens_has_slab(b.g.ni, b.g.nj, b.g.nk, E.cluster, bytes) ? ENS_SLAB : ENS_GLOBAL;
+    auto *fn = routes == ENS_SLAB     ? k_ens_solve<ENS_SLAB>
+               : routes == ENS_GLOBAL ? k_ens_solve<ENS_GLOBAL>
+                                      : k_ens_solve<ENS_SLAB | ENS_GLOBAL>;
     /* the limit belongs to the kernel, not to this ensemble: always the same
      * value, or another thread's ensemble could lower it before the launch */
     cudaError_t fe = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ENS_SLAB_MAX);
